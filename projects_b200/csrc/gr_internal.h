@@ -178,10 +178,11 @@ struct RowArgs {
 // as one complex line (gridrec_kernels.cu); backprojection in gridrec_fbp.cu.
 struct FbpFilterArgs {
   const float* sino;     // [slice][n_ang][n]
-  float* filt;           // [slice][n_ang][n]
+  float* filt;           // [slice / group][n_ang][n][slice % group]
   const float* lut;      // n filter weights
   const float2* tw;      // two-level twiddle table for n
   int n, n_ang, slices;
+  int group;             // slices interleaved in filt (slices is a multiple of it)
 };
 cudaError_t launch_fbp_filter(const FbpFilterArgs& a, cudaStream_t s);
 

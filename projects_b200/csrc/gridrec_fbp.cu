@@ -19,42 +19,146 @@
 namespace gr {
 namespace {
 
-constexpr int kBpX = 32, kBpY = 8;
+// A block covers kBpTile x 8 R pixels of S slices: the sample a (pixel, angle) takes
+// depends on the geometry only, so one index serves all S slices, whose filtered rows are
+// interleaved ([angle][k][slice], one S-float load).  A warp covers 8 x 4 pixels, whose
+// samples at one angle span a few consecutive elements whatever the direction, and a
+// thread R pixels, eight rows apart: R independent chains per angle.
+// Bound by the instruction issue: about 8 instructions per (pixel, angle) for the index
+// and one load and S additions for the sums.  The index (int)((r + 1) n/2) comes from an
+// addition of 2^23 rounded toward zero (exact for 0 <= t < 2^23) instead of a conversion,
+// whose pipe runs at a quarter of the rate.  In blocks that lie well inside the unit
+// circle -1 < r < 1 holds for every angle, so they skip the range test and the clamp.
+// 2 slices of 2048 x 1500: 2.89 ms with the filter, against 7.70 ms for one slice and one
+// pixel per thread with a conversion and a range test per sample.
+constexpr int kBpTile = 32, kBpThreads = 256;
 
-__global__ void __launch_bounds__(kBpX * kBpY) fbp_backproject_kernel(const float* filt,
-                                                                     const float2* cs,
-                                                                     float* recon, int n,
-                                                                     int n_ang) {
-  extern __shared__ float2 s_cs[];
-  const int tid = threadIdx.y * kBpX + threadIdx.x;
-  for (int i = tid; i < n_ang; i += kBpX * kBpY) s_cs[i] = cs[i];
-  __syncthreads();
-  const int xi = blockIdx.x * kBpX + threadIdx.x, yi = blockIdx.y * kBpY + threadIdx.y;
-  const int s = blockIdx.z;
-  if (xi >= n || yi >= n) return;
-  const float h = (float)n / 2.0f;
-  const float x = __fdiv_rn(__fsub_rn((float)xi, h), h);
-  const float y = __fdiv_rn(__fsub_rn((float)yi, h), h);
-  const float* f = filt + (size_t)s * n_ang * n;
-  float acc = 0.f;
-  for (int a = 0; a < n_ang; ++a) {
-    const float2 c = s_cs[a];  // (cos, sin)
-    const float r = __fadd_rn(__fmul_rn(x, c.x), __fmul_rn(y, c.y));
-    if (r >= -1.f && r < 1.f) {
-      // r just below 1 can round (r + 1) n/2 up to n; the reference then reads
-      // the next row (or past its buffer), here the last sample of the row
-      const int k = min((int)__fmul_rn(__fadd_rn(r, 1.f), h), n - 1);
-      acc = __fadd_rn(acc, __ldg(&f[(size_t)a * n + k]));
+template <int S>
+struct BpVec;
+template <>
+struct BpVec<1> {
+  using T = float;
+  static __device__ __forceinline__ void add(float (&a)[1], float v) { a[0] = __fadd_rn(a[0], v); }
+};
+template <>
+struct BpVec<2> {
+  using T = float2;
+  static __device__ __forceinline__ void add(float (&a)[2], float2 v) {
+    a[0] = __fadd_rn(a[0], v.x);
+    a[1] = __fadd_rn(a[1], v.y);
+  }
+};
+template <>
+struct BpVec<4> {
+  using T = float4;
+  static __device__ __forceinline__ void add(float (&a)[4], float4 v) {
+    a[0] = __fadd_rn(a[0], v.x);
+    a[1] = __fadd_rn(a[1], v.y);
+    a[2] = __fadd_rn(a[2], v.z);
+    a[3] = __fadd_rn(a[3], v.w);
+  }
+};
+
+template <int S, int R, bool kInside>
+__device__ __forceinline__ void bp_angles(const typename BpVec<S>::T* f, const float2* cs, int n,
+                                          int n_ang, float h, float x, const float (&y)[R],
+                                          float (&acc)[R][S]) {
+  using T = typename BpVec<S>::T;
+  // the bits of t + 2^23 are 0x4b000000 + floor(t): the offset goes into the row pointer
+  const char* row = reinterpret_cast<const char*>(f) - (size_t)0x4b000000u * sizeof(T);
+#pragma unroll 4
+  for (int a = 0; a < n_ang; ++a, row += (size_t)n * sizeof(T)) {
+    const float2 c = cs[a];  // (cos, sin)
+    const float xc = __fmul_rn(x, c.x);
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const float r = __fadd_rn(xc, __fmul_rn(y[i], c.y));
+      const float t = __fmul_rn(__fadd_rn(r, 1.f), h);
+      unsigned k = __float_as_uint(__fadd_rz(t, 8388608.f));
+      if (!kInside) {
+        // r just below 1 can round (r + 1) n/2 up to n; the reference then reads
+        // the next row (or past its buffer), here the last sample of the row
+        if (!(r >= -1.f && r < 1.f)) continue;
+        k = min(k, 0x4b000000u + (unsigned)(n - 1));
+      }
+      BpVec<S>::add(acc[i], __ldg(reinterpret_cast<const T*>(row + (size_t)k * sizeof(T))));
     }
   }
-  recon[((size_t)s * n + yi) * n + xi] = acc;
 }
+
+template <int S, int R>
+__global__ void __launch_bounds__(kBpThreads) fbp_backproject_kernel(const float* filt,
+                                                                     const float2* cs,
+                                                                     float* recon, int n,
+                                                                     int n_ang, bool finite) {
+  extern __shared__ float2 s_cs[];
+  for (int i = threadIdx.x; i < n_ang; i += kBpThreads) s_cs[i] = cs[i];
+  __syncthreads();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int xi = blockIdx.x * kBpTile + (warp & 3) * 8 + (lane & 7);
+  const int yi = blockIdx.y * (8 * R) + (warp >> 2) * 4 + (lane >> 3);
+  const float h = (float)n / 2.0f;
+  const float x = __fdiv_rn(__fsub_rn((float)xi, h), h);
+  float y[R], acc[R][S];
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    y[i] = __fdiv_rn(__fsub_rn((float)(yi + 8 * i), h), h);
+#pragma unroll
+    for (int s = 0; s < S; ++s) acc[i][s] = 0.f;
+  }
+  // the block's corner farthest from the centre, in units of the half width; 1e-3 covers
+  // the rounding of r and of (cos, sin) many times over
+  const float cx = fmaxf(fabsf(blockIdx.x * kBpTile - h), fabsf(blockIdx.x * kBpTile + (kBpTile - 1) - h));
+  const float cy = fmaxf(fabsf(blockIdx.y * (8 * R) - h), fabsf(blockIdx.y * (8 * R) + (8 * R - 1) - h));
+  const bool inside = finite && cx * cx + cy * cy < (1.f - 1e-3f) * (1.f - 1e-3f) * h * h;
+  const typename BpVec<S>::T* f =
+      reinterpret_cast<const typename BpVec<S>::T*>(filt) + (size_t)blockIdx.z * n_ang * n;
+  if (inside) bp_angles<S, R, true>(f, s_cs, n, n_ang, h, x, y, acc);
+  else bp_angles<S, R, false>(f, s_cs, n, n_ang, h, x, y, acc);
+  if (xi >= n) return;
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    if (yi + 8 * i >= n) break;
+#pragma unroll
+    for (int s = 0; s < S; ++s)
+      recon[(((size_t)blockIdx.z * S + s) * n + yi + 8 * i) * n + xi] = acc[i][s];
+  }
+}
+
+template <int S, int R>
+cudaError_t launch_backproject_r(const float* filt, const float2* cs, float* recon, int n, int n_ang,
+                                 bool finite, int groups, int smem, cudaStream_t st) {
+  if (smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(fbp_backproject_kernel<S, R>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+  }
+  const dim3 grid((n + kBpTile - 1) / kBpTile, (n + 8 * R - 1) / (8 * R), groups);
+  fbp_backproject_kernel<S, R><<<grid, kBpThreads, smem, st>>>(filt, cs, recon, n, n_ang, finite);
+  return cudaGetLastError();
+}
+
+// Four rows per thread where that leaves four blocks per SM, else one (us for 4 / 1 rows:
+// 2 slices of 2048 x 1500 2893 / 3656, of 1024 x 720 468 / 481, of 512 x 360 122 / 81, of
+// 256 x 180 70 / 27).
+template <int S>
+cudaError_t launch_backproject(const float* filt, const float2* cs, float* recon, int n, int n_ang,
+                               bool finite, int groups, int smem, cudaStream_t st) {
+  const long t = (n + kBpTile - 1) / kBpTile;
+  return t * t * groups >= 4 * 148
+             ? launch_backproject_r<S, 4>(filt, cs, recon, n, n_ang, finite, groups, smem, st)
+             : launch_backproject_r<S, 1>(filt, cs, recon, n, n_ang, finite, groups, smem, st);
+}
+
+// Slices backprojected together: 4, then 2, then 1 of what is left of a call's chunk.
+int bp_group(int slices) { return slices >= 4 ? 4 : (slices >= 2 ? 2 : 1); }
 
 }  // namespace
 }  // namespace gr
 
 struct gr_fbp {
   int device = 0, n = 0, n_ang = 0, max_slices = 1;
+  bool finite = true;  // every angle is a number: |r| is bounded by the pixel's radius
   float* d_lut = nullptr;
   float2* d_tw = nullptr;
   float2* d_cs = nullptr;
@@ -116,6 +220,7 @@ int gr_fbp_create(int n_det, int n_ang, const float* theta_deg, int max_slices, 
   p->n = n;
   p->n_ang = n_ang;
   p->max_slices = max_slices;
+  for (const float2& c : cs) p->finite = p->finite && std::isfinite(c.x) && std::isfinite(c.y);
   cudaError_t e = cudaMalloc(&p->d_lut, n * sizeof(float));
   if (e == cudaSuccess) e = cudaMalloc(&p->d_tw, tw.size() * sizeof(float2));
   if (e == cudaSuccess) e = cudaMalloc(&p->d_cs, n_ang * sizeof(float2));
@@ -142,22 +247,21 @@ int gr_fbp_reconstruct(gr_fbp* f, const float* sinos, int n_slices, float* recon
   const int n = f->n;
   const size_t slice_in = (size_t)f->n_ang * n, slice_out = (size_t)n * n;
   const int smem_bp = f->n_ang * (int)sizeof(float2);
-  if (smem_bp > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(fbp_backproject_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bp);
-    if (e != cudaSuccess) return fail(GR_ERR_UNSUPPORTED, "fbp: %d angles: %s", f->n_ang,
-                                      cudaGetErrorString(e));
-  }
-  for (int s0 = 0; s0 < n_slices; s0 += f->max_slices) {
-    const int ns = std::min(f->max_slices, n_slices - s0);
-    FbpFilterArgs fa{sinos + s0 * slice_in, f->d_filt, f->d_lut, f->d_tw, n, f->n_ang, ns};
+  for (int s0 = 0; s0 < n_slices;) {
+    // whole groups of one size, as many as the filtered-row buffer holds
+    const int S = bp_group(std::min(f->max_slices, n_slices - s0));
+    const int groups = std::min(f->max_slices, n_slices - s0) / S;
+    FbpFilterArgs fa{sinos + s0 * slice_in, f->d_filt, f->d_lut, f->d_tw, n, f->n_ang, groups * S, S};
     cudaError_t e = launch_fbp_filter(fa, st);
     if (e != cudaSuccess) return fail(GR_ERR_CUDA, "fbp filter: %s", cudaGetErrorString(e));
-    dim3 grid((n + kBpX - 1) / kBpX, (n + kBpY - 1) / kBpY, ns);
-    fbp_backproject_kernel<<<grid, dim3(kBpX, kBpY), smem_bp, st>>>(
-        f->d_filt, f->d_cs, recons + s0 * slice_out, n, f->n_ang);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return fail(GR_ERR_CUDA, "fbp backprojection: %s", cudaGetErrorString(e));
+    float* out = recons + s0 * slice_out;
+    e = S == 4 ? launch_backproject<4>(f->d_filt, f->d_cs, out, n, f->n_ang, f->finite, groups, smem_bp, st)
+        : S == 2 ? launch_backproject<2>(f->d_filt, f->d_cs, out, n, f->n_ang, f->finite, groups, smem_bp, st)
+                 : launch_backproject<1>(f->d_filt, f->d_cs, out, n, f->n_ang, f->finite, groups, smem_bp, st);
+    if (e != cudaSuccess)
+      return fail(smem_bp > 48 * 1024 ? GR_ERR_UNSUPPORTED : GR_ERR_CUDA, "fbp: %d angles: %s",
+                  f->n_ang, cudaGetErrorString(e));
+    s0 += groups * S;
   }
   return GR_OK;
 }

@@ -2097,12 +2097,13 @@ __global__ void __launch_bounds__(MAXT, 1024 / MAXT) fbp_filter_kernel(FbpFilter
   for (int r = 0; r < 16; ++r) v[r] = buf[swz(tid + r * nthr)];
   __syncthreads();
   fft_line<-1, NT>(v, buf, n, tid, nthr, tw, tw + 64);
-  float* ya = a.filt + ((size_t)s * a.n_ang + ra) * n;
+  const int grp = a.group;
+  float* ya = a.filt + ((size_t)(s / grp) * a.n_ang + ra) * n * grp + s % grp;
 #pragma unroll
   for (int idx = 0; idx < 16; ++idx) {
     const int k = tid + nthr * out_index(idx, Rl);
-    ya[k] = v[idx].x;
-    if (xb) ya[n + k] = v[idx].y;
+    ya[(size_t)k * grp] = v[idx].x;
+    if (xb) ya[(size_t)(n + k) * grp] = v[idx].y;
   }
 }
 
