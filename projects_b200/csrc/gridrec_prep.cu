@@ -57,11 +57,12 @@ __device__ __forceinline__ double block_sum_d(double v, double* red) {
 //   x_ij <- v_ij - coeff t_j  where positive, else 0
 // Two launches per round: the row update fused with the next round's row means
 // and column partial sums over chunks of rows, then the column means.  The
-// first round's partials come from a column pass over the input.  The
+// first round's partials come from a pass over the input.  The
 // renormalised value is formed as (x g) / r in float, the reference's expression.
 
-// Rows per chunk of the column passes (32: measured fastest of 4..32 at
-// 16 x 2048 x 1500; more row chunks add partial-sum traffic, fewer leave SMs idle).
+// Rows per chunk of the column passes over rows wider than 4096 or not made of aligned
+// 16-byte pieces (32: measured fastest of 4..32 at 16 x 2048 x 1500; more row chunks add
+// partial-sum traffic, fewer leave SMs idle).
 constexpr int kRingRows = 32;
 
 int ring_chunks(int n_ang) { return (n_ang + kRingRows - 1) / kRingRows; }
@@ -86,10 +87,21 @@ __device__ __forceinline__ float slice_gmean(const float* rm, int n_ang, float* 
   return g_s;
 }
 
+// Whether some chunk of slice s has a row of mean 0 that is not all zero (flags: one per
+// chunk of every slice).  Called by the whole block.
+__device__ __forceinline__ bool slice_flagged(const int* flags, int R) {
+  bool f = false;
+  for (int q = threadIdx.x; q < R; q += blockDim.x) f = f || flags[q] != 0;
+  return __syncthreads_or(f);
+}
+
+// flags given: only for slices with a flagged chunk (the others' partials are there).
 __global__ void ring_colpart_kernel(const float* data, const float* rowmean, float* part,
-                                    float* gmean, int n_det, int n_ang, int rows_per_chunk) {
+                                    float* gmean, int n_det, int n_ang, int rows_per_chunk,
+                                    const int* flags) {
   __shared__ float red[32];
   const int r = blockIdx.y, s = blockIdx.z, R = gridDim.y;
+  if (flags && !slice_flagged(flags + (size_t)s * R, R)) return;
   const float* rm = rowmean + (size_t)s * n_ang;
   const float g = slice_gmean(rm, n_ang, red);
   if (threadIdx.x == 0 && blockIdx.x == 0 && r == 0) gmean[s] = g;
@@ -106,33 +118,39 @@ __global__ void ring_colpart_kernel(const float* data, const float* rowmean, flo
   part[((size_t)s * R + r) * n_det + j] = acc;
 }
 
-// Column means c_j = g / n_ang * sum_q part[q][j] (32 columns x 8 chunk
+// Column means c_j = g / n_ang * sum_q part[q][j] (32 columns x 16 chunk
 // strides per block).  scaled = 1: partials already include g (first round,
 // sums of v); scaled = 0: partials are sums of x / r_i and g, the mean of the
-// row means, is formed here and recorded for the next update.
-__global__ void __launch_bounds__(256) ring_colmean_kernel(const float* part, const float* rowmean,
+// row means, is formed here and recorded for the next update.  flags given: scaled for
+// the slices that ring_colpart_kernel did.
+constexpr int kColStrides = 16;
+
+__global__ void __launch_bounds__(32 * kColStrides) ring_colmean_kernel(const float* part, const float* rowmean,
                                                           float* colmean, float* gmean, int n_det,
-                                                          int n_ang, int R, int scaled) {
+                                                          int n_ang, int R, int scaled,
+                                                          const int* flags) {
   __shared__ float red[32];
-  __shared__ float acc_s[8][33];
+  __shared__ float acc_s[kColStrides][33];
   const int s = blockIdx.y;
   float g = 1.f;
+  if (flags) scaled = slice_flagged(flags + (size_t)s * R, R);
   if (!scaled) {
     g = slice_gmean(rowmean + (size_t)s * n_ang, n_ang, red);
-    if (threadIdx.x == 0 && threadIdx.y == 0 && blockIdx.x == 0) gmean[s] = g;
+    if (threadIdx.x == 0 && blockIdx.x == 0) gmean[s] = g;
   }
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int j = blockIdx.x * 32 + tx;
   float acc = 0.f;
   if (j < n_det) {
     const float* p = part + (size_t)s * R * n_det + j;
-    for (int q = ty; q < R; q += 8) acc += p[(size_t)q * n_det];
+#pragma unroll 4
+    for (int q = ty; q < R; q += kColStrides) acc += p[(size_t)q * n_det];
   }
   acc_s[ty][tx] = acc;
   __syncthreads();
   if (ty == 0 && j < n_det) {
     float c = 0.f;
-    for (int q = 0; q < 8; ++q) c += acc_s[q][tx];
+    for (int q = 0; q < kColStrides; ++q) c += acc_s[q][tx];
     colmean[(size_t)s * n_det + j] = c * g / n_ang;
   }
 }
@@ -232,6 +250,172 @@ __global__ void __launch_bounds__(kPrepThreads) ring_round_kernel(
   for (int k = 0; k < KPT; ++k) {
     const int j = threadIdx.x + k * kPrepThreads;
     if (j < n_det) part[((size_t)s * R + r) * n_det + j] = acc[k];
+  }
+}
+
+// a / b correctly rounded for every a that is 0 or in [kDivLo, 2^100] and b in
+// [2^-40, 2^40], with y = RN(1 / b): RN(a y) is within 2 ulp of a / b, one residual step
+// brings it within 1 ulp, and a second one rounds correctly (Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", 1990; the residuals are
+// exact in this range).  One reciprocal serves a row.
+constexpr float kDivLo = 0x1p-60f;
+__device__ __forceinline__ float div_by(float a, float b, float y) {
+  float q = __fmul_rn(a, y);
+  q = __fmaf_rn(__fmaf_rn(-q, b, a), y, q);
+  return __fmaf_rn(__fmaf_rn(-q, b, a), y, q);
+}
+
+// Threads of a block for rows of n_det, and blocks per SM at the kernel's registers.
+constexpr int ring_threads(int n_det) { return n_det <= 2048 ? 128 : 256; }
+constexpr int ring_blocks(int threads) { return threads == 128 ? 5 : 2; }
+
+// The same round on rows of whole aligned 16-byte pieces: thread t of NT owns the pieces
+// t, t + NT, ... of a row (KV of them), so a row of 2048 costs four loads and four stores
+// per thread, the work per row (means, reciprocals, exchanges) is shared by 16 samples
+// of a thread, and rows whose mean and data are in div_by's range divide by one
+// reciprocal.  kFirst: the data may be negative (the first round), where the row mean
+// does not bound the samples and every division is the general one.  kStart: no update,
+// only the input's row means and column partials, with a flag per chunk for a row of mean
+// 0 that is not all zero (its samples enter the column means unscaled: the general
+// column pass redoes such slices).
+// Bound: DRAM once a call's slices exceed L2, then issue (50 % active).  16 slices of
+// 2048 x 1500: 62 us per round for 393 MB read and written against 101 us for the scalar
+// kernel (32 instructions per sample there, 17 here); 20 rounds 2.40 -> 1.48 ms with the
+// start pass (38 us for two passes of 97 and 109) and the backward rounds (65 -> 62 us per
+// round, part of the data still being in L2).  One slice 0.88 -> 0.36 ms.  256 threads of
+// half the pieces cost 74 us per round, groups of slices that fit L2 more than one wave
+// of all slices (80 MB groups 2.30 ms for the call).
+enum RingMode { kStart, kFirst, kLater };
+template <int NT, int KV, int RB, RingMode kMode>
+__global__ void __launch_bounds__(NT, ring_blocks(NT)) ring_round_vec_kernel(
+    float* data, float* rowmean, const float* colmean, const float* gmean, float* part, int n_det,
+    int n_ang, int rows_per_chunk, float coeff, bool backward, int* flags) {
+  constexpr int NW = NT / 32;
+  __shared__ __align__(16) float red[2][RB][NW];
+  const int r = blockIdx.x, s = blockIdx.y, R = gridDim.x;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const float g = kMode == kStart ? 0.f : gmean[s];
+  const float* c = colmean + (size_t)s * n_det;
+  float d[KV][4], acc[KV][4];
+  bool odd_row = false;
+#pragma unroll
+  for (int k = 0; k < KV; ++k)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int j = 4 * (threadIdx.x + k * NT) + e;
+      float t = 0.f;
+      if (kMode != kStart && j > 0 && j < n_det - 1) t = c[j] - (c[j - 1] + c[j] + c[j + 1]) / 3.f;
+      d[k][e] = __fmul_rn(t, coeff);
+      acc[k][e] = 0.f;
+    }
+  float* rm = rowmean + (size_t)s * n_ang;
+  const int i0 = r * rows_per_chunk, i1 = min(n_ang, i0 + rows_per_chunk);
+  const bool g_ok = !(kMode != kLater) && g >= 0x1p-40f && g <= 0x1p40f;
+  // odd rounds walk the rows backwards: what the previous round wrote last is in L2
+  const int nb = (i1 - i0 + RB - 1) / RB;
+  int buf = 0;
+  for (int t = 0; t < nb; ++t, buf ^= 1) {
+    const int ib = i0 + (backward ? nb - 1 - t : t) * RB;
+    float4 y[RB][KV];
+    float ri[RB], sum[RB];
+    // all loads of the RB rows first, so they are in flight together
+#pragma unroll
+    for (int b = 0; b < RB; ++b) {
+      const int i = ib + b;
+      ri[b] = kMode != kStart && i < i1 ? rm[i] : 0.f;
+      const float4* row = reinterpret_cast<const float4*>(data + ((size_t)s * n_ang + i) * n_det);
+#pragma unroll
+      for (int k = 0; k < KV; ++k) {
+        const int q = threadIdx.x + k * NT;
+        y[b][k] = (i < i1 && 4 * q < n_det) ? row[q] : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    }
+#pragma unroll
+    for (int b = 0; b < RB; ++b) {
+      const int i = ib + b;
+      sum[b] = 0.f;
+      float4* row = reinterpret_cast<float4*>(data + ((size_t)s * n_ang + i) * n_det);
+      // data >= 0: no sample exceeds n_det times its row's mean
+      const bool fast = g_ok && ri[b] >= 0x1p-40f && ri[b] <= 0x1p40f;
+      const float inv = __frcp_rn(fast ? ri[b] : 1.f);
+#pragma unroll
+      for (int k = 0; k < KV; ++k) {
+        const int q = threadIdx.x + k * NT;
+        float* x = reinterpret_cast<float*>(&y[b][k]);
+        if (kMode == kStart) {
+          sum[b] += (x[0] + x[1]) + (x[2] + x[3]);
+          continue;
+        }
+        float v[4];
+        bool ok = fast;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float a = __fmul_rn(x[e], g);
+          v[e] = div_by(a, ri[b], inv);
+          ok = ok && __float_as_uint(a) - 1u >= __float_as_uint(kDivLo) - 1u;  // 0 or >= kDivLo
+        }
+        if (!ok) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e)  // zeros as in ring_round_kernel
+            v[e] = (ri[b] != 0.f && x[e] != 0.f) ? __fdiv_rn(__fmul_rn(x[e], g), ri[b]) : x[e];
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          x[e] = fmaxf(__fsub_rn(v[e], d[k][e]), 0.f);  // NaN gives 0, as z > 0 ? z : 0
+        }
+        if (i < i1 && 4 * q < n_det) {
+          row[q] = y[b][k];
+          sum[b] += (x[0] + x[1]) + (x[2] + x[3]);
+        }
+      }
+    }
+#pragma unroll
+    for (int b = 0; b < RB; ++b) {
+      float v = sum[b];
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (lane == 0) red[buf][b][w] = v;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int b = 0; b < RB; ++b) {
+      float tot = 0.f;
+#pragma unroll
+      for (int q = 0; q < NW; q += 4) {
+        const float4 p = *reinterpret_cast<const float4*>(&red[buf][b][q]);
+        tot += (p.x + p.y) + (p.z + p.w);
+      }
+      const float rn = tot / n_det;
+      const int i = ib + b;
+      if (i < i1) {
+        if (threadIdx.x == 0) rm[i] = rn;
+        if (kMode == kStart && rn == 0.f) {
+#pragma unroll
+          for (int k = 0; k < KV; ++k)
+            odd_row = odd_row || y[b][k].x != 0.f || y[b][k].y != 0.f || y[b][k].z != 0.f || y[b][k].w != 0.f;
+        }
+        if (rn != 0.f) {
+          const float inv = 1.f / rn;
+#pragma unroll
+          for (int k = 0; k < KV; ++k) {
+            acc[k][0] += y[b][k].x * inv;
+            acc[k][1] += y[b][k].y * inv;
+            acc[k][2] += y[b][k].z * inv;
+            acc[k][3] += y[b][k].w * inv;
+          }
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < KV; ++k) {
+    const int q = threadIdx.x + k * NT;
+    if (4 * q < n_det)
+      reinterpret_cast<float4*>(part + ((size_t)s * R + r) * n_det)[q] =
+          make_float4(acc[k][0], acc[k][1], acc[k][2], acc[k][3]);
+  }
+  if (kMode == kStart) {
+    const bool any = __syncthreads_or(odd_row);
+    if (threadIdx.x == 0) flags[(size_t)s * R + r] = any;
   }
 }
 
@@ -686,6 +870,33 @@ void launch_ring_round(dim3 grid, cudaStream_t st, float* x, float* rm, const fl
   ring_round_kernel<KPT, RB><<<grid, kPrepThreads, 0, st>>>(x, rm, c, g, part, n_det, n_ang,
                                                             kRingRows, coeff);
 }
+
+// round -1: the start pass.
+template <int NT, int KV, int RB>
+void launch_ring_round_vec(int round, int rows, dim3 grid, cudaStream_t st, float* x, float* rm,
+                           const float* c, const float* g, float* part, int n_det, int n_ang,
+                           float coeff, int* flags) {
+  if (round < 0)
+    ring_round_vec_kernel<NT, KV, RB, kStart><<<grid, NT, 0, st>>>(x, rm, c, g, part, n_det, n_ang,
+                                                                   rows, coeff, false, flags);
+  else if (round == 0)
+    ring_round_vec_kernel<NT, KV, RB, kFirst><<<grid, NT, 0, st>>>(x, rm, c, g, part, n_det, n_ang,
+                                                                   rows, coeff, true, flags);
+  else
+    ring_round_vec_kernel<NT, KV, RB, kLater><<<grid, NT, 0, st>>>(
+        x, rm, c, g, part, n_det, n_ang, rows, coeff, (round & 1) == 0, flags);
+}
+
+constexpr int kRingRB = 2;  // rows at once at 2048 and 4096 columns, twice that below
+
+// Rows per chunk on rows of whole 16-byte pieces: one wave of blocks over the GPU, in
+// equal chunks of whole row groups.
+int ring_rows_vec(int n_slices, int n_det, int n_ang) {
+  const long waves = ring_blocks(ring_threads(n_det)) * 148L;
+  const int rows = (int)(((long)n_ang * n_slices + waves - 1) / waves);
+  const int chunks = (n_ang + rows - 1) / rows;
+  return ((n_ang + chunks - 1) / chunks + 2 * kRingRB - 1) / (2 * kRingRB) * (2 * kRingRB);
+}
 }  // namespace
 }  // namespace gr
 
@@ -695,11 +906,11 @@ extern "C" {
 
 size_t gr_ring_workspace_bytes(int n_slices, int n_det, int n_ang) {
   if (n_slices < 1 || n_det < 1 || n_ang < 1) return 0;
-  const int R = ring_chunks(n_ang);
-  const size_t floats = (size_t)n_slices * ((size_t)n_ang + (size_t)R * n_det + n_det + 1);
+  const int rows = std::min(kRingRows, ring_rows_vec(n_slices, n_det, n_ang));
+  const size_t R = (n_ang + rows - 1) / rows;  // chunk partials of either kind of rows
+  const size_t floats = (size_t)n_slices * ((size_t)n_ang + R * (n_det + 1) + n_det + 1) + 4;
   return floats * sizeof(float);
 }
-
 
 int gr_ring_removal(float* sinos, int n_slices, int n_det, int n_ang, float ring_coeff,
                     int iterations, void* workspace, void* stream) {
@@ -709,13 +920,17 @@ int gr_ring_removal(float* sinos, int n_slices, int n_det, int n_ang, float ring
                             "iterations >= 0");
   if (iterations == 0) return GR_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  const int R = ring_chunks(n_ang);
-  float* rowmean = static_cast<float*>(workspace);
-  float* part = rowmean + (size_t)n_slices * n_ang;
-  float* colmean = part + (size_t)n_slices * R * n_det;
-  float* gmean = colmean + (size_t)n_slices * n_det;
   const int bx = (n_det + kPrepThreads - 1) / kPrepThreads;
   const int cx = (n_det + 31) / 32;
+  const int cthreads = 32 * kColStrides;
+  const bool vec = bx <= 16 && n_det % 4 == 0 && (reinterpret_cast<uintptr_t>(sinos) & 15) == 0;
+  const int rows = vec ? ring_rows_vec(n_slices, n_det, n_ang) : kRingRows;
+  const int R = (n_ang + rows - 1) / rows;
+  // the chunk partials first, on a 16-byte boundary
+  float* part = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(workspace) + 15) & ~uintptr_t(15));
+  float* rowmean = part + (size_t)n_slices * R * n_det;
+  float* colmean = rowmean + (size_t)n_slices * n_ang;
+  float* gmean = colmean + (size_t)n_slices * n_det;
   const int kpt = bx <= 1 ? 1 : bx <= 2 ? 2 : bx <= 4 ? 4 : bx <= 8 ? 8 : 16;
   const bool fused = bx <= 16;
   {
@@ -725,12 +940,30 @@ int gr_ring_removal(float* sinos, int n_slices, int n_det, int n_ang, float ring
     float* pt = part;
     float* cm = colmean;
     float* gm = gmean;
-    ring_rowmean_kernel<<<dim3(n_ang, ns), kPrepThreads, 0, st>>>(x, rm, n_det, n_ang);
-    ring_colpart_kernel<<<dim3(bx, R, ns), kPrepThreads, 0, st>>>(x, rm, pt, gm, n_det, n_ang,
-                                                                  kRingRows);
-    ring_colmean_kernel<<<dim3(cx, ns), 256, 0, st>>>(pt, rm, cm, gm, n_det, n_ang, R, 1);
+    int* flags = reinterpret_cast<int*>(gmean + n_slices);
+    auto vec_round = [&](int m) {
+      const dim3 grid(R, ns);
+      auto* fn = n_det <= 512    ? launch_ring_round_vec<128, 1, 2 * kRingRB>
+                 : n_det <= 1024 ? launch_ring_round_vec<128, 2, 2 * kRingRB>
+                 : n_det <= 2048 ? launch_ring_round_vec<128, 4, kRingRB>
+                                 : launch_ring_round_vec<256, 4, kRingRB>;
+      fn(m, rows, grid, st, x, rm, cm, gm, pt, n_det, n_ang, ring_coeff, flags);
+    };
+    if (vec) {
+      vec_round(-1);
+    } else {
+      ring_rowmean_kernel<<<dim3(n_ang, ns), kPrepThreads, 0, st>>>(x, rm, n_det, n_ang);
+      flags = nullptr;
+    }
+    ring_colpart_kernel<<<dim3(bx, R, ns), kPrepThreads, 0, st>>>(x, rm, pt, gm, n_det, n_ang, rows,
+                                                                  flags);
+    ring_colmean_kernel<<<dim3(cx, ns), cthreads, 0, st>>>(pt, rm, cm, gm, n_det, n_ang, R, 1, flags);
     for (int m = 0; m < iterations; ++m) {
-      if (fused) {
+      if (vec) {
+        vec_round(m);
+        if (m + 1 < iterations)
+          ring_colmean_kernel<<<dim3(cx, ns), cthreads, 0, st>>>(pt, rm, cm, gm, n_det, n_ang, R, 0, nullptr);
+      } else if (fused) {
         const dim3 grid(R, ns);
         switch (kpt) {
           case 1: launch_ring_round<1, 4>(grid, st, x, rm, cm, gm, pt, n_det, n_ang, ring_coeff); break;
@@ -740,13 +973,14 @@ int gr_ring_removal(float* sinos, int n_slices, int n_det, int n_ang, float ring
           default: launch_ring_round<16, 2>(grid, st, x, rm, cm, gm, pt, n_det, n_ang, ring_coeff);
         }
         if (m + 1 < iterations)
-          ring_colmean_kernel<<<dim3(cx, ns), 256, 0, st>>>(pt, rm, cm, gm, n_det, n_ang, R, 0);
+          ring_colmean_kernel<<<dim3(cx, ns), cthreads, 0, st>>>(pt, rm, cm, gm, n_det, n_ang, R, 0, nullptr);
       } else {
         // Rows wider than 4096: separate update and column passes.
         if (m > 0) {
           ring_colpart_kernel<<<dim3(bx, R, ns), kPrepThreads, 0, st>>>(x, rm, pt, gm, n_det,
-                                                                        n_ang, kRingRows);
-          ring_colmean_kernel<<<dim3(cx, ns), 256, 0, st>>>(pt, rm, cm, gm, n_det, n_ang, R, 1);
+                                                                        n_ang, kRingRows, nullptr);
+          ring_colmean_kernel<<<dim3(cx, ns), cthreads, 0, st>>>(pt, rm, cm, gm, n_det, n_ang, R, 1,
+                                                                 nullptr);
         }
         ring_update_kernel<<<dim3(n_ang, ns), kPrepThreads, 0, st>>>(x, rm, cm, gm, n_det, n_ang,
                                                                      ring_coeff);

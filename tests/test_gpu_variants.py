@@ -33,3 +33,32 @@ def test_fbp_groups_same_bits_and_oracle(n, a, S, group):
         ref = O.port_optimized_fbp(sinos[s], th)
         assert ph.rel_l2(got[s], ref) < 1e-5
     one.close()
+
+
+@pytest.mark.parametrize("n,a,S", [(4, 3, 1), (12, 40, 2), (512, 37, 3), (516, 5, 2), (1024, 130, 2),
+                                   (1028, 33, 1), (2048, 70, 3), (2052, 9, 2), (4096, 21, 2),
+                                   (4100, 11, 1)])
+def test_ring_removal_widths_and_row_values(n, a, S):
+    """Widths at the edges of the vector kernels (and one beyond them), with rows that
+    leave the one-reciprocal division: all zero, mean 0 but not zero, samples near the
+    smallest normal float, a row mean above 2^40.  Against the float64 oracle, and the
+    scalar kernels on the same data off its 16-byte alignment."""
+    rng = np.random.default_rng(n + a)
+    x = rng.uniform(0.1, 2.0, (S, a, n)).astype(np.float32)
+    x[rng.uniform(size=x.shape) < 0.04] = 0.0
+    x[0, 0] = 0.0
+    x[-1, 1, ::2], x[-1, 1, 1::2] = 0.5, -0.5  # mean 0
+    x[0, 2, : n // 2] = 2e-38
+    ref = np.stack([O.port_ring_removal(s, 1.0, 5) for s in x])
+    got = G.ring_removal(_dev(x), 1.0, 5)
+    buf = torch.empty(x.size + 1, device="cuda")
+    off = buf[1:].view(x.shape)
+    off.copy_(_dev(x))
+    G.ring_removal(off, 1.0, 5)
+    # FP32 rounds against float64: the bound of the other ring tests
+    assert ph.rel_l2(got.cpu().numpy(), ref) < 2e-5
+    assert ph.rel_l2(off.cpu().numpy(), ref) < 2e-5
+    y = x.copy()
+    y[0, 0] = 2.0 ** 50
+    ref = np.stack([O.port_ring_removal(s, 1.0, 5) for s in y])
+    assert ph.rel_l2(G.ring_removal(_dev(y), 1.0, 5).cpu().numpy(), ref) < 2e-5
