@@ -6,9 +6,9 @@
 // sum accumulates in FP32.  conv2 -- 2304 of the 2592 multiply-adds per pixel --
 // runs on the tensor cores (mma.sync m16n8k16, BF16 in, FP32 accumulate), in the
 // forward pass and, with flipped and transposed weights, for the gradient with
-// respect to its input; the thin 1 -> 16 and 16 -> 1 layers and the weight
-// gradients (sums over all pixels) run on the CUDA cores with fixed-order
-// partial sums, so training is deterministic.
+// respect to its input, and so do the weight gradients (contractions over all pixels);
+// the thin 1 -> 16 and 16 -> 1 layers run on the CUDA cores.  Partial sums are added in
+// a fixed order, so training is deterministic.
 //
 // Parameters: one float32 array of kCnnParams entries:
 //   w1[tap][co] (144), b1 (16), w2[tap][co][ci] (2304), b2 (16), w3[tap][ci] (144), b3 (1)
@@ -242,107 +242,229 @@ __global__ void cnn_conv3_bwd_kernel(const float* params, const float* gy,
   }
 }
 
-// Weight gradients of all three layers over one row segment of kSeg pixels:
-// partial sums of the kCnnParams gradient entries, written to part[segment].
-constexpr int kSeg = 128;
+// Weight gradients of all three layers on the tensor cores, contracted over pixels.
+// A block of 4 warps walks down a strip of kWgW columns, 16 pixels of the row per warp;
+// per row and warp (mma.m16n8k16, K = the 16 pixels q, FP32 accumulators kept for the
+// whole strip segment):
+//   dW2[tap][co][ci] = sum_q gz2[q][co] h1[q + off][ci]   A = gz2^T, B = h1 shifted, 18 MMAs
+//   dW1[tap][co]     = sum_q gz1[q][co] x[q + off]         A = gz1^T, B = x's taps and a one
+//   dW3[tap][ci]     = sum_q gy[q - off] h2[q][ci]         A = gy's taps, B = h2
+//   db2[co] = sum gz2, db1 (the column of ones of dW1's B), db3 = sum gy
+// gz1, gz2, h1 and h2 are BF16 already, so their products are exact; the FP32 operands x
+// and gy enter as three BF16 parts each, which add up to the FP32 value.  Rows arrive by
+// cp.async a row ahead into rings (three rows of h1, x and gy are in use); pixels lie 48
+// bytes apart, so that the eight 16-byte rows of an ldmatrix fall on distinct banks.
+// Bound: the latency of a row's exchanges (one row of 64 pixels per barrier), then DRAM
+// (136 bytes per pixel).  4 x 1024 x 1024: 232 us and 5 us for the reduction of 384 blocks,
+// against 2179 us on the CUDA cores and 1444 us for the reduction of 32768 segments.
+constexpr int kWgW = 64, kWgThreads = 128, kWgBlocks = 3;  // blocks per SM
+constexpr int kWgPx = 48;                                  // bytes between pixels in shared memory
+constexpr int kWgHalo = kWgW + 2;
+struct WgSmem {
+  alignas(16) unsigned char h1[4][kWgHalo * kWgPx];        // ring over rows y - 1 .. y + 2
+  alignas(16) unsigned char g1[2][kWgW * kWgPx], g2[2][kWgW * kWgPx], h2[2][kWgW * kWgPx];
+  float x[4][kWgHalo], gy[4][kWgHalo];
+};
 
-__global__ void __launch_bounds__(256) cnn_wgrad_kernel(const float* x, const float* gy,
-                                                        const __nv_bfloat16* h1,
-                                                        const __nv_bfloat16* h2,
-                                                        const __nv_bfloat16* gz1,
-                                                        const __nv_bfloat16* gz2, float* part,
-                                                        int h, int w, int segs_per_row) {
-  extern __shared__ float sm[];
-  const int W2 = kSeg + 2;
-  float* s_x = sm;                       // [3][W2]
-  float* s_h1 = s_x + 3 * W2;            // [3][W2][16]
-  float* s_h2 = s_h1 + 3 * W2 * kC;      // [3][W2][16]
-  float* s_gz1 = s_h2 + 3 * W2 * kC;     // [kSeg][16]
-  float* s_gz2 = s_gz1 + kSeg * kC;      // [kSeg][16]
-  float* s_gy = s_gz2 + kSeg * kC;       // [kSeg]
-  const int seg = blockIdx.x % segs_per_row, yi = blockIdx.x / segs_per_row, im = blockIdx.y;
-  const int x0 = seg * kSeg;
-  const size_t img = (size_t)im * h * w;
-  for (int i = threadIdx.x; i < 3 * W2; i += blockDim.x) {
-    const int r = i / W2, c = i % W2;
-    const int yy = yi + r - 1, xx = x0 + c - 1;
-    const bool ok = yy >= 0 && yy < h && xx >= 0 && xx < w;
-    const size_t p = img + (size_t)yy * w + xx;
-    s_x[i] = ok ? x[p] : 0.f;
-    for (int ch = 0; ch < kC; ++ch) {
-      s_h1[i * kC + ch] = ok ? __bfloat162float(h1[p * kC + ch]) : 0.f;
-      s_h2[i * kC + ch] = ok ? __bfloat162float(h2[p * kC + ch]) : 0.f;
-    }
-  }
-  for (int i = threadIdx.x; i < kSeg; i += blockDim.x) {
-    const int xx = x0 + i;
-    const bool ok = xx < w;
-    const size_t p = img + (size_t)yi * w + xx;
-    s_gy[i] = ok ? gy[p] : 0.f;
-    for (int ch = 0; ch < kC; ++ch) {
-      s_gz1[i * kC + ch] = ok ? __bfloat162float(gz1[p * kC + ch]) : 0.f;
-      s_gz2[i * kC + ch] = ok ? __bfloat162float(gz2[p * kC + ch]) : 0.f;
-    }
-  }
-  __syncthreads();
-  float* out = part + ((size_t)im * gridDim.x + blockIdx.x) * kCnnParams;
-  const int tid = threadIdx.x;
-  // dW2[tap][co][ci] = sum_p gz2[p][co] h1[p + off][ci]; thread = (co, ci), all taps
-  {
-    const int co = tid / kC, ci = tid % kC;
-    float a[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int i = 0; i < kSeg; ++i) {
-      const float gv = s_gz2[i * kC + co];
+static_assert(sizeof(WgSmem) <= 48 * 1024 && sizeof(WgSmem) >= kCnnParams * sizeof(float),
+              "default shared-memory limit; the sums fit over the rings");
+
+// Segments of a strip, so that the blocks fill the GPU about once.
+int wg_segments(int n_img, int h, int w) {
+  const long strips = (long)n_img * ((w + kWgW - 1) / kWgW);
+  return (int)std::max(1L, std::min<long>(h, kWgBlocks * 148L / strips));
+}
+long wg_blocks(int n_img, int h, int w) {
+  return (long)n_img * ((w + kWgW - 1) / kWgW) * wg_segments(n_img, h, w);
+}
+
+__device__ __forceinline__ void cp_async_zfill16(void* dst, const void* src, bool ok) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_u32(dst)), "l"(src),
+               "r"(ok ? 16 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_zfill4(void* dst, const void* src, bool ok) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(smem_u32(dst)), "l"(src),
+               "r"(ok ? 4 : 0)
+               : "memory");
+}
+// Four 8 x 8 BF16 blocks of 16 pixels x 16 channels at `px` (pixel stride kWgPx), transposed:
+// r[0] pixels 0..7 of channels 0..7, r[1] channels 8..15, r[2], r[3] pixels 8..15 -- the
+// A fragment (row = channel, column = pixel) in the order a0 a1 a2 a3, and the B fragments
+// (row = pixel, column = channel) of the channel halves, (r[0], r[2]) and (r[1], r[3]).
+__device__ __forceinline__ void ldm_t(unsigned (&r)[4], const unsigned char* px, int lane) {
+  const unsigned char* p = px + ((lane & 7) + ((lane >> 4) & 1) * 8) * kWgPx + ((lane >> 3) & 1) * 16;
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(smem_u32(p))
+               : "memory");
+}
+// (a, b) as three packed BF16 pairs that sum to the FP32 values
+__device__ __forceinline__ void split3(float a, float b, unsigned (&o)[3]) {
 #pragma unroll
-      for (int tap = 0; tap < 9; ++tap) {
-        const int r = tap / 3, c = i + tap % 3;
-        a[tap] = fmaf(gv, s_h1[(r * W2 + c) * kC + ci], a[tap]);
-      }
-    }
-#pragma unroll
-    for (int tap = 0; tap < 9; ++tap) out[kW2 + (tap * kC + co) * kC + ci] = a[tap];
-  }
-  if (tid < kC) {  // dW1[tap][co] = sum_p gz1[p][co] x[p + off]; db1
-    float a[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, b = 0.f;
-    for (int i = 0; i < kSeg; ++i) {
-      const float gv = s_gz1[i * kC + tid];
-      b += gv;
-#pragma unroll
-      for (int tap = 0; tap < 9; ++tap) a[tap] = fmaf(gv, s_x[(tap / 3) * W2 + i + tap % 3], a[tap]);
-    }
-#pragma unroll
-    for (int tap = 0; tap < 9; ++tap) out[kW1 + tap * kC + tid] = a[tap];
-    out[kB1 + tid] = b;
-  } else if (tid < 2 * kC) {  // db2
-    const int c = tid - kC;
-    float b = 0.f;
-    for (int i = 0; i < kSeg; ++i) b += s_gz2[i * kC + c];
-    out[kB2 + c] = b;
-  } else if (tid < 3 * kC) {  // dW3[tap][ci] = sum_p gy[p] h2[p + off][ci]
-    const int ci = tid - 2 * kC;
-    float a[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int i = 0; i < kSeg; ++i) {
-      const float gv = s_gy[i];
-#pragma unroll
-      for (int tap = 0; tap < 9; ++tap)
-        a[tap] = fmaf(gv, s_h2[((tap / 3) * W2 + i + tap % 3) * kC + ci], a[tap]);
-    }
-#pragma unroll
-    for (int tap = 0; tap < 9; ++tap) out[kW3 + tap * kC + ci] = a[tap];
-  } else if (tid == 3 * kC) {
-    float b = 0.f;
-    for (int i = 0; i < kSeg; ++i) b += s_gy[i];
-    out[kB3] = b;
+  for (int k = 0; k < 3; ++k) {
+    o[k] = pack_bf16(a, b);
+    const float2 h = unpack_bf16(o[k]);
+    a -= h.x;
+    b -= h.y;
   }
 }
 
-// grads[k] = sum over segments (fixed order) of part[seg][k]
-__global__ void cnn_reduce_kernel(const float* part, long nseg, float* grads) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= kCnnParams) return;
+__global__ void __launch_bounds__(kWgThreads, kWgBlocks) cnn_wgrad_kernel(
+    const float* x, const float* gy, const __nv_bfloat16* h1, const __nv_bfloat16* h2,
+    const __nv_bfloat16* gz1, const __nv_bfloat16* gz2, float* part, int h, int w, int segs) {
+  extern __shared__ __align__(16) unsigned char smw[];
+  WgSmem& sm = *reinterpret_cast<WgSmem*>(smw);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int strip = blockIdx.x / segs, seg = blockIdx.x - strip * segs, im = blockIdx.y;
+  const int x0 = strip * kWgW;
+  const int y0 = (int)((long)h * seg / segs), y1 = (int)((long)h * (seg + 1) / segs);
+  const size_t img = (size_t)im * h * w;
+  // row y with a pixel of halo on both sides: h1, x and gy
+  auto load_halo_row = [&](int y) {
+    const int slot = y & 3;
+    const bool row = y >= 0 && y < h;
+    for (int i = tid; i < 2 * kWgHalo; i += kWgThreads) {
+      const int c = i >> 1, xx = x0 + c - 1;
+      const bool ok = row && xx >= 0 && xx < w;
+      const size_t p = ok ? img + (size_t)y * w + xx : 0;
+      cp_async_zfill16(sm.h1[slot] + c * kWgPx + (i & 1) * 16,
+                       reinterpret_cast<const unsigned char*>(h1) + p * 32 + (i & 1) * 16, ok);
+      if (i & 1) cp_async_zfill4(&sm.x[slot][c], x + p, ok);
+      else cp_async_zfill4(&sm.gy[slot][c], gy + p, ok);
+    }
+  };
+  // row y without halo: gz1, gz2 and h2
+  auto load_row = [&](int y) {
+    const int slot = y & 1;
+    for (int i = tid; i < 2 * kWgW; i += kWgThreads) {
+      const int c = i >> 1, xx = x0 + c;
+      const bool ok = y < h && xx < w;
+      const size_t p = (ok ? img + (size_t)y * w + xx : 0) * 32 + (i & 1) * 16;
+      const int o = c * kWgPx + (i & 1) * 16;
+      cp_async_zfill16(sm.g1[slot] + o, reinterpret_cast<const unsigned char*>(gz1) + p, ok);
+      cp_async_zfill16(sm.g2[slot] + o, reinterpret_cast<const unsigned char*>(gz2) + p, ok);
+      cp_async_zfill16(sm.h2[slot] + o, reinterpret_cast<const unsigned char*>(h2) + p, ok);
+    }
+  };
+  float a2[9][2][4], a1[2][4], a3[2][4], ab[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+#pragma unroll
+    for (int n = 0; n < 2; ++n) {
+#pragma unroll
+      for (int tap = 0; tap < 9; ++tap) a2[tap][n][i] = 0.f;
+      a1[n][i] = a3[n][i] = 0.f;
+    }
+    ab[i] = 0.f;
+  }
+  float b3 = 0.f;
+  const unsigned one2 = lane < 4 ? 0x3f803f80u : 0u;  // B column 0 of ones
+  load_halo_row(y0 - 1);
+  load_halo_row(y0);
+  load_halo_row(y0 + 1);
+  load_row(y0);
+  asm volatile("cp.async.commit_group;\n" ::: "memory");
+  const int g = lane >> 2, t = lane & 3;
+  const int q0 = warp * 16;  // this warp's pixels of the row
+  for (int y = y0; y < y1; ++y) {
+    if (y + 1 < y1) {
+      load_halo_row(y + 2);
+      load_row(y + 1);
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    __syncthreads();  // row y and its neighbours are there for every thread
+    unsigned fa[4], fb[4];
+    ldm_t(fa, sm.g2[y & 1] + q0 * kWgPx, lane);
+    mma_bf16(ab, fa, one2, one2);
+#pragma unroll
+    for (int tap = 0; tap < 9; ++tap) {
+      ldm_t(fb, sm.h1[(y + tap_dy(tap)) & 3] + (q0 + 1 + tap_dx(tap)) * kWgPx, lane);
+      mma_bf16(a2[tap][0], fa, fb[0], fb[2]);
+      mma_bf16(a2[tap][1], fa, fb[1], fb[3]);
+    }
+    // dW1: B column n = tap (n = 9: ones); this lane's columns g and g + 8
+    ldm_t(fa, sm.g1[y & 1] + q0 * kWgPx, lane);
+    {
+      const float* r = sm.x[(y + g / 3 - 1) & 3] + q0 + g % 3;  // x[q + off(g)], halo offset in
+      unsigned lo[3], hi[3];
+      split3(r[2 * t], r[2 * t + 1], lo);
+      split3(r[2 * t + 8], r[2 * t + 9], hi);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) mma_bf16(a1[0], fa, lo[k], hi[k]);
+      const float* r8 = sm.x[(y + 1) & 3] + q0 + 2;             // tap 8
+      split3(r8[2 * t], r8[2 * t + 1], lo);
+      split3(r8[2 * t + 8], r8[2 * t + 9], hi);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const unsigned one = g == 1 && k == 0 ? 0x3f803f80u : 0u;
+        mma_bf16(a1[1], fa, g == 0 ? lo[k] : one, g == 0 ? hi[k] : one);
+      }
+    }
+    // dW3: A row m = tap; this lane's rows g and g + 8 (tap 8 for g = 0)
+    ldm_t(fb, sm.h2[y & 1] + q0 * kWgPx, lane);
+    {
+      const float* r = sm.gy[(y - (g / 3 - 1)) & 3] + q0 + 2 - g % 3;  // gy[q - off(g)]
+      const float* r8 = sm.gy[(y - 1) & 3] + q0;                        // tap 8
+      unsigned lo[3], hi[3], lo8[3], hi8[3];
+      split3(r[2 * t], r[2 * t + 1], lo);
+      split3(r[2 * t + 8], r[2 * t + 9], hi);
+      split3(r8[2 * t], r8[2 * t + 1], lo8);
+      split3(r8[2 * t + 8], r8[2 * t + 9], hi8);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const unsigned a[4] = {lo[k], g == 0 ? lo8[k] : 0u, hi[k], g == 0 ? hi8[k] : 0u};
+        mma_bf16(a3[0], a, fb[0], fb[2]);
+        mma_bf16(a3[1], a, fb[1], fb[3]);
+      }
+      if (lane < 16) b3 += sm.gy[y & 3][q0 + 1 + lane];
+    }
+    __syncthreads();  // the rings' oldest rows are read before they are refilled
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  // the four warps' sums in warp order, in shared memory over the rings
+  float* acc = reinterpret_cast<float*>(smw);
+  for (int o = 16; o > 0; o >>= 1) b3 += __shfl_xor_sync(0xffffffffu, b3, o);
+  for (int k = 0; k < kWgThreads / 32; ++k) {
+    __syncthreads();
+    if (warp != k) continue;
+    auto put = [&](int i, float v) { acc[i] = k == 0 ? v : acc[i] + v; };
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int row = g + (i >> 1) * 8, col = 2 * t + (i & 1);
+#pragma unroll
+      for (int n = 0; n < 2; ++n) {
+#pragma unroll
+        for (int tap = 0; tap < 9; ++tap) put(kW2 + (tap * kC + row) * kC + n * 8 + col, a2[tap][n][i]);
+        const int tap1 = n * 8 + col;                      // a1: row = co, column = tap
+        if (tap1 < 9) put(kW1 + tap1 * kC + row, a1[n][i]);
+        if (tap1 == 9) put(kB1 + row, a1[n][i]);
+        if (row < 9) put(kW3 + row * kC + n * 8 + col, a3[n][i]);  // a3: row = tap, column = ci
+      }
+      if (col == 0) put(kB2 + row, ab[i]);
+    }
+    if (lane == 0) put(kB3, b3);
+  }
+  __syncthreads();
+  float* out = part + ((size_t)im * gridDim.x + blockIdx.x) * kCnnParams;
+  for (int i = tid; i < kCnnParams; i += kWgThreads) out[i] = acc[i];
+}
+
+// grads[k] = sum over blocks (fixed order) of part[block][k], in double: 32 parameters x 8
+// strides per block.
+__global__ void __launch_bounds__(256) cnn_reduce_kernel(const float* part, long nblk, float* grads) {
+  __shared__ double sums[8][32];
+  const int k = blockIdx.x * 32 + (threadIdx.x & 31), q = threadIdx.x >> 5;
   double s = 0.0;
-  for (long i = 0; i < nseg; ++i) s += part[i * kCnnParams + k];
-  grads[k] = (float)s;
+  if (k < kCnnParams)
+    for (long i = q; i < nblk; i += 8) s += part[i * kCnnParams + k];
+  sums[q][threadIdx.x & 31] = s;
+  __syncthreads();
+  if (q == 0 && k < kCnnParams) {
+    for (int i = 1; i < 8; ++i) s += sums[i][threadIdx.x & 31];
+    grads[k] = (float)s;
+  }
 }
 
 __global__ void cnn_adam_kernel(float* params, const float* grads, float* m, float* v, int n,
@@ -745,9 +867,8 @@ int gr_cnn_param_count(void) { return kCnnParams; }
 
 size_t gr_cnn_workspace_bytes(int n_img, int h, int w) {
   const size_t px = (size_t)n_img * h * w;
-  const long segs = (long)n_img * h * ((w + kSeg - 1) / kSeg);
-  // h1, h2, gz1, gz2 (bf16 x 16) + gy (f32) + segment partials + loss partials
-  return 4 * px * kC * 2 + px * 4 + (size_t)segs * kCnnParams * 4 + 1024 * 8 + 1024;
+  // h1, h2, gz1, gz2 (bf16 x 16) + gy (f32) + block partials + loss partials
+  return 4 * px * kC * 2 + px * 4 + (size_t)wg_blocks(n_img, h, w) * kCnnParams * 4 + 1024 * 8 + 1024;
 }
 
 size_t gr_cnn_forward_workspace_bytes(int n_img, int h, int w) {
@@ -785,23 +906,20 @@ int gr_cnn_backward(const float* params, const float* x, const float* y, const f
   __nv_bfloat16* gz1 = h2 + px * kC;
   __nv_bfloat16* gz2 = gz1 + px * kC;
   float* gy = reinterpret_cast<float*>(gz2 + px * kC);
-  const int segs_row = (w + kSeg - 1) / kSeg;
-  const long segs = (long)n_img * h * segs_row;
+  const int segs = wg_segments(n_img, h, w);
+  const long blocks = wg_blocks(n_img, h, w);
   float* part = gy + px;
-  double* lpart = reinterpret_cast<double*>(part + (size_t)segs * kCnnParams);
+  double* lpart = reinterpret_cast<double*>(part + (size_t)blocks * kCnnParams);
   lpart = reinterpret_cast<double*>(((uintptr_t)lpart + 7) & ~(uintptr_t)7);
   const int lblocks = 1024;
   cnn_loss_kernel<<<lblocks, 256, 0, st>>>(y, target, gy, lpart, (long)px);
   const dim3 gp((w + 127) / 128, h, n_img);
   cnn_conv3_bwd_kernel<<<gp, 128, 0, st>>>(params, gy, h2, gz2, h, w);
   cnn_conv2_kernel<<<dim3((w + 64 * kConv2Tiles - 1) / (64 * kConv2Tiles), h, n_img), 128, 0, st>>>(params, gz2, h1, gz1, h, w, 1);
-  const int smem = (3 * (kSeg + 2) * (1 + 2 * kC) + kSeg * (2 * kC + 1)) * (int)sizeof(float);
-  cudaError_t e = cudaFuncSetAttribute(cnn_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       smem);
-  if (e != cudaSuccess) return fail(GR_ERR_CUDA, "cnn wgrad smem: %s", cudaGetErrorString(e));
-  cnn_wgrad_kernel<<<dim3(h * segs_row, n_img), 256, smem, st>>>(x, gy, h1, h2, gz1, gz2, part, h,
-                                                                 w, segs_row);
-  cnn_reduce_kernel<<<(kCnnParams + 255) / 256, 256, 0, st>>>(part, segs, grads);
+  cnn_wgrad_kernel<<<dim3((unsigned)(blocks / n_img), n_img), kWgThreads, sizeof(WgSmem), st>>>(
+      x, gy, h1, h2, gz1, gz2, part, h, w, segs);
+  cnn_reduce_kernel<<<(kCnnParams + 31) / 32, 256, 0, st>>>(part, blocks, grads);
+  cudaError_t e = cudaSuccess;
   if (loss) {
     double lp[lblocks];
     e = cudaMemcpyAsync(lp, lpart, sizeof(lp), cudaMemcpyDeviceToHost, st);

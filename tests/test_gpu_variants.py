@@ -62,3 +62,30 @@ def test_ring_removal_widths_and_row_values(n, a, S):
     y[0, 0] = 2.0 ** 50
     ref = np.stack([O.port_ring_removal(s, 1.0, 5) for s in y])
     assert ph.rel_l2(G.ring_removal(_dev(y), 1.0, 5).cpu().numpy(), ref) < 2e-5
+
+
+@pytest.mark.parametrize("shape", [(1, 4, 5), (1, 1, 70), (1, 3, 65), (3, 9, 64), (2, 70, 127),
+                                   (1, 130, 63), (2, 200, 130)])
+def test_network_gradients_ragged_shapes(shape):
+    """Loss and weight gradients at image sizes around the strip kernels' 64 columns and 16
+    pixels, one row, one segment per row and several rows per segment: the float64 oracle
+    with BF16 activations, the bound of the other gradient test."""
+    from oracle import cnn_oracle as CO
+    from projects_b200 import learned as L
+    rng = np.random.default_rng(sum(shape))
+    p = L.init_params(4)
+    p[144:160] = rng.normal(0, 0.1, 16)
+    p[2464:2480] = rng.normal(0, 0.1, 16)
+    p[2480:] = rng.normal(0, 0.05, 145)
+    x = rng.normal(0, 1, shape).astype(np.float32)
+    t = (x + rng.normal(0, 0.3, shape)).astype(np.float32)
+    net = L.CorrectionNet(p)
+    loss = net.loss_and_grads(_dev(x), _dev(t))
+    g = net.grads.cpu().numpy().astype(np.float64)
+    q = p.astype(np.float64).copy()
+    q[160:2464] = CO._bf16(p[160:2464])
+    ref_loss, ref = CO.loss_and_grads(q, x, t, bf16=True)
+    assert abs(loss - ref_loss) <= 2e-3 * ref_loss
+    for a, b in ((0, 144), (144, 160), (160, 2464), (2464, 2480), (2480, 2624), (2624, 2625)):
+        err = np.linalg.norm(g[a:b] - ref[a:b]) / max(np.linalg.norm(ref[a:b]), 1e-30)
+        assert err < 2e-2, (a, err)
