@@ -43,7 +43,7 @@ __device__ __forceinline__ float2 unpack_bf16(unsigned u) {
 // ---------------------------------------------------------------- conv1 (1 -> 16)
 __global__ void cnn_conv1_kernel(const float* params, const float* x, __nv_bfloat16* h1, int h,
                                  int w) {
-  __shared__ float sp[kB1 + kC];  // w1, b1
+  __shared__ __align__(16) float sp[kB1 + kC];  // w1, b1
   for (int i = threadIdx.x; i < kB1 + kC; i += blockDim.x) sp[i] = params[i];
   __syncthreads();
   const int xi = blockIdx.x * blockDim.x + threadIdx.x, yi = blockIdx.y, im = blockIdx.z;
@@ -57,14 +57,18 @@ __global__ void cnn_conv1_kernel(const float* params, const float* x, __nv_bfloa
   }
   unsigned o[kC / 2];
 #pragma unroll
-  for (int c = 0; c < kC; c += 2) {
-    float z0 = sp[kB1 + c], z1 = sp[kB1 + c + 1];
+  for (int c = 0; c < kC; c += 4) {  // 16-byte weight loads: a quarter of the 4-byte ones
+    float4 z = *reinterpret_cast<const float4*>(sp + kB1 + c);
 #pragma unroll
     for (int tap = 0; tap < 9; ++tap) {
-      z0 = fmaf(sp[kW1 + tap * kC + c], in[tap], z0);
-      z1 = fmaf(sp[kW1 + tap * kC + c + 1], in[tap], z1);
+      const float4 wt = *reinterpret_cast<const float4*>(sp + kW1 + tap * kC + c);
+      z.x = fmaf(wt.x, in[tap], z.x);
+      z.y = fmaf(wt.y, in[tap], z.y);
+      z.z = fmaf(wt.z, in[tap], z.z);
+      z.w = fmaf(wt.w, in[tap], z.w);
     }
-    o[c / 2] = pack_bf16(fmaxf(z0, 0.f), fmaxf(z1, 0.f));
+    o[c / 2] = pack_bf16(fmaxf(z.x, 0.f), fmaxf(z.y, 0.f));
+    o[c / 2 + 1] = pack_bf16(fmaxf(z.z, 0.f), fmaxf(z.w, 0.f));
   }
   uint4* out = reinterpret_cast<uint4*>(h1 + (((size_t)im * h + yi) * w + xi) * kC);
   out[0] = make_uint4(o[0], o[1], o[2], o[3]);
@@ -72,7 +76,7 @@ __global__ void cnn_conv1_kernel(const float* params, const float* x, __nv_bfloa
 }
 
 // ---------------------------------------------------------------- conv2 (16 -> 16), tensor cores
-// One warp: 16 consecutive pixels of a row (the M = 16 rows of the mma) x 16
+// One warp step: 16 consecutive pixels of a row (the M = 16 rows of the mma) x 16
 // output channels (two n = 8 tiles); K = 16 input channels per tap, 9 taps.
 // Fragments of mma.m16n8k16 (g = lane / 4, t = lane % 4): A rows g, g + 8 and
 // columns 2t, 2t + 1, 2t + 8, 2t + 9 (pixel, input channel); B rows (input
@@ -90,85 +94,137 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const unsigned (&a)[4], 
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-constexpr int kConv2Tiles = 4;  // 16-pixel tiles per warp
+// A block of 4 warps walks down a strip of kStW columns, 16 pixels of the row per warp: the
+// three input rows in use lie in a ring in shared memory (pixels kStPx bytes apart, so that
+// the eight 16-byte rows of an ldmatrix fall on distinct banks), filled by cp.async a row
+// ahead, so an input pixel is read once per strip instead of once per tap.  The output
+// goes through shared memory to whole 16-byte stores.  4 x 1024 x 1024: CONV2FIG
+constexpr int kStW = 64, kStThreads = 128, kStBlocks = 4;  // blocks per SM
+constexpr int kStPx = 48;                                  // bytes between pixels in shared memory
+constexpr int kStHalo = kStW + 2;
+struct Conv2Smem {
+  alignas(16) unsigned char in[4][kStHalo * kStPx];        // ring over rows y - 1 .. y + 2
+  alignas(16) unsigned char mask[2][kStW * kStPx];
+  alignas(16) unsigned char out[kStW * kStPx];
+};
 
-__global__ void __launch_bounds__(128) cnn_conv2_kernel(const float* params,
-                                                        const __nv_bfloat16* in,
-                                                        const __nv_bfloat16* mask,
-                                                        __nv_bfloat16* out, int h, int w,
-                                                        int backward) {
-  // B fragments (packed BF16 pairs) of all taps and both output-channel tiles,
-  // built once per block from the FP32 weights: sb[tap][nt][half][lane]
-  __shared__ unsigned sb[9 * 2 * 2 * 32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int e = threadIdx.x; e < 9 * 2 * 2 * 32; e += blockDim.x) {
-    const int ln = e & 31, half = (e >> 5) & 1, nt = (e >> 6) & 1, tap = e >> 7;
-    const int n = nt * 8 + (ln >> 2);       // output channel
-    const int k = 2 * (ln & 3) + 8 * half;  // input channels k, k + 1
-    float w0, w1;
-    if (!backward) {
-      w0 = params[kW2 + (tap * kC + n) * kC + k];
-      w1 = params[kW2 + (tap * kC + n) * kC + k + 1];
-    } else {
-      w0 = params[kW2 + ((8 - tap) * kC + k) * kC + n];
-      w1 = params[kW2 + ((8 - tap) * kC + k + 1) * kC + n];
-    }
-    sb[e] = pack_bf16(w0, w1);
-  }
-  __syncthreads();
+// Segments of a strip, so that `per_sm` blocks per SM fill the GPU about once.
+int strip_segments(int n_img, int h, int w, int per_sm) {
+  const long strips = (long)n_img * ((w + kStW - 1) / kStW);
+  return (int)std::max(1L, std::min<long>(h, per_sm * 148L / strips));
+}
+
+__device__ __forceinline__ void cp_async_zfill16(void* dst, const void* src, bool ok) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_u32(dst)), "l"(src),
+               "r"(ok ? 16 : 0)
+               : "memory");
+}
+
+__global__ void __launch_bounds__(kStThreads, kStBlocks) cnn_conv2_kernel(
+    const float* params, const __nv_bfloat16* in, const __nv_bfloat16* mask, __nv_bfloat16* out,
+    int h, int w, int backward, int segs) {
+  __shared__ Conv2Smem sm;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
-  const int yi = blockIdx.y, im = blockIdx.z;
-  for (int mt = 0; mt < kConv2Tiles; ++mt) {
-  const int x0 = ((blockIdx.x * 4 + warp) * kConv2Tiles + mt) * 16;
-  if (x0 >= w) return;
-  const unsigned* in32 = reinterpret_cast<const unsigned*>(in) + (size_t)im * h * w * (kC / 2);
-  float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-#pragma unroll
-  for (int tap = 0; tap < 9; ++tap) {
-    const int yy = yi + tap_dy(tap);
-    const int xa = x0 + g + tap_dx(tap), xb = xa + 8;
-    const bool row_ok = yy >= 0 && yy < h;
-    const bool oka = row_ok && xa >= 0 && xa < w, okb = row_ok && xb >= 0 && xb < w;
-    const size_t pa = ((size_t)yy * w + xa) * (kC / 2), pb = ((size_t)yy * w + xb) * (kC / 2);
-    unsigned a[4];
-    a[0] = oka ? __ldg(&in32[pa + t]) : 0u;      // row g, channels 2t, 2t+1
-    a[1] = okb ? __ldg(&in32[pb + t]) : 0u;      // row g + 8
-    a[2] = oka ? __ldg(&in32[pa + t + 4]) : 0u;  // row g, channels 2t+8, 2t+9
-    a[3] = okb ? __ldg(&in32[pb + t + 4]) : 0u;
-    const unsigned* b = sb + tap * 128 + lane;
-    mma_bf16(acc[0], a, b[0], b[32]);
-    mma_bf16(acc[1], a, b[64], b[96]);
-  }
-  unsigned* out32 = reinterpret_cast<unsigned*>(out) + (size_t)im * h * w * (kC / 2);
-  const unsigned* m32 =
-      mask ? reinterpret_cast<const unsigned*>(mask) + (size_t)im * h * w * (kC / 2) : nullptr;
+  const int strip = blockIdx.x / segs, seg = blockIdx.x - strip * segs, im = blockIdx.y;
+  const int x0 = strip * kStW;
+  const int y0 = (int)((long)h * seg / segs), y1 = (int)((long)h * (seg + 1) / segs);
+  const size_t img = (size_t)im * h * w;
+  auto load_in = [&](int y) {
+    const bool row = y >= 0 && y < h;
+    for (int i = tid; i < 2 * kStHalo; i += kStThreads) {
+      const int c = i >> 1, xx = x0 + c - 1;
+      const bool ok = row && xx >= 0 && xx < w;
+      const size_t p = ok ? img + (size_t)y * w + xx : 0;
+      cp_async_zfill16(sm.in[y & 3] + c * kStPx + (i & 1) * 16,
+                       reinterpret_cast<const unsigned char*>(in) + p * 32 + (i & 1) * 16, ok);
+    }
+  };
+  auto load_mask = [&](int y) {
+    for (int i = tid; i < 2 * kStW; i += kStThreads) {
+      const int c = i >> 1, xx = x0 + c;
+      const bool ok = y < h && xx < w;
+      const size_t p = (ok ? img + (size_t)y * w + xx : 0) * 32 + (i & 1) * 16;
+      cp_async_zfill16(sm.mask[y & 1] + c * kStPx + (i & 1) * 16,
+                       reinterpret_cast<const unsigned char*>(mask) + p, ok);
+    }
+  };
+  load_in(y0 - 1);
+  load_in(y0);
+  load_in(y0 + 1);
+  if (mask) load_mask(y0);
+  asm volatile("cp.async.commit_group;\n" ::: "memory");
+  // this lane's B fragments (packed BF16 pairs) of all taps and both output-channel tiles
+  unsigned wb[9][2][2];
+  float bias[2][2];
 #pragma unroll
   for (int nt = 0; nt < 2; ++nt) {
-    const int c = nt * 8 + 2 * t;  // output channels c, c + 1
+    const int n = nt * 8 + g;  // output channel
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      const int xi = x0 + g + 8 * half;
-      if (xi >= w) continue;
-      float z0 = acc[nt][2 * half], z1 = acc[nt][2 * half + 1];
-      const size_t po = ((size_t)yi * w + xi) * (kC / 2) + c / 2;
-      if (!backward) {
-        z0 = fmaxf(z0 + __ldg(&params[kB2 + c]), 0.f);
-        z1 = fmaxf(z1 + __ldg(&params[kB2 + c + 1]), 0.f);
-      } else {
-        const float2 m = unpack_bf16(__ldg(&m32[po]));
-        z0 = m.x > 0.f ? z0 : 0.f;
-        z1 = m.y > 0.f ? z1 : 0.f;
+    for (int tap = 0; tap < 9; ++tap)
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const int k = 2 * t + 8 * half;  // input channels k, k + 1
+        const float* p0 = params + kW2 + (backward ? ((8 - tap) * kC + k) * kC + n : (tap * kC + n) * kC + k);
+        wb[tap][nt][half] = pack_bf16(__ldg(p0), __ldg(p0 + (backward ? kC : 1)));
       }
-      out32[po] = pack_bf16(z0, z1);
-    }
+#pragma unroll
+    for (int e = 0; e < 2; ++e) bias[nt][e] = backward ? 0.f : __ldg(&params[kB2 + nt * 8 + 2 * t + e]);
   }
-  }  // tiles
+  const int q0 = warp * 16;
+  const int lrow = (lane & 7) + ((lane >> 3) & 1) * 8, lcol = (lane >> 4) * 16;
+  for (int y = y0; y < y1; ++y) {
+    if (y + 1 < y1) {
+      load_in(y + 2);
+      if (mask) load_mask(y + 1);
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    __syncthreads();  // row y and its neighbours are there for every thread
+    float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll
+    for (int tap = 0; tap < 9; ++tap) {
+      unsigned a[4];
+      asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                   : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3])
+                   : "r"(smem_u32(sm.in[(y + tap_dy(tap)) & 3] + (q0 + 1 + tap_dx(tap) + lrow) * kStPx + lcol))
+                   : "memory");
+      mma_bf16(acc[0], a, wb[tap][0][0], wb[tap][0][1]);
+      mma_bf16(acc[1], a, wb[tap][1][0], wb[tap][1][1]);
+    }
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const int o = (q0 + g + 8 * half) * kStPx + (nt * 8 + 2 * t) * 2;
+        float z0 = acc[nt][2 * half], z1 = acc[nt][2 * half + 1];
+        if (!backward) {
+          z0 = fmaxf(z0 + bias[nt][0], 0.f);
+          z1 = fmaxf(z1 + bias[nt][1], 0.f);
+        } else {
+          const float2 m = unpack_bf16(*reinterpret_cast<const unsigned*>(sm.mask[y & 1] + o));
+          z0 = m.x > 0.f ? z0 : 0.f;
+          z1 = m.y > 0.f ? z1 : 0.f;
+        }
+        *reinterpret_cast<unsigned*>(sm.out + o) = pack_bf16(z0, z1);
+      }
+    __syncwarp();
+    {
+      const int c = q0 + (lane >> 1), xx = x0 + c;
+      if (xx < w)
+        *reinterpret_cast<uint4*>(reinterpret_cast<unsigned char*>(out) +
+                                  (img + (size_t)y * w + xx) * 32 + (lane & 1) * 16) =
+            *reinterpret_cast<const uint4*>(sm.out + c * kStPx + (lane & 1) * 16);
+    }
+    __syncthreads();  // the ring's oldest row is read before it is refilled
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
 }
 
 // ---------------------------------------------------------------- conv3 (16 -> 1) + residual
 __global__ void cnn_conv3_kernel(const float* params, const float* x, const __nv_bfloat16* h2,
                                  float* y, int h, int w) {
-  __shared__ float sp[9 * kC + 1];  // w3, b3
+  __shared__ __align__(16) float sp[9 * kC + 1];  // w3, b3
   for (int i = threadIdx.x; i < 9 * kC + 1; i += blockDim.x) sp[i] = params[kW3 + i];
   __syncthreads();
   const int xi = blockIdx.x * blockDim.x + threadIdx.x, yi = blockIdx.y, im = blockIdx.z;
@@ -183,10 +239,13 @@ __global__ void cnn_conv3_kernel(const float* params, const float* x, const __nv
     const uint4 q0 = __ldg(&p[0]), q1 = __ldg(&p[1]);
     const unsigned u[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
 #pragma unroll
-    for (int c = 0; c < kC; c += 2) {
-      const float2 v = unpack_bf16(u[c / 2]);
-      z = fmaf(sp[tap * kC + c], v.x, z);
-      z = fmaf(sp[tap * kC + c + 1], v.y, z);
+    for (int c = 0; c < kC; c += 4) {
+      const float4 wt = *reinterpret_cast<const float4*>(sp + tap * kC + c);
+      const float2 v = unpack_bf16(u[c / 2]), v2 = unpack_bf16(u[c / 2 + 1]);
+      z = fmaf(wt.x, v.x, z);
+      z = fmaf(wt.y, v.y, z);
+      z = fmaf(wt.z, v2.x, z);
+      z = fmaf(wt.w, v2.y, z);
     }
   }
   const size_t o = ((size_t)im * h + yi) * w + xi;
@@ -217,6 +276,9 @@ __global__ void cnn_loss_kernel(const float* y, const float* target, float* gy, 
 // g_z2[p][c] = (h2[p][c] > 0) * sum_tap w3[tap][c] gy[p - (dy, dx)]
 __global__ void cnn_conv3_bwd_kernel(const float* params, const float* gy,
                                      const __nv_bfloat16* h2, __nv_bfloat16* gz2, int h, int w) {
+  __shared__ __align__(16) float sp[9 * kC];  // w3
+  for (int i = threadIdx.x; i < 9 * kC; i += blockDim.x) sp[i] = params[kW3 + i];
+  __syncthreads();
   const int xi = blockIdx.x * blockDim.x + threadIdx.x, yi = blockIdx.y, im = blockIdx.z;
   if (xi >= w) return;
   const float* gm = gy + (size_t)im * h * w;
@@ -227,18 +289,29 @@ __global__ void cnn_conv3_bwd_kernel(const float* params, const float* gy,
     gin[tap] = (yy >= 0 && yy < h && xx >= 0 && xx < w) ? gm[(size_t)yy * w + xx] : 0.f;
   }
   const size_t p = ((size_t)im * h + yi) * w + xi;
-  const unsigned* h32 = reinterpret_cast<const unsigned*>(h2) + p * (kC / 2);
-  unsigned* g32 = reinterpret_cast<unsigned*>(gz2) + p * (kC / 2);
+  const uint4* m128 = reinterpret_cast<const uint4*>(h2) + p * 2;
+  uint4* g128 = reinterpret_cast<uint4*>(gz2) + p * 2;
 #pragma unroll
-  for (int c = 0; c < kC; c += 2) {
-    float z0 = 0.f, z1 = 0.f;
+  for (int half = 0; half < 2; ++half) {
+    const uint4 mq = __ldg(&m128[half]);
+    const unsigned mu[4] = {mq.x, mq.y, mq.z, mq.w};
+    unsigned o[4];
 #pragma unroll
-    for (int tap = 0; tap < 9; ++tap) {
-      z0 = fmaf(__ldg(&params[kW3 + tap * kC + c]), gin[tap], z0);
-      z1 = fmaf(__ldg(&params[kW3 + tap * kC + c + 1]), gin[tap], z1);
+    for (int c = 0; c < 8; c += 4) {
+      float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int tap = 0; tap < 9; ++tap) {
+        const float4 wt = *reinterpret_cast<const float4*>(sp + tap * kC + half * 8 + c);
+        z.x = fmaf(wt.x, gin[tap], z.x);
+        z.y = fmaf(wt.y, gin[tap], z.y);
+        z.z = fmaf(wt.z, gin[tap], z.z);
+        z.w = fmaf(wt.w, gin[tap], z.w);
+      }
+      const float2 m0 = unpack_bf16(mu[c / 2]), m1 = unpack_bf16(mu[c / 2 + 1]);
+      o[c / 2] = pack_bf16(m0.x > 0.f ? z.x : 0.f, m0.y > 0.f ? z.y : 0.f);
+      o[c / 2 + 1] = pack_bf16(m1.x > 0.f ? z.z : 0.f, m1.y > 0.f ? z.w : 0.f);
     }
-    const float2 m = unpack_bf16(__ldg(&h32[c / 2]));
-    g32[c / 2] = pack_bf16(m.x > 0.f ? z0 : 0.f, m.y > 0.f ? z1 : 0.f);
+    g128[half] = make_uint4(o[0], o[1], o[2], o[3]);
   }
 }
 
@@ -257,8 +330,8 @@ __global__ void cnn_conv3_bwd_kernel(const float* params, const float* gy,
 // Bound: the latency of a row's exchanges (one row of 64 pixels per barrier), then DRAM
 // (136 bytes per pixel).  4 x 1024 x 1024: 232 us and 5 us for the reduction of 384 blocks,
 // against 2179 us on the CUDA cores and 1444 us for the reduction of 32768 segments.
-constexpr int kWgW = 64, kWgThreads = 128, kWgBlocks = 3;  // blocks per SM
-constexpr int kWgPx = 48;                                  // bytes between pixels in shared memory
+constexpr int kWgW = kStW, kWgThreads = 128, kWgBlocks = 3;  // blocks per SM
+constexpr int kWgPx = kStPx;
 constexpr int kWgHalo = kWgW + 2;
 struct WgSmem {
   alignas(16) unsigned char h1[4][kWgHalo * kWgPx];        // ring over rows y - 1 .. y + 2
@@ -269,20 +342,11 @@ struct WgSmem {
 static_assert(sizeof(WgSmem) <= 48 * 1024 && sizeof(WgSmem) >= kCnnParams * sizeof(float),
               "default shared-memory limit; the sums fit over the rings");
 
-// Segments of a strip, so that the blocks fill the GPU about once.
-int wg_segments(int n_img, int h, int w) {
-  const long strips = (long)n_img * ((w + kWgW - 1) / kWgW);
-  return (int)std::max(1L, std::min<long>(h, kWgBlocks * 148L / strips));
-}
+int wg_segments(int n_img, int h, int w) { return strip_segments(n_img, h, w, kWgBlocks); }
 long wg_blocks(int n_img, int h, int w) {
   return (long)n_img * ((w + kWgW - 1) / kWgW) * wg_segments(n_img, h, w);
 }
 
-__device__ __forceinline__ void cp_async_zfill16(void* dst, const void* src, bool ok) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_u32(dst)), "l"(src),
-               "r"(ok ? 16 : 0)
-               : "memory");
-}
 __device__ __forceinline__ void cp_async_zfill4(void* dst, const void* src, bool ok) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(smem_u32(dst)), "l"(src),
                "r"(ok ? 4 : 0)
@@ -886,7 +950,9 @@ int gr_cnn_forward(const float* params, const float* x, float* y, int n_img, int
   __nv_bfloat16* h2 = h1 + px * kC;
   const dim3 gp((w + 127) / 128, h, n_img);
   cnn_conv1_kernel<<<gp, 128, 0, st>>>(params, x, h1, h, w);
-  cnn_conv2_kernel<<<dim3((w + 64 * kConv2Tiles - 1) / (64 * kConv2Tiles), h, n_img), 128, 0, st>>>(params, h1, nullptr, h2, h, w, 0);
+  const int s2 = strip_segments(n_img, h, w, kStBlocks);
+  const dim3 g2((w + kStW - 1) / kStW * s2, n_img);
+  cnn_conv2_kernel<<<g2, kStThreads, 0, st>>>(params, h1, nullptr, h2, h, w, 0, s2);
   cnn_conv3_kernel<<<gp, 128, 0, st>>>(params, x, h2, y, h, w);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? GR_OK : fail(GR_ERR_CUDA, "cnn forward: %s", cudaGetErrorString(e));
@@ -915,7 +981,9 @@ int gr_cnn_backward(const float* params, const float* x, const float* y, const f
   cnn_loss_kernel<<<lblocks, 256, 0, st>>>(y, target, gy, lpart, (long)px);
   const dim3 gp((w + 127) / 128, h, n_img);
   cnn_conv3_bwd_kernel<<<gp, 128, 0, st>>>(params, gy, h2, gz2, h, w);
-  cnn_conv2_kernel<<<dim3((w + 64 * kConv2Tiles - 1) / (64 * kConv2Tiles), h, n_img), 128, 0, st>>>(params, gz2, h1, gz1, h, w, 1);
+  const int s2 = strip_segments(n_img, h, w, kStBlocks);
+  cnn_conv2_kernel<<<dim3((w + kStW - 1) / kStW * s2, n_img), kStThreads, 0, st>>>(params, gz2, h1, gz1,
+                                                                                  h, w, 1, s2);
   cnn_wgrad_kernel<<<dim3((unsigned)(blocks / n_img), n_img), kWgThreads, sizeof(WgSmem), st>>>(
       x, gy, h1, h2, gz1, gz2, part, h, w, segs);
   cnn_reduce_kernel<<<(kCnnParams + 31) / 32, 256, 0, st>>>(part, blocks, grads);
