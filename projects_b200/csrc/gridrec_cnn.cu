@@ -40,39 +40,60 @@ __device__ __forceinline__ float2 unpack_bf16(unsigned u) {
   return __bfloat1622float2(v);
 }
 
+// Pixels per thread of the thin layers (rows, or columns in conv3): the weights' 16-byte
+// shared-memory reads, which bound them, serve that many pixels.
+constexpr int kThinPx = 2;
+
 // ---------------------------------------------------------------- conv1 (1 -> 16)
-__global__ void cnn_conv1_kernel(const float* params, const float* x, __nv_bfloat16* h1, int h,
-                                 int w) {
+// Thread: pixels (xi, yi) .. (xi, yi + kThinPx - 1).
+__global__ void __launch_bounds__(128) cnn_conv1_kernel(const float* params, const float* x,
+                                                        __nv_bfloat16* h1, int h, int w) {
   __shared__ __align__(16) float sp[kB1 + kC];  // w1, b1
   for (int i = threadIdx.x; i < kB1 + kC; i += blockDim.x) sp[i] = params[i];
   __syncthreads();
-  const int xi = blockIdx.x * blockDim.x + threadIdx.x, yi = blockIdx.y, im = blockIdx.z;
+  const int xi = blockIdx.x * blockDim.x + threadIdx.x, yi = blockIdx.y * kThinPx, im = blockIdx.z;
   if (xi >= w) return;
   const float* xm = x + (size_t)im * h * w;
-  float in[9];
+  float in[kThinPx + 2][3];
 #pragma unroll
-  for (int tap = 0; tap < 9; ++tap) {
-    const int yy = yi + tap_dy(tap), xx = xi + tap_dx(tap);
-    in[tap] = (yy >= 0 && yy < h && xx >= 0 && xx < w) ? xm[(size_t)yy * w + xx] : 0.f;
-  }
-  unsigned o[kC / 2];
+  for (int r = 0; r < kThinPx + 2; ++r)
 #pragma unroll
-  for (int c = 0; c < kC; c += 4) {  // 16-byte weight loads: a quarter of the 4-byte ones
-    float4 z = *reinterpret_cast<const float4*>(sp + kB1 + c);
-#pragma unroll
-    for (int tap = 0; tap < 9; ++tap) {
-      const float4 wt = *reinterpret_cast<const float4*>(sp + kW1 + tap * kC + c);
-      z.x = fmaf(wt.x, in[tap], z.x);
-      z.y = fmaf(wt.y, in[tap], z.y);
-      z.z = fmaf(wt.z, in[tap], z.z);
-      z.w = fmaf(wt.w, in[tap], z.w);
+    for (int c = 0; c < 3; ++c) {
+      const int yy = yi + r - 1, xx = xi + c - 1;
+      in[r][c] = (yy >= 0 && yy < h && xx >= 0 && xx < w) ? xm[(size_t)yy * w + xx] : 0.f;
     }
-    o[c / 2] = pack_bf16(fmaxf(z.x, 0.f), fmaxf(z.y, 0.f));
-    o[c / 2 + 1] = pack_bf16(fmaxf(z.z, 0.f), fmaxf(z.w, 0.f));
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    unsigned o[kThinPx][4];
+#pragma unroll
+    for (int c = 0; c < 8; c += 4) {
+      float4 z[kThinPx];
+#pragma unroll
+      for (int p = 0; p < kThinPx; ++p) z[p] = *reinterpret_cast<const float4*>(sp + kB1 + half * 8 + c);
+#pragma unroll
+      for (int tap = 0; tap < 9; ++tap) {
+        const float4 wt = *reinterpret_cast<const float4*>(sp + kW1 + tap * kC + half * 8 + c);
+#pragma unroll
+        for (int p = 0; p < kThinPx; ++p) {
+          const float v = in[p + tap / 3][tap % 3];
+          z[p].x = fmaf(wt.x, v, z[p].x);
+          z[p].y = fmaf(wt.y, v, z[p].y);
+          z[p].z = fmaf(wt.z, v, z[p].z);
+          z[p].w = fmaf(wt.w, v, z[p].w);
+        }
+      }
+#pragma unroll
+      for (int p = 0; p < kThinPx; ++p) {
+        o[p][c / 2] = pack_bf16(fmaxf(z[p].x, 0.f), fmaxf(z[p].y, 0.f));
+        o[p][c / 2 + 1] = pack_bf16(fmaxf(z[p].z, 0.f), fmaxf(z[p].w, 0.f));
+      }
+    }
+#pragma unroll
+    for (int p = 0; p < kThinPx; ++p)
+      if (yi + p < h)
+        reinterpret_cast<uint4*>(h1 + (((size_t)im * h + yi + p) * w + xi) * kC)[half] =
+            make_uint4(o[p][0], o[p][1], o[p][2], o[p][3]);
   }
-  uint4* out = reinterpret_cast<uint4*>(h1 + (((size_t)im * h + yi) * w + xi) * kC);
-  out[0] = make_uint4(o[0], o[1], o[2], o[3]);
-  out[1] = make_uint4(o[4], o[5], o[6], o[7]);
 }
 
 // ---------------------------------------------------------------- conv2 (16 -> 16), tensor cores
@@ -98,7 +119,8 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const unsigned (&a)[4], 
 // three input rows in use lie in a ring in shared memory (pixels kStPx bytes apart, so that
 // the eight 16-byte rows of an ldmatrix fall on distinct banks), filled by cp.async a row
 // ahead, so an input pixel is read once per strip instead of once per tap.  The output
-// goes through shared memory to whole 16-byte stores.  4 x 1024 x 1024: CONV2FIG
+// goes through shared memory to whole 16-byte stores.  4 x 1024 x 1024: 99 us
+// forward or backward (201 us with A fragments loaded from global memory, 4 bytes a lane).
 constexpr int kStW = 64, kStThreads = 128, kStBlocks = 4;  // blocks per SM
 constexpr int kStPx = 48;                                  // bytes between pixels in shared memory
 constexpr int kStHalo = kStW + 2;
@@ -222,34 +244,67 @@ __global__ void __launch_bounds__(kStThreads, kStBlocks) cnn_conv2_kernel(
 }
 
 // ---------------------------------------------------------------- conv3 (16 -> 1) + residual
-__global__ void cnn_conv3_kernel(const float* params, const float* x, const __nv_bfloat16* h2,
-                                 float* y, int h, int w) {
+// A thread walks down kConv3Rows rows of kThinPx columns, 128 apart, with the sums of
+// three output rows of each: a loaded pixel of h2 serves three taps (6 instead of 18
+// 16-byte loads per output) and a weight all columns.  Each sum takes its taps in order
+// 0..8 (rows y - 1, y, y + 1).  L1-bound (16-byte loads 32 bytes apart and the weights'
+// broadcasts).
+constexpr int kConv3Rows = 16;
+
+__global__ void __launch_bounds__(128) cnn_conv3_kernel(const float* params, const float* x,
+                                                        const __nv_bfloat16* h2, float* y, int h,
+                                                        int w) {
   __shared__ __align__(16) float sp[9 * kC + 1];  // w3, b3
   for (int i = threadIdx.x; i < 9 * kC + 1; i += blockDim.x) sp[i] = params[kW3 + i];
   __syncthreads();
-  const int xi = blockIdx.x * blockDim.x + threadIdx.x, yi = blockIdx.y, im = blockIdx.z;
+  const int xi = blockIdx.x * (128 * kThinPx) + threadIdx.x, im = blockIdx.z;
   if (xi >= w) return;
   const uint4* h128 = reinterpret_cast<const uint4*>(h2) + (size_t)im * h * w * 2;
-  float z = sp[9 * kC];
+  const int y0 = blockIdx.y * kConv3Rows, y1 = min(h, y0 + kConv3Rows);
+  const float bias = sp[9 * kC];
+  float zp[kThinPx], zc[kThinPx], zn[kThinPx];  // output rows r - 1, r, r + 1
 #pragma unroll
-  for (int tap = 0; tap < 9; ++tap) {
-    const int yy = yi + tap_dy(tap), xx = xi + tap_dx(tap);
-    if (yy < 0 || yy >= h || xx < 0 || xx >= w) continue;
-    const uint4* p = h128 + ((size_t)yy * w + xx) * 2;
-    const uint4 q0 = __ldg(&p[0]), q1 = __ldg(&p[1]);
-    const unsigned u[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+  for (int p = 0; p < kThinPx; ++p) zp[p] = zc[p] = zn[p] = bias;
+  for (int r = y0 - 1; r <= y1; ++r) {
+    if (r >= 0 && r < h) {
 #pragma unroll
-    for (int c = 0; c < kC; c += 4) {
-      const float4 wt = *reinterpret_cast<const float4*>(sp + tap * kC + c);
-      const float2 v = unpack_bf16(u[c / 2]), v2 = unpack_bf16(u[c / 2 + 1]);
-      z = fmaf(wt.x, v.x, z);
-      z = fmaf(wt.y, v.y, z);
-      z = fmaf(wt.z, v2.x, z);
-      z = fmaf(wt.w, v2.y, z);
+      for (int dx = 0; dx < 3; ++dx) {
+        uint4 q[kThinPx][2];
+#pragma unroll
+        for (int p = 0; p < kThinPx; ++p) {
+          const int xx = xi + 128 * p + dx - 1;
+          const bool ok = xx >= 0 && xx < w;
+          const uint4* s = h128 + ((size_t)r * w + (ok ? xx : 0)) * 2;
+          q[p][0] = ok ? __ldg(&s[0]) : make_uint4(0u, 0u, 0u, 0u);
+          q[p][1] = ok ? __ldg(&s[1]) : make_uint4(0u, 0u, 0u, 0u);
+        }
+#pragma unroll
+        for (int c = 0; c < kC; c += 4) {
+          const float4 w0 = *reinterpret_cast<const float4*>(sp + dx * kC + c);
+          const float4 w1 = *reinterpret_cast<const float4*>(sp + (3 + dx) * kC + c);
+          const float4 w2 = *reinterpret_cast<const float4*>(sp + (6 + dx) * kC + c);
+#pragma unroll
+          for (int p = 0; p < kThinPx; ++p) {
+            const uint4 u = q[p][c / 8];
+            const float2 v = unpack_bf16((c & 4) ? u.z : u.x), v2 = unpack_bf16((c & 4) ? u.w : u.y);
+            zn[p] = fmaf(w0.w, v2.y, fmaf(w0.z, v2.x, fmaf(w0.y, v.y, fmaf(w0.x, v.x, zn[p]))));
+            zc[p] = fmaf(w1.w, v2.y, fmaf(w1.z, v2.x, fmaf(w1.y, v.y, fmaf(w1.x, v.x, zc[p]))));
+            zp[p] = fmaf(w2.w, v2.y, fmaf(w2.z, v2.x, fmaf(w2.y, v.y, fmaf(w2.x, v.x, zp[p]))));
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int p = 0; p < kThinPx; ++p) {
+      if (r - 1 >= y0 && xi + 128 * p < w) {
+        const size_t o = ((size_t)im * h + r - 1) * w + xi + 128 * p;
+        y[o] = x[o] + zp[p];
+      }
+      zp[p] = zc[p];
+      zc[p] = zn[p];
+      zn[p] = bias;
     }
   }
-  const size_t o = ((size_t)im * h + yi) * w + xi;
-  y[o] = x[o] + z;
 }
 
 // ---------------------------------------------------------------- backward pieces
@@ -279,39 +334,58 @@ __global__ void cnn_conv3_bwd_kernel(const float* params, const float* gy,
   __shared__ __align__(16) float sp[9 * kC];  // w3
   for (int i = threadIdx.x; i < 9 * kC; i += blockDim.x) sp[i] = params[kW3 + i];
   __syncthreads();
-  const int xi = blockIdx.x * blockDim.x + threadIdx.x, yi = blockIdx.y, im = blockIdx.z;
+  const int xi = blockIdx.x * blockDim.x + threadIdx.x, yi = blockIdx.y * kThinPx, im = blockIdx.z;
   if (xi >= w) return;
   const float* gm = gy + (size_t)im * h * w;
-  float gin[9];
+  float gin[kThinPx + 2][3];  // gy around the thread's pixels
 #pragma unroll
-  for (int tap = 0; tap < 9; ++tap) {
-    const int yy = yi - tap_dy(tap), xx = xi - tap_dx(tap);
-    gin[tap] = (yy >= 0 && yy < h && xx >= 0 && xx < w) ? gm[(size_t)yy * w + xx] : 0.f;
-  }
-  const size_t p = ((size_t)im * h + yi) * w + xi;
-  const uint4* m128 = reinterpret_cast<const uint4*>(h2) + p * 2;
-  uint4* g128 = reinterpret_cast<uint4*>(gz2) + p * 2;
+  for (int r = 0; r < kThinPx + 2; ++r)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const int yy = yi + r - 1, xx = xi + c - 1;
+      gin[r][c] = (yy >= 0 && yy < h && xx >= 0 && xx < w) ? gm[(size_t)yy * w + xx] : 0.f;
+    }
 #pragma unroll
   for (int half = 0; half < 2; ++half) {
-    const uint4 mq = __ldg(&m128[half]);
-    const unsigned mu[4] = {mq.x, mq.y, mq.z, mq.w};
-    unsigned o[4];
+    unsigned mu[kThinPx][4], o[kThinPx][4];
+#pragma unroll
+    for (int p = 0; p < kThinPx; ++p) {
+      const size_t px = ((size_t)im * h + min(yi + p, h - 1)) * w + xi;
+      const uint4 mq = __ldg(reinterpret_cast<const uint4*>(h2) + px * 2 + half);
+      mu[p][0] = mq.x;
+      mu[p][1] = mq.y;
+      mu[p][2] = mq.z;
+      mu[p][3] = mq.w;
+    }
 #pragma unroll
     for (int c = 0; c < 8; c += 4) {
-      float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+      float4 z[kThinPx];
+#pragma unroll
+      for (int p = 0; p < kThinPx; ++p) z[p] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
       for (int tap = 0; tap < 9; ++tap) {
         const float4 wt = *reinterpret_cast<const float4*>(sp + tap * kC + half * 8 + c);
-        z.x = fmaf(wt.x, gin[tap], z.x);
-        z.y = fmaf(wt.y, gin[tap], z.y);
-        z.z = fmaf(wt.z, gin[tap], z.z);
-        z.w = fmaf(wt.w, gin[tap], z.w);
+#pragma unroll
+        for (int p = 0; p < kThinPx; ++p) {
+          const float v = gin[p + 2 - tap / 3][2 - tap % 3];  // gy[p - (dy, dx)]
+          z[p].x = fmaf(wt.x, v, z[p].x);
+          z[p].y = fmaf(wt.y, v, z[p].y);
+          z[p].z = fmaf(wt.z, v, z[p].z);
+          z[p].w = fmaf(wt.w, v, z[p].w);
+        }
       }
-      const float2 m0 = unpack_bf16(mu[c / 2]), m1 = unpack_bf16(mu[c / 2 + 1]);
-      o[c / 2] = pack_bf16(m0.x > 0.f ? z.x : 0.f, m0.y > 0.f ? z.y : 0.f);
-      o[c / 2 + 1] = pack_bf16(m1.x > 0.f ? z.z : 0.f, m1.y > 0.f ? z.w : 0.f);
+#pragma unroll
+      for (int p = 0; p < kThinPx; ++p) {
+        const float2 m0 = unpack_bf16(mu[p][c / 2]), m1 = unpack_bf16(mu[p][c / 2 + 1]);
+        o[p][c / 2] = pack_bf16(m0.x > 0.f ? z[p].x : 0.f, m0.y > 0.f ? z[p].y : 0.f);
+        o[p][c / 2 + 1] = pack_bf16(m1.x > 0.f ? z[p].z : 0.f, m1.y > 0.f ? z[p].w : 0.f);
+      }
     }
-    g128[half] = make_uint4(o[0], o[1], o[2], o[3]);
+#pragma unroll
+    for (int p = 0; p < kThinPx; ++p)
+      if (yi + p < h)
+        reinterpret_cast<uint4*>(gz2)[(((size_t)im * h + yi + p) * w + xi) * 2 + half] =
+            make_uint4(o[p][0], o[p][1], o[p][2], o[p][3]);
   }
 }
 
@@ -948,12 +1022,13 @@ int gr_cnn_forward(const float* params, const float* x, float* y, int n_img, int
   const size_t px = (size_t)n_img * h * w;
   __nv_bfloat16* h1 = static_cast<__nv_bfloat16*>(workspace);
   __nv_bfloat16* h2 = h1 + px * kC;
-  const dim3 gp((w + 127) / 128, h, n_img);
+  const dim3 gp((w + 127) / 128, (h + kThinPx - 1) / kThinPx, n_img);
   cnn_conv1_kernel<<<gp, 128, 0, st>>>(params, x, h1, h, w);
   const int s2 = strip_segments(n_img, h, w, kStBlocks);
   const dim3 g2((w + kStW - 1) / kStW * s2, n_img);
   cnn_conv2_kernel<<<g2, kStThreads, 0, st>>>(params, h1, nullptr, h2, h, w, 0, s2);
-  cnn_conv3_kernel<<<gp, 128, 0, st>>>(params, x, h2, y, h, w);
+  cnn_conv3_kernel<<<dim3((w + 128 * kThinPx - 1) / (128 * kThinPx), (h + kConv3Rows - 1) / kConv3Rows, n_img), 128, 0, st>>>(
+      params, x, h2, y, h, w);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? GR_OK : fail(GR_ERR_CUDA, "cnn forward: %s", cudaGetErrorString(e));
 }
@@ -979,7 +1054,7 @@ int gr_cnn_backward(const float* params, const float* x, const float* y, const f
   lpart = reinterpret_cast<double*>(((uintptr_t)lpart + 7) & ~(uintptr_t)7);
   const int lblocks = 1024;
   cnn_loss_kernel<<<lblocks, 256, 0, st>>>(y, target, gy, lpart, (long)px);
-  const dim3 gp((w + 127) / 128, h, n_img);
+  const dim3 gp((w + 127) / 128, (h + kThinPx - 1) / kThinPx, n_img);
   cnn_conv3_bwd_kernel<<<gp, 128, 0, st>>>(params, gy, h2, gz2, h, w);
   const int s2 = strip_segments(n_img, h, w, kStBlocks);
   cnn_conv2_kernel<<<dim3((w + kStW - 1) / kStW * s2, n_img), kStThreads, 0, st>>>(params, gz2, h1, gz1,
