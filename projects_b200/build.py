@@ -16,8 +16,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libgridrec_b200.so")
-SOURCES = ["gridrec_kernels.cu", "gridrec_plan.cu", "gridrec_prep.cu", "gridrec_fbp.cu",
-           "gridrec_cnn.cu", "gridrec_cpp.cu"]
+SOURCES = ["gridrec_kernels.cu", "gridrec_grid.cu", "gridrec_plan.cu", "gridrec_prep.cu",
+           "gridrec_fbp.cu", "gridrec_cnn.cu", "gridrec_cpp.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

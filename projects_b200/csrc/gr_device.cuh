@@ -65,4 +65,12 @@ __device__ __forceinline__ void tc_fence_after() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 
+// (int)(d * ts + 0.5) for d >= 0 -- the nearest-neighbour table index of
+// gridrec.h:53 -- in FP64 with the product and the sum rounded separately, as
+// the FP64 restatement forms them; capped so that far taps stay in int range
+// (callers clamp to the table length and zero taps beyond L/2).
+__device__ __forceinline__ int table_index64(double d, double ts) {
+  return (int)fmin(__dadd_rn(__dmul_rn(d, ts), 0.5), 2.0e9);
+}
+
 }  // namespace gr

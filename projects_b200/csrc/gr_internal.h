@@ -52,6 +52,28 @@ constexpr int kW32MinBlocks = 4;
 // Index of a zero weight (a tap beyond L/2) in the kernel's table copy.
 inline int w32_zero_index(int ltbl) { return ltbl + 1; }
 
+// The gridding kernel of chunks of a few pairs (grid_group_kernel): a warp grids 32 / G
+// kWideRows x kWideCols sub-tiles at once for G pairs.  Its record of one (sub-tile,
+// sample): the table indices of the 4 rows and 8 columns (ltbl + 1, a zero weight, for a
+// tap beyond L/2) and the sample's place in the spectra, (direction * J / 4 + j / 4) * 4 +
+// j % 4.
+struct alignas(32) TapRec {
+  unsigned short idx[kWideRows + kWideCols];
+  unsigned place;
+  unsigned pad;
+};
+constexpr int kGrpMinBlocks = 4;
+// It grids chunks of up to kGroupPairs pairs by default (gr_params.wide_grid = 0), those of
+// one pair only where the list has at most kGroupOneItems sub-tiles (M <= 1024).  Per pair
+// against the kernel that took the chunk otherwise (the tile kernel up to 6 pairs, the
+// 16-pair kernel above), us at 1024 x 720 and 2048 x 1500: 8 pairs 12.2 / 19.7 and 35.3 /
+// 71.0, 6 pairs 17.5 / 29.0 and 53.6 / 89.7, 4 pairs 20 / 31 and 58 / 95, 2 pairs 33 / 57 and 108 /
+// 110, one pair 60 / 97 and 205 / 133 (32 items of a bundle for one pair cost more table
+// lookups than the tile kernel's pass over them).  For 9 to 16 pairs two groups cost what the
+// 16-pair kernel does, for more the 32-pair kernel is faster (31 a pair).
+constexpr int kGroupPairs = 8;
+constexpr int kGroupOneItems = 1 << 15;
+
 // The tensor-core gridding kernel (grid_tc_kernel): a CTA accumulates a
 // kTcRows x kTcCols sub-tile (128 cells, the MMA M) for 16 pairs x (re, im)
 // (the MMA N) in tensor memory, 8 samples (the MMA K) per step.
@@ -101,9 +123,8 @@ struct SpectraArgs {
   const float2* tw;      // two-level twiddle table for pdim (see gridrec_kernels.cu)
   int n_det, n_ang, pdim, J, pairs;
   const double* roi_off; // per angle (X0 cos + Y0 sin) pi of the ROI offset, or null
-  // 0: plain [pair][dir][j]; 16 or 32: the 16- or 32-pair gridding kernel's
-  // [pair / G][dir][j / 4][pair % G][j % 4] (G = wide), for G = 32 with the two
-  // 16-byte halves of a pair's chunk swapped when (pair / 4) is odd
+  // 0: plain [pair][dir][j]; G = wide, a power of two: the layout of gridding by G pairs,
+  // [pair / G][dir][j / 4][pair % G][j % 4], for G = 32 with the two 16-byte halves of a pair's chunk swapped when (pair / 4) is odd
   int wide = 0;
   // device error word for the bounded wait of the staged input (null: the rows are
   // loaded element by element, with no wait)
@@ -151,6 +172,10 @@ struct GridArgs {
   // the 16-bit table indices (launch_w32_index)
   const int4* xmeta = nullptr;
   const unsigned short* xidx = nullptr;
+  // grid_group_kernel: a record per (sub-tile, sample); its items' run_begin / run_end
+  // are ranges of records
+  const TapRec* rec = nullptr;
+  int n_long = 0;  // the items it grids by a warp each, the first of the list
 };
 
 struct ColArgs {
@@ -227,6 +252,7 @@ struct DeviceGuard {
 
 // Kernel launchers (gridrec_kernels.cu).  Return cudaGetLastError().
 cudaError_t init_kernel_attributes();
+void add_grid_kernels(std::vector<const void*>& f);  // gridrec_grid.cu
 cudaError_t launch_phase(const PhaseArgs& a, cudaStream_t s);
 cudaError_t launch_spectra(const SpectraArgs& a, gr_dtype dt, cudaStream_t s);
 // Gridding: grid_kernel over 32 x 32 tiles (two pairs per warp) or
@@ -246,6 +272,11 @@ cudaError_t launch_w32_index(const GridArgs& a, int n_runs, const int2* rinfo,
 cudaError_t launch_dark_log(const float* flat, const float* dark, long flat_stride, int slice_base,
                             int n_valid, int n_det, float2* out, cudaStream_t s);
 cudaError_t launch_grid_w32(const GridArgs& a, cudaStream_t s);
+// Gridding by groups of G pairs (1, 2, 4 or 8), and the records of a work list (once per list;
+// see tap_record_kernel).
+cudaError_t launch_grid_group(const GridArgs& a, int G, cudaStream_t s);
+cudaError_t launch_tap_records(const GridArgs& a, int subs, int spw, int* counts, const int* base,
+                               TapRec* rec, cudaStream_t s);
 int cols_group(int M);
 cudaError_t launch_cols(const ColArgs& a, cudaStream_t s);
 cudaError_t launch_rows(const RowArgs& a, cudaStream_t s);

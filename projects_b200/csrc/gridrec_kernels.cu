@@ -529,8 +529,8 @@ __global__ void __launch_bounds__(MAXT, 1024 / MAXT) spectra_kernel(SpectraArgs 
   __shared__ uint64_t in_bar;
   float2* tw = sm;
   float2* buf = sm + kTwSlots;
-  // wide layouts: pairs vary fastest, so the 16 or 32 pairs sharing each 512- or
-  // 1024-byte span of the interleaved spectra write it at about the same time
+  // wide layouts: pairs vary fastest, so the pairs sharing each span of the interleaved
+  // spectra write it at about the same time
   const int n = a.wide ? blockIdx.y : blockIdx.x, pair = a.wide ? blockIdx.x : blockIdx.y;
   const int tid = threadIdx.x, nthr = blockDim.x;
   load_twiddles(tw, a.tw, a.pdim);
@@ -627,7 +627,7 @@ __global__ void __launch_bounds__(MAXT, 1024 / MAXT) spectra_kernel(SpectraArgs 
   }
   __syncthreads();
   const float4* pq = a.pq + (size_t)pair * a.J;
-  // plain: [pair][dir][j]; wide (G = 16 or 32 pairs): [pair / G][dir][j / 4][pair % G][j % 4],
+  // plain: [pair][dir][j]; wide (G pairs, a power of two): [pair / G][dir][j / 4][pair % G][j % 4],
   // so each pair still writes whole 32-byte sectors and the gridding kernel stages a
   // run of G pairs as one contiguous range.  For G = 32 the two 16-byte halves of
   // pair p's chunk are swapped when (p / 4) is odd (sample j at position
@@ -638,7 +638,7 @@ __global__ void __launch_bounds__(MAXT, 1024 / MAXT) spectra_kernel(SpectraArgs 
   int qshift, qmask, qlog, rot = 0;
   if (a.wide) {
     const int G = a.wide;
-    qlog = G == 32 ? 7 : 6;  // float2 per quad: 4 samples x G pairs
+    qlog = 33 - __clz(G);  // log2 of the float2 per quad, 4 samples x G pairs
     const size_t per_dir = (size_t)(a.J >> 2) << qlog;
     o1 = a.spec + ((size_t)(pair / G) * 2 * a.n_ang + 2 * n) * per_dir + (pair % G) * 4;
     o2 = o1 + per_dir;
@@ -711,14 +711,6 @@ __global__ void __launch_bounds__(MAXT, 1024 / MAXT) spectra_kernel(SpectraArgs 
 
 constexpr int kTileStride = kTile + 1;
 constexpr int kGridWarps = 4;
-
-// (int)(d * ts + 0.5) for d >= 0 -- the nearest-neighbour table index of
-// gridrec.h:53 -- in FP64 with the product and the sum rounded separately, as
-// the FP64 restatement forms them; capped so that far taps stay in int range
-// (callers clamp to the table length and zero taps beyond L/2).
-__device__ __forceinline__ int table_index64(double d, double ts) {
-  return (int)fmin(__dadd_rn(__dmul_rn(d, ts), 0.5), 2.0e9);
-}
 
 // A cell of PG pairs gridded together: float4 (C_A, C_B) for two, float2 for one.
 template <int PG>
@@ -2170,6 +2162,7 @@ cudaError_t init_kernel_attributes() {
   fns.push_back((const void*)grid_wide_kernel);
   fns.push_back((const void*)grid_tc_kernel);
   fns.push_back((const void*)grid_w32_kernel);
+  add_grid_kernels(fns);
   for (const void* f : fns) {
     if (e != cudaSuccess) break;
     // the opt-in limit covers static and dynamic shared memory together

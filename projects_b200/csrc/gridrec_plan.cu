@@ -99,6 +99,23 @@ double filter_value(int code, double x) {
 
 // ------------------------------------------------------------------ the plan
 
+// A work list as grid_group_kernel takes it.
+struct GroupList {
+  Item* d_items = nullptr;       // run_begin / run_end: ranges of records
+  TapRec* d_rec = nullptr;
+  int4* d_split_list = nullptr;  // (sub-tile, first slot, items, slots apart)
+  float4* d_scratch = nullptr;   // [group of G pairs][slot][32 cells x G pairs] complex
+  size_t scratch_cells = 0;
+  int items = 0, slots = 0, split_tiles = 0;
+  size_t records = 0;
+  std::vector<int> longer;       // items of length class c and above (grp_class)
+  bool ready = false;
+};
+
+// Length class of an item of c records, an eighth of an octave wide: 0 for none.
+int grp_class(int c) { return c <= 0 ? 0 : 1 + (int)(8.f * std::log2((float)c)); }
+constexpr int kGrpClasses = 1 + 8 * 31 + 1;
+
 struct Plan {
   int device = 0;
   int n_det = 0, n_ang = 0, pdim = 0, M = 0, M02 = 0, M0 = 0, J = 0, ltbl = 0, filter = 0;
@@ -157,6 +174,9 @@ struct Plan {
   float4* d_x_scratch = nullptr;      // [pair group of 32][slot][32 cells x 32 pairs] complex
   size_t x_scratch_cells = 0;
   bool x_ready = false;
+  // gridding by groups of pairs (grid_group_kernel), with the sums in the order of the tile
+  // kernel's list and of the 16-pair kernel's
+  GroupList g_tiles, g_wide;
   int cols_G = 0;                   // column-FFT group width (0 = cols_group(M); autotuned)
   int cols_ring = 0;                // 1: persistent double-buffered column FFT (autotuned)
   // gridding kernel of full chunks (max_pairs pairs) in the default mode, chosen by the
@@ -460,6 +480,118 @@ void build_work_list(int M, int J, double L, int n_ang, const std::vector<double
   wl->total = total;
 }
 
+// Whether chunks of this plan can grid by groups of pairs in the order of the tile kernel
+// (1 .. 6 pairs) or of the 16-pair kernel (7 and 8 pairs).
+bool group_tiles_possible(const Plan* p) {
+  return p->wide_mode == 0 &&
+         (p->max_pairs > 1 || (long)p->M * p->M / (kWideRows * kWideCols) <= kGroupOneItems);
+}
+bool group_wide_possible(const Plan* p) { return p->wide_mode == 0 && p->max_pairs >= kWideMinPairs; }
+
+void drop_group_list(Plan* p, GroupList* g) {
+  dev_free(p, &g->d_items);
+  dev_free(p, &g->d_rec);
+  dev_free(p, &g->d_split_list);
+  dev_free(p, &g->d_scratch);
+  *g = GroupList{};
+}
+
+// The list `wl` (its items and runs on the device) as grid_group_kernel takes it: an item
+// per sub-tile of each item, with the records of the samples that have a tap there.  A
+// list that does not fit (memory, index range) is left out: the chunks then use the
+// kernel whose list it is.
+int install_group_list(Plan* p, GroupList* out, const WorkList& wl, const Item* d_items,
+                       const Run* d_runs, int subs, int spw) {
+  drop_group_list(p, out);
+  const size_t n = wl.items.size() * subs;
+  if (n > (size_t)INT_MAX || (size_t)wl.n_slots * subs > (size_t)INT_MAX ||
+      (size_t)2 * p->n_ang * p->J > (size_t)UINT_MAX)
+    return GR_OK;
+  GridArgs g{};
+  g.items = d_items;
+  g.n_items = (int)wl.items.size();
+  g.runs = d_runs;
+  g.dir = p->d_dir;
+  g.M = p->M;
+  g.J = p->J;
+  g.tiles_v = wl.tiles_v;
+  g.ltbl = p->ltbl;
+  g.L2 = p->L / 2;
+  g.tblspcg = 2.0 * p->ltbl / p->L;
+  int* d_at = nullptr;
+  if (dev_alloc(p, &d_at, n)) return GR_OK;
+  std::vector<int> at(n);
+  cudaError_t e = launch_tap_records(g, subs, spw, d_at, nullptr, nullptr, 0);
+  if (e == cudaSuccess) e = cudaMemcpy(at.data(), d_at, n * sizeof(int), cudaMemcpyDeviceToHost);
+  // sub-tile index and slot of item i's sub-tile s
+  const int tv32 = wl.tiles_v, tv48 = p->M / kWideCols;
+  constexpr int kSubCols = kTile / kWideCols;
+  auto sub_tile = [&](int tile, int s) {
+    return subs == 1 ? tile
+                     : (tile / tv32 * (kTile / kWideRows) + s / kSubCols) * tv48 +
+                           tile % tv32 * kSubCols + s % kSubCols;
+  };
+  // items in classes of length, longest first: the items of a bundle are of similar
+  // length, and no long one starts late
+  std::vector<size_t> first(kGrpClasses, 0);
+  size_t n_rec = 0, n_items = 0;
+  for (size_t i = 0; i < n && e == cudaSuccess; ++i)
+    if (at[i] >= 0) {
+      first[grp_class(at[i])]++;
+      n_rec += at[i];
+      ++n_items;
+    }
+  if (e == cudaSuccess && n_rec <= (size_t)INT_MAX && dev_alloc(p, &out->d_rec, std::max<size_t>(n_rec, 1)) == GR_OK) {
+    out->longer.resize(first.size());
+    for (size_t c = first.size(), sum = 0; c-- > 0;) {
+      const size_t k = first[c];
+      first[c] = sum;
+      sum += k;
+      out->longer[c] = (int)sum;
+    }
+    std::vector<Item> items(n_items);
+    std::vector<int> base(n, 0);
+    int next = 0;
+    for (size_t i = 0; i < n; ++i) {
+      if (at[i] < 0) continue;
+      const Item& it = wl.items[i / subs];
+      const int s = (int)(i % subs);
+      items[first[grp_class(at[i])]++] = {sub_tile(it.tile, s), next, next + at[i],
+                                    it.slot < 0 ? -1 : it.slot * subs + s};
+      base[i] = next;
+      next += at[i];
+    }
+    std::vector<int4> splits;
+    for (size_t t = 0; t < wl.splits.size(); ++t)
+      if (wl.splits[t].nsplit > 1)
+        for (int s = 0; s < subs; ++s) {
+          if (subs > 1 && ((int)t / tv32 * kTile + s / kSubCols * kWideRows >= p->M ||
+                           (int)t % tv32 * kTile + s % kSubCols * kWideCols >= p->M))
+            continue;
+          splits.push_back(make_int4(sub_tile((int)t, s), wl.splits[t].slot0 * subs + s,
+                                     wl.splits[t].nsplit, subs));
+        }
+    const size_t slots = (size_t)std::max(wl.n_slots * subs, 1);
+    const size_t cells = slots * kGroupPairs * (kWideRows * kWideCols / 2);
+    e = cudaMemcpy(d_at, base.data(), n * sizeof(int), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = launch_tap_records(g, subs, spw, nullptr, d_at, out->d_rec, 0);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(0);
+    if (e == cudaSuccess && upload(p, &out->d_items, items) == GR_OK &&
+        upload(p, &out->d_split_list, splits) == GR_OK && dev_alloc(p, &out->d_scratch, cells) == GR_OK) {
+      out->scratch_cells = cells;
+      out->items = (int)n_items;
+      out->slots = (int)slots;
+      out->split_tiles = (int)splits.size();
+      out->records = n_rec;
+      out->ready = true;
+    }
+  }
+  dev_free(p, &d_at);
+  if (!out->ready) drop_group_list(p, out);
+  if (e != cudaSuccess) return fail(GR_ERR_CUDA, "tap records: %s", cudaGetErrorString(e));
+  return GR_OK;
+}
+
 // Builds the work list with the given item cap and (re)places it on the
 // device; grows the split-tile scratch when needed.
 int install_work_list(Plan* p, int item_cap) {
@@ -493,7 +625,10 @@ int install_work_list(Plan* p, int item_cap) {
   p->total_samples = wl.total;
   p->n_split_tiles = (int)split_list.size();
   p->item_cap = item_cap;
-  return GR_OK;
+  if (!group_tiles_possible(p)) return GR_OK;
+  const int nt = p->ntaps <= 3 ? 3 : (p->ntaps <= 4 ? 4 : kMaxTaps);  // grid_kernel's lanes per sample
+  return install_group_list(p, &p->g_tiles, wl, p->d_items, p->d_runs, (kTile / kWideRows) * (kTile / kWideCols),
+                            32 / nt);
 }
 
 // Whether chunks of this plan can use the 16-pair kernel (its weights) or the
@@ -527,7 +662,10 @@ int install_work_list_wide(Plan* p, int item_cap) {
   if (n_rec > (size_t)INT_MAX) return fail(GR_ERR_UNSUPPORTED, "work list too large");
   // the 32-pair kernel's records: per run an index block of n * 12 16-bit indices,
   // padded to whole 16-byte units (its bulk copies move whole units)
-  const bool need16 = wide16_possible(p), need32 = w32_possible(p);
+  // (a plan whose chunks of 7 and 8 pairs grid by groups and has no larger ones needs no
+  // weights)
+  const bool need32 = w32_possible(p);
+  if (group_wide_possible(p)) drop_group_list(p, &p->g_wide);
   std::vector<int2> rinfo;
   size_t n_units = 0;
   if (need32) {
@@ -548,8 +686,13 @@ int install_work_list_wide(Plan* p, int item_cap) {
   p->x_ready = false;
   int rc;
   if ((rc = upload(p, &p->d_w_items, wl.items)) || (rc = upload(p, &p->d_w_runs, wl.runs)) ||
-      (rc = upload(p, &p->d_w_split_list, split_list)) ||
-      (need16 && ((rc = upload(p, &p->d_w_meta, meta)) ||
+      (rc = upload(p, &p->d_w_split_list, split_list)))
+    return rc;
+  if (group_wide_possible(p) &&
+      (rc = install_group_list(p, &p->g_wide, wl, p->d_w_items, p->d_w_runs, 1, 32)))
+    return rc;
+  const bool need16 = wide16_possible(p) && !(p->g_wide.ready && p->max_pairs <= kGroupPairs);
+  if ((need16 && ((rc = upload(p, &p->d_w_meta, meta)) ||
                   (rc = dev_alloc(p, &p->d_w_wts, std::max<size_t>(n_rec, 1) * kWideRec)))))
     return rc;
   GridArgs g{};
@@ -672,6 +815,17 @@ bool use_wide(const Plan* p, int pairs) {
   return p->wide_mode == 1 || pairs >= kWideMinPairs;
 }
 
+// The list by which a chunk of `pairs` pairs grids by groups, null where another kernel
+// grids it: by default 1 to 8 pairs, in the order of the kernel that would grid it
+// otherwise.
+const GroupList* group_list(const Plan* p, int pairs) {
+  if (pairs > kGroupPairs || p->wide_mode != 0 || use_w32(p, pairs)) return nullptr;
+  const GroupList* g = use_wide(p, pairs) ? &p->g_wide : &p->g_tiles;
+  if (!g->ready || (pairs == 1 && (long)p->M * p->M / (kWideRows * kWideCols) > kGroupOneItems)) return nullptr;
+  return g;
+}
+int group_size(int pairs) { return pairs <= 2 ? pairs : (pairs <= 4 ? 4 : 8); }
+
 GridArgs grid_args_tc(const Plan* p, int pairs) {
   GridArgs g{p->d_spec, p->d_H, p->d_t_scratch, p->d_queue, p->d_t_items, nullptr,
              p->d_t_split_list, p->t_split_tiles, p->d_dir, p->d_wtbl, p->t_items, pairs,
@@ -705,6 +859,26 @@ GridArgs grid_args_w32(const Plan* p, int pairs) {
   g.err = p->d_err;
   g.xmeta = p->d_x_meta;
   g.xidx = p->d_x_idx;
+  return g;
+}
+
+GridArgs grid_args_group(const Plan* p, const GroupList* l, int pairs) {
+  GridArgs g{p->d_spec, p->d_H, l->d_scratch, p->d_queue, l->d_items, nullptr,
+             l->d_split_list, l->split_tiles, p->d_dir, p->d_wtbl, l->items, pairs,
+             p->n_ang, p->J, p->M, p->M / kWideCols, l->slots, p->ltbl, p->L / 2,
+             2.0 * p->ltbl / p->L};
+  g.rec = l->d_rec;
+  // Items of more than `share` of a warp's part of all records are long, gridded by a warp
+  // each: a bundle takes as many steps as its longest item, and one that holds a large
+  // part of a warp's whole work ends after all others.  Per pair at 2048 x 1500, share 0.05 /
+  // 0.15 / 0.4 / 1 / none long: 42.2 / 36.3 / 35.3 / 39.6 / 39.4 us for 8 pairs, 68.2 / 62.0 /
+  // 57.7 / 66.4 / 78.4 for 4, 109 / 113 / 105 / 126 / 229 for 2; at 1024 x 720 12.9 / 12.7 / 12.2 /
+  // 13.9 / 23.1 for 8, 33.0 / 33.5 / 35.8 / 37.7 / 141 for 2, 60 / 60 / 64 / 74 / 440 for one (a
+  // bundle of 32 or 16 items is the less efficient form of the two).
+  const int G = group_size(pairs);
+  const double share = G >= 4 ? 0.3 : 0.05;
+  const double part = (double)l->records * G / 32 / (kGrpMinBlocks * 4 * 148);
+  g.n_long = l->longer[std::min(grp_class((int)std::min(part * share, 1e9)), kGrpClasses - 1)];
   return g;
 }
 
@@ -848,19 +1022,23 @@ int launch_chunk(Plan* p, int pairs, int n_valid, int slice_base, const void* s1
   GR_MARK();
   const bool tc = use_tc(p, pairs);
   const bool w32 = use_w32(p, pairs);
-  const bool wide = use_wide(p, pairs);
+  const GroupList* gl = tc ? nullptr : group_list(p, pairs);
+  const int grp = gl ? group_size(pairs) : 0;
+  const bool wide = !grp && use_wide(p, pairs);
   SpectraArgs sa{s1, s2, in_pair_stride, n_valid, slice_base, flat, dark, flat_stride, p->d_pq,
                  p->d_spec,
                  p->d_tw_p, p->n_det, p->n_ang, p->pdim, p->J, pairs, p->d_roi_off,
-                 w32 ? kW32Pairs : ((wide || tc) ? kWidePairs : 0), p->d_err};
+                 w32 ? kW32Pairs : ((wide || tc) ? kWidePairs : (grp > 1 ? grp : 0)), p->d_err};
   if (dl) sa.dl = p->d_dl;
   GR_CUDA(launch_spectra(sa, dt, st));
   GR_MARK();
   const GridArgs ga = tc ? grid_args_tc(p, pairs)
-                         : (w32 ? grid_args_w32(p, pairs) : grid_args(p, pairs, wide));
+                         : (w32 ? grid_args_w32(p, pairs)
+                                : (grp ? grid_args_group(p, gl, pairs) : grid_args(p, pairs, wide)));
   GR_CUDA(tc ? launch_grid_tc(ga, st)
              : (w32 ? launch_grid_w32(ga, st)
-                    : (wide ? launch_grid_wide(ga, st) : launch_grid(ga, p->ntaps, st))));
+                    : (grp ? launch_grid_group(ga, grp, st)
+                           : (wide ? launch_grid_wide(ga, st) : launch_grid(ga, p->ntaps, st)))));
   GR_MARK();
   ColArgs ca{p->d_H, p->d_tw_m, p->M, pairs, p->d_err, p->cols_G, p->cols_ring};
   GR_CUDA(launch_cols(ca, st));
@@ -1264,7 +1442,8 @@ int gr::plan_create_ex(const gr_params* prm, const Pswf* pswf, float (*filter_fn
   }
   const size_t P = (size_t)p->max_pairs;
   // the 16- and 32-pair kernels' spectra layouts hold whole groups of pairs
-  const size_t G_spec = p->x_ready ? kW32Pairs : ((p->w_items || p->t_items) ? kWidePairs : 1);
+  const size_t G_spec = p->x_ready ? kW32Pairs
+                        : ((p->w_items || p->t_items) ? kWidePairs : (p->g_tiles.ready ? kGroupPairs : 1));
   const size_t P_spec = (P + G_spec - 1) / G_spec * G_spec;
   p->spec_pairs = (int)P_spec;
   if ((rc = dev_alloc(p, &p->d_spec, P_spec * p->n_ang * 2 * p->J)) ||
@@ -1494,10 +1673,13 @@ int gr_plan_autotune(gr_plan* p, void* stream) {
                                         : std::vector<int>{512, 1024, 2048, 4096, 8192};
     for (int cap : caps) {
       if ((rc = install(kernel, cap))) break;
-      const GridArgs ga =
-          kernel == 3 ? grid_args_w32(p, pairs) : grid_args(p, pairs, kernel == 1);
+      if (p->wide_mode == 0) p->tuned_kernel = kernel;  // what group_list() makes of a full chunk
+      const GroupList* gl = kernel == 3 ? nullptr : group_list(p, pairs);
+      const GridArgs ga = kernel == 3 ? grid_args_w32(p, pairs)
+                                      : (gl ? grid_args_group(p, gl, pairs) : grid_args(p, pairs, kernel == 1));
       const float t = time_ms([&] {
         if (kernel == 3) launch_grid_w32(ga, st);
+        else if (gl) launch_grid_group(ga, group_size(pairs), st);
         else if (kernel == 1) launch_grid_wide(ga, st);
         else launch_grid(ga, p->ntaps, st);
       });

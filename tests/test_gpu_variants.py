@@ -14,6 +14,32 @@ def _dev(a):
     return torch.as_tensor(np.ascontiguousarray(a)).cuda()
 
 
+@pytest.mark.parametrize("n,a,C_,S", [(9, 5, 6.0, 16), (16, 7, 4.0, 5), (64, 48, 6.0, 7),
+                                      (90, 45, 7.0, 15), (130, 33, 5.0, 11), (257, 60, 6.0, 13),
+                                      (256, 300, 6.0, 16), (250, 310, 6.0, 6),
+                                      (9, 5, 6.0, 1), (64, 48, 6.0, 2), (90, 45, 7.0, 3),
+                                      (130, 33, 5.0, 4), (256, 300, 6.0, 1), (257, 310, 6.0, 4)])
+def test_group_gridding_same_bits(n, a, C_, S):
+    """Chunks of 1 to 8 pairs (whole and partly filled groups of 1, 2, 4 and 8, an odd slice at the
+    end, split centre sub-tiles at 256 x 300): the bits of the kernel whose work list the
+    groups follow, tiles up to 6 pairs and 16 pairs above (the oracle's tests hold those)."""
+    th = ph.angles_deg(a)
+    rng = np.random.default_rng(n + a)
+    centers = (n / 2 + rng.uniform(-1.5, 1.5, S)).astype(np.float32)
+    sinos = np.stack([ph.random_ellipse_sinogram(n + a + s, n, a, center=float(c))[0]
+                      for s, c in enumerate(centers)])
+    outs = []
+    for mode in (0, -1 if (S + 1) // 2 < 7 else 1):
+        with G.Plan(n, a, th, filter=G.FILTER_HANN, pswf_c=C_, max_pairs=8, wide_grid=mode) as plan:
+            M0 = plan.M0
+            o = torch.full((S, M0, max(M0, n)), float("nan"), device="cuda")
+            plan.reconstruct_batch(_dev(sinos), o, centers=_dev(centers))
+            torch.cuda.synchronize()
+            plan.device_status()
+            outs.append(o.cpu().numpy()[:, :, :M0])
+    np.testing.assert_array_equal(outs[0], outs[1])
+
+
 @pytest.mark.parametrize("n,a,S,group", [(16, 5, 1, 4), (32, 40, 3, 4), (64, 45, 7, 4),
                                          (128, 33, 5, 3), (256, 21, 2, 1)])
 def test_fbp_groups_same_bits_and_oracle(n, a, S, group):
