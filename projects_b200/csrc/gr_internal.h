@@ -124,7 +124,8 @@ struct SpectraArgs {
   int n_det, n_ang, pdim, J, pairs;
   const double* roi_off; // per angle (X0 cos + Y0 sin) pi of the ROI offset, or null
   // 0: plain [pair][dir][j]; G = wide, a power of two: the layout of gridding by G pairs,
-  // [pair / G][dir][j / 4][pair % G][j % 4], for G = 32 with the two 16-byte halves of a pair's chunk swapped when (pair / 4) is odd
+  // [pair / G][dir][j / 4][pair % G][j % 4], for G = 32 with the two 16-byte halves of a
+  // pair's chunk swapped when (pair / 4) is odd
   int wide = 0;
   // device error word for the bounded wait of the staged input (null: the rows are
   // loaded element by element, with no wait)
@@ -178,6 +179,12 @@ struct GridArgs {
   int n_long = 0;  // the items it grids by a warp each, the first of the list
 };
 
+// The part of the M0 x M0 images that a call wants: rows row0 .. row0 + rows - 1 and
+// columns col0 .. col0 + cols - 1, written from the start of the output rows.
+struct ImageWindow {
+  int row0, rows, col0, cols;
+};
+
 struct ColArgs {
   float2* H;
   const float2* tw;      // two-level twiddle table for M
@@ -185,6 +192,8 @@ struct ColArgs {
   int* err;              // device error word for bounded-wait timeouts (null: plain loads)
   int G = 0;             // columns per CTA (0: cols_group(M))
   int ring = 0;          // 1: persistent CTAs with two landing buffers (cols_ring_kernel)
+  // rows of H that are read afterwards: row iu with (iu + shift) mod M in [row0, row0 + rows)
+  int shift = 0, row0 = 0, rows = 1 << 30;
 };
 
 struct RowArgs {
@@ -197,6 +206,7 @@ struct RowArgs {
   long out_stride;
   int n_slices_valid;
   int M, M0, M02, pairs;
+  ImageWindow win;       // within the M0 x M0 image
 };
 
 // FBP comparator: OptimizedFBP's row filter on pairs of projection rows packed
@@ -236,6 +246,7 @@ int plan_create_ex(const gr_params* p, const Pswf* pswf, float (*filter_fn)(floa
 int plan_shape(const gr_plan* p, int* n_det, int* n_ang, int* M0, int* max_pairs, int* device);
 // Grow-only device scratch owned by the plan (the slice-pipeline entry points).
 int plan_scratch(gr_plan* p, size_t bytes, void** out);
+int plan_reconstruct(gr_plan* p, const gr_batch_desc* b, const ImageWindow* win, cudaStream_t st);
 
 // Makes `dev` current for the scope and restores the caller's device after.
 struct DeviceGuard {

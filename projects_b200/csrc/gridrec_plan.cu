@@ -999,7 +999,9 @@ cudaEvent_t next_event(Plan* p) {
 int launch_chunk(Plan* p, int pairs, int n_valid, int slice_base, const void* s1,
                  const void* s2, long in_pair_stride, gr_dtype dt, const float* centers,
                  const float* flat, const float* dark, long flat_stride, float* o1, float* o2,
-                 long out_pair_stride, long out_stride, cudaStream_t st) {
+                 long out_pair_stride, long out_stride, const ImageWindow* win, cudaStream_t st) {
+  const ImageWindow full{0, p->M0, 0, p->M0};
+  const ImageWindow& w = win ? *win : full;
   GR_MARK();
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
@@ -1041,10 +1043,15 @@ int launch_chunk(Plan* p, int pairs, int n_valid, int slice_base, const void* s1
                            : (wide ? launch_grid_wide(ga, st) : launch_grid(ga, p->ntaps, st)))));
   GR_MARK();
   ColArgs ca{p->d_H, p->d_tw_m, p->M, pairs, p->d_err, p->cols_G, p->cols_ring};
+  if (win) {
+    ca.shift = p->M02;
+    ca.row0 = win->row0;
+    ca.rows = win->rows;
+  }
   GR_CUDA(launch_cols(ca, st));
   GR_MARK();
   RowArgs ra{p->d_H, p->d_tw_m, p->d_winv, o1, o2, out_pair_stride, out_stride, n_valid,
-             p->M, p->M0, p->M02, pairs};
+             p->M, p->M0, p->M02, pairs, w};
   GR_CUDA(launch_rows(ra, st));
   GR_MARK();
   // (phase unless its ramps are cached, dark/log for raw counts,) spectra, grid (+ split
@@ -1064,11 +1071,12 @@ size_t dtype_size(gr_dtype dt) {
   return 0;
 }
 
-int validate_batch(const Plan* p, const gr_batch_desc* b) {
+// out_cols: the columns written of an image.
+int validate_batch(const Plan* p, const gr_batch_desc* b, int out_cols) {
   if (!b || b->n_slices < 1 || !b->sinos || !b->outs)
     return fail(GR_ERR_ARG, "batch: n_slices >= 1, sinos and outs are required");
-  if (b->out_stride < p->M0)
-    return fail(GR_ERR_ARG, "out_stride %ld < M0 %d", b->out_stride, p->M0);
+  if (b->out_stride < out_cols)
+    return fail(GR_ERR_ARG, "out_stride %ld < M0 %d", b->out_stride, out_cols);
   if (dtype_size(b->dtype) == 0) return fail(GR_ERR_ARG, "unknown dtype %d", (int)b->dtype);
   if ((b->dtype == GR_DTYPE_U16_RAW || b->dtype == GR_DTYPE_U16_LINEAR) && (!b->flat || !b->dark))
     return fail(GR_ERR_ARG, "raw uint16 dtypes need flat and dark rows");
@@ -1206,7 +1214,7 @@ int pair_host_staged(Plan* p, const float* sino1, const float* sino2, float* out
   if (cuda_err) rc = fail(GR_ERR_CUDA, "staged host-to-device copy failed");
   if (rc == GR_OK)
     rc = launch_chunk(p, 1, n_valid, 0, p->d_pair_in, p->d_pair_in + slice, 0, GR_DTYPE_F32,
-                      nullptr, nullptr, nullptr, 0, p->d_pair_out, p->d_pair_out + img, 0, p->M0, st);
+                      nullptr, nullptr, nullptr, 0, p->d_pair_out, p->d_pair_out + img, 0, p->M0, nullptr, st);
   for (size_t k = 0; k < out.size() && rc == GR_OK; ++k) {
     const OutChunk& c = out[k];
     const size_t off = (size_t)c.image * img + (size_t)c.r0 * p->M0;
@@ -1267,6 +1275,30 @@ int plan_scratch(gr_plan* p, size_t bytes, void** out) {
     p->prep_bytes = bytes;
   }
   *out = p->d_prep;
+  return GR_OK;
+}
+
+// gr_reconstruct_batch of a window of the images (within M0 x M0; null: all of it).
+int plan_reconstruct(gr_plan* p, const gr_batch_desc* b, const ImageWindow* win, cudaStream_t st) {
+  if (!p) return fail(GR_ERR_ARG, "null plan");
+  int rc = validate_batch(p, b, win ? win->cols : p->M0);
+  if (rc) return rc;
+  DeviceGuard g(p->device);
+  const size_t es = dtype_size(b->dtype);
+  const long slice_in = (long)p->n_ang * p->n_det;
+  const long slice_out = (long)(win ? win->rows : p->M0) * b->out_stride;
+  const int n_pairs = (b->n_slices + 1) / 2;
+  for (int c0 = 0; c0 < n_pairs; c0 += p->max_pairs) {
+    const int pairs = std::min(p->max_pairs, n_pairs - c0);
+    const int s0 = 2 * c0;
+    const int n_valid = std::min(2 * pairs, b->n_slices - s0);
+    const char* base = static_cast<const char*>(b->sinos) + (size_t)s0 * slice_in * es;
+    float* ob = b->outs + (size_t)s0 * slice_out;
+    rc = launch_chunk(p, pairs, n_valid, s0, base, base + slice_in * es, 2 * slice_in,
+                      b->dtype, b->centers, b->flat, b->dark, b->flat_stride, ob, ob + slice_out,
+                      2 * slice_out, b->out_stride, win, st);
+    if (rc) return rc;
+  }
   return GR_OK;
 }
 }  // namespace gr
@@ -1806,7 +1838,7 @@ int gr_reconstruct_pair(gr_plan* p, const float* sino1, const float* sino2, floa
   DeviceGuard g(p->device);
   const int n_valid = (sino2 && out2) ? 2 : 1;
   return launch_chunk(p, 1, n_valid, 0, sino1, sino2 ? sino2 : sino1, 0, GR_DTYPE_F32, nullptr,
-                      nullptr, nullptr, 0, out1, out2 ? out2 : out1, 0, out_stride,
+                      nullptr, nullptr, 0, out1, out2 ? out2 : out1, 0, out_stride, nullptr,
                       (cudaStream_t)stream);
 }
 
@@ -1833,7 +1865,7 @@ int gr_reconstruct_pair_host(gr_plan* p, const float* sino1, const float* sino2,
       GR_CUDA(cudaMemcpyAsync(p->d_pair_in + slice, sino2, slice * sizeof(float),
                               cudaMemcpyHostToDevice, st));
     rc = launch_chunk(p, 1, n_valid, 0, p->d_pair_in, p->d_pair_in + slice, 0, GR_DTYPE_F32, nullptr,
-                      nullptr, nullptr, 0, p->d_pair_out, p->d_pair_out + img, 0, p->M0, st);
+                      nullptr, nullptr, 0, p->d_pair_out, p->d_pair_out + img, 0, p->M0, nullptr, st);
     if (rc) return rc;
     const size_t row = (size_t)p->M0 * sizeof(float);
     GR_CUDA(cudaMemcpy2DAsync(out1, (size_t)out_stride * sizeof(float), p->d_pair_out, row, row,
@@ -1852,34 +1884,13 @@ int gr_reconstruct_pair_host(gr_plan* p, const float* sino1, const float* sino2,
 }
 
 int gr_reconstruct_batch(gr_plan* p, const gr_batch_desc* b, void* stream) {
-  using namespace gr;
-  if (!p) return fail(GR_ERR_ARG, "null plan");
-  int rc = validate_batch(p, b);
-  if (rc) return rc;
-  DeviceGuard g(p->device);
-  const size_t es = dtype_size(b->dtype);
-  const long slice_in = (long)p->n_ang * p->n_det;
-  const long slice_out = (long)p->M0 * b->out_stride;
-  const int n_pairs = (b->n_slices + 1) / 2;
-  for (int c0 = 0; c0 < n_pairs; c0 += p->max_pairs) {
-    const int pairs = std::min(p->max_pairs, n_pairs - c0);
-    const int s0 = 2 * c0;
-    const int n_valid = std::min(2 * pairs, b->n_slices - s0);
-    const char* base = static_cast<const char*>(b->sinos) + (size_t)s0 * slice_in * es;
-    float* ob = b->outs + (size_t)s0 * slice_out;
-    rc = launch_chunk(p, pairs, n_valid, s0, base, base + slice_in * es, 2 * slice_in,
-                      b->dtype, b->centers, b->flat, b->dark, b->flat_stride, ob, ob + slice_out,
-                      2 * slice_out,
-                      b->out_stride, (cudaStream_t)stream);
-    if (rc) return rc;
-  }
-  return GR_OK;
+  return gr::plan_reconstruct(p, b, nullptr, (cudaStream_t)stream);
 }
 
 int gr_reconstruct_host(gr_plan* p, const gr_batch_desc* b, void* stream) {
   using namespace gr;
   if (!p) return fail(GR_ERR_ARG, "null plan");
-  int rc = validate_batch(p, b);
+  int rc = validate_batch(p, b, p->M0);
   if (rc) return rc;
   DeviceGuard g(p->device);
   cudaStream_t st = (cudaStream_t)stream;
@@ -1989,7 +2000,7 @@ int gr_reconstruct_host(gr_plan* p, const gr_batch_desc* b, void* stream) {
     rc = launch_chunk(p, pairs, n_valid, s0, dbase, dbase + slice_in, 2 * slice_in_el, b->dtype,
                       d_centers, d_flat, d_dark, b->flat_stride, p->d_out[k],
                       p->d_out[k] + slice_out_el,
-                      2 * slice_out_el, b->out_stride, st);
+                      2 * slice_out_el, b->out_stride, nullptr, st);
     if (rc) { cleanup(); return rc; }
     GR_CUDA(cudaEventRecord(p->ev_comp[k], st));
     GR_CUDA(cudaStreamWaitEvent(p->d2h_stream, p->ev_comp[k], 0));
@@ -2105,7 +2116,8 @@ extern "C" int gr_reconstruct_pair_noalloc(gr_plan* p, const float* sino1, const
   // the column FFT is reported by gr_plan_device_status, as for the plan's other calls
   ColArgs ca{H, p->d_tw_m, p->M, 1, p->d_err, p->cols_G, p->cols_ring};
   GR_CUDA(launch_cols(ca, st));
-  RowArgs ra{H, p->d_tw_m, p->d_winv, out1, o2, 0, out_stride, n_valid, p->M, p->M0, p->M02, 1};
+  RowArgs ra{H, p->d_tw_m, p->d_winv, out1, o2, 0, out_stride, n_valid, p->M, p->M0, p->M02, 1,
+             {0, p->M0, 0, p->M0}};
   GR_CUDA(launch_rows(ra, st));
   // phase, spectra, grid (+ split reduction when tiles are split), cols, rows
   p->launches += 5 + (ga.n_items > 0 && ga.n_split_tiles > 0 ? 1 : 0);
@@ -2133,7 +2145,7 @@ int gr_graph_create(const gr_graph_item* items, int n_items, gr_graph** out) {
     if (!p) return fail(GR_ERR_ARG, "graph: item %d has no plan", i);
     if (p->device != dev) return fail(GR_ERR_ARG, "graph: all plans must be on one device");
     if (p->timing) return fail(GR_ERR_ARG, "graph: disable stage timing before capture");
-    int rc = validate_batch(p, &items[i].batch);
+    int rc = validate_batch(p, &items[i].batch, p->M0);
     if (rc) return rc;
     if (std::find(plans.begin(), plans.end(), p) == plans.end()) plans.push_back(p);
   }

@@ -1084,11 +1084,10 @@ int gr_reconstruct_padded(gr_plan* plan, const float* sinos, int n_slices, int n
   const int chunk = std::min(n_slices, 2 * max_pairs);
   Carve c;
   c.take<float>((size_t)chunk * n_ang * pn);
-  c.take<float>((size_t)chunk * M0 * M0);
   if ((rc = plan_scratch(plan, c.off + 256, (void**)&c.base))) return rc;
   c.off = 0;
   float* sp = c.take<float>((size_t)chunk * n_ang * pn);
-  float* rec = c.take<float>((size_t)chunk * M0 * M0);
+  const ImageWindow win{off, n_det, off, n_det};  // the crop: only it is transformed and written
   for (int s0 = 0; s0 < n_slices; s0 += chunk) {
     const int ns = std::min(chunk, n_slices - s0);
     launch_shift_pad(n_ang, ns, st, sinos + (size_t)s0 * n_ang * n_det, (long)n_ang * n_det, ns,
@@ -1098,13 +1097,9 @@ int gr_reconstruct_padded(gr_plan* plan, const float* sinos, int n_slices, int n
     b.n_slices = ns;
     b.dtype = GR_DTYPE_F32;
     b.sinos = sp;
-    b.outs = rec;
-    b.out_stride = M0;
-    if ((rc = gr_reconstruct_batch(plan, &b, st))) return rc;
-    crop_kernel<<<dim3(n_det, ns), kPrepThreads, 0, st>>>(
-        rec, M0, (long)M0 * M0, outs + (size_t)s0 * n_det * out_stride, out_stride,
-        (long)n_det * out_stride, n_det, off, 0);
-    if ((rc = check_launch("padded: crop"))) return rc;
+    b.outs = outs + (size_t)s0 * n_det * out_stride;
+    b.out_stride = out_stride;
+    if ((rc = plan_reconstruct(plan, &b, &win, st))) return rc;
   }
   return GR_OK;
 }
@@ -1129,7 +1124,8 @@ int gr_center_search(gr_plan* plan, const float* sino1, const float* sino2, int 
   cudaStream_t st = (cudaStream_t)stream;
   const int chunk = std::min(n_cand, max_pairs);  // candidates per batch (one pair each)
   const long slice_in = (long)n_ang * n_det;
-  const long slice_rec = (long)M0 * M0;
+  const long slice_rec = (long)n_det * n_det;
+  const ImageWindow win{off, n_det, off, n_det};  // the crop: only it is transformed and written
   Carve c;
   for (int pass = 0; pass < 2; ++pass) {
     if (pass == 1) {
@@ -1166,9 +1162,9 @@ int gr_center_search(gr_plan* plan, const float* sino1, const float* sino2, int 
     b.dtype = GR_DTYPE_F32;
     b.sinos = sp;
     b.outs = rec;
-    b.out_stride = M0;
-    if ((rc = gr_reconstruct_batch(plan, &b, st))) return rc;
-    Window w{rec + (size_t)off * M0 + off, M0, slice_rec, 2 * slice_rec, n_det, n_det, 2};
+    b.out_stride = n_det;
+    if ((rc = plan_reconstruct(plan, &b, &win, st))) return rc;
+    Window w{rec, n_det, slice_rec, 2 * slice_rec, n_det, n_det, 2};
     if ((rc = launch_entropy(w, nc, hist_lo, hist_hi, nbins, gh, sc + c0, st))) return rc;
   }
   e = cudaMemcpyAsync(scores, sc, n_cand * sizeof(float), cudaMemcpyDeviceToHost, st);
@@ -1186,12 +1182,9 @@ int gr_center_search(gr_plan* plan, const float* sino1, const float* sino2, int 
     b.n_slices = 2;
     b.dtype = GR_DTYPE_F32;
     b.sinos = sp;
-    b.outs = rec;
-    b.out_stride = M0;
-    if ((rc = gr_reconstruct_batch(plan, &b, st))) return rc;
-    crop_kernel<<<dim3(n_det, 2), kPrepThreads, 0, st>>>(rec, M0, slice_rec, best_images, n_det,
-                                                         (long)n_det * n_det, n_det, off, 0);
-    if ((rc = check_launch("centre search: crop"))) return rc;
+    b.outs = best_images;
+    b.out_stride = n_det;
+    if ((rc = plan_reconstruct(plan, &b, &win, st))) return rc;
   }
   return GR_OK;
 }

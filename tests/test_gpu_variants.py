@@ -115,3 +115,22 @@ def test_network_gradients_ragged_shapes(shape):
     for a, b in ((0, 144), (144, 160), (160, 2464), (2464, 2480), (2480, 2624), (2624, 2625)):
         err = np.linalg.norm(g[a:b] - ref[a:b]) / max(np.linalg.norm(ref[a:b]), 1e-30)
         assert err < 2e-2, (a, err)
+
+
+@pytest.mark.parametrize("n,a,S,pairs", [(8, 5, 1, 1), (33, 20, 3, 1), (64, 45, 5, 2), (100, 60, 4, 4)])
+def test_padded_window_same_bits(n, a, S, pairs):
+    """The padded reconstruction transforms and writes its centre window only: the bits of the
+    whole image reconstructed from the padded rows, then cropped (odd widths, an odd last
+    slice, several chunks, output rows longer than the window stay untouched beyond it)."""
+    th = ph.angles_deg(a)
+    rng = np.random.default_rng(n + S)
+    sinos = _dev(rng.uniform(0.0, 2.0, (S, a, n)).astype(np.float32))
+    with G.Plan(2 * n, a, th, filter=G.FILTER_HANN, max_pairs=pairs) as plan:
+        got = G.reconstruct_padded(plan, sinos, 0.75)
+        whole = torch.empty((S, plan.M0, max(plan.M0, 2 * n)), device="cuda")
+        padded = G.shift_pad(sinos, torch.full((S,), 0.75), out_width=2 * n)
+        plan.reconstruct_batch(padded, whole)
+        want = G.crop_center(whole, n, n // 2)
+        torch.cuda.synchronize()
+        plan.device_status()
+    np.testing.assert_array_equal(got.cpu().numpy()[..., :n], want.cpu().numpy())
