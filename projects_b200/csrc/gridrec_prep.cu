@@ -633,18 +633,25 @@ struct Window {
   int rows, cols, group;
 };
 
+// A block counts rows blockIdx.x, + gridDim.x, ... in a histogram of its own and adds its
+// counters to the group's.  Bound by the shared-memory counters (neighbouring pixels fall
+// in the same or nearby bins): 16 windows of 1024 x 1024 in 10001 bins 47 -> 43 us with one
+// reciprocal for all quotients; several rows at once or 1024 threads a block do not help
+// (44 to 63 us).
 __global__ void hist_kernel(Window w, float vmin, float inv, int nbins, unsigned* ghist) {
   extern __shared__ unsigned hist[];
   for (int b = threadIdx.x; b <= nbins; b += blockDim.x) hist[b] = 0u;
   __syncthreads();
   const int g = blockIdx.y;
   const int total_rows = w.rows * w.group;
+  const float rinv = inv >= 0x1p-40f && inv <= 0x1p40f ? __frcp_rn(inv) : 0.f;  // div_by's divisors
   for (int q = blockIdx.x; q < total_rows; q += gridDim.x) {
     const int im = q / w.rows, r = q - im * w.rows;
     const float* row = w.base + (size_t)g * w.group_stride + (size_t)im * w.image_stride +
                        (size_t)r * w.row_stride;
     for (int k = threadIdx.x; k < w.cols; k += blockDim.x) {
-      const float f = __fdiv_rn(__fsub_rn(row[k], vmin), inv);
+      const float d = __fsub_rn(row[k], vmin), m = fabsf(d);
+      const float f = rinv != 0.f && m >= kDivLo && m <= 0x1p100f ? div_by(d, inv, rinv) : __fdiv_rn(d, inv);
       const int ind = (int)f;  // NaN is skipped (a host cast gives INT_MIN for it)
       if (f == f && ind >= 0 && ind <= nbins) atomicAdd(&hist[ind], 1u);
     }
@@ -655,7 +662,11 @@ __global__ void hist_kernel(Window w, float vmin, float inv, int nbins, unsigned
     if (hist[b]) atomicAdd(&gh[b], hist[b]);
 }
 
-__global__ void entropy_final_kernel(const unsigned* ghist, int nbins, double n, float* out) {
+// One block per group, a counter per thread and pass: a chain of FP64 logarithms and
+// quotients (10001 bins: 28 us with 256 threads, 12 with 1024).
+constexpr int kEntropyThreads = 1024;
+
+__global__ void __launch_bounds__(kEntropyThreads) entropy_final_kernel(const unsigned* ghist, int nbins, double n, float* out) {
   __shared__ double red[32];
   const unsigned* gh = ghist + (size_t)blockIdx.x * (nbins + 1);
   double acc = 0.0;
@@ -683,7 +694,7 @@ int launch_entropy(const Window& w, int n_groups, float vmin, float vmax, int nb
   const int total_rows = w.rows * w.group;
   const int bx = std::max(1, std::min(total_rows, (4 * 148 + n_groups - 1) / n_groups));
   hist_kernel<<<dim3(bx, n_groups), 512, smem, st>>>(w, vmin, inv, nbins, ghist);
-  entropy_final_kernel<<<n_groups, 256, 0, st>>>(ghist, nbins,
+  entropy_final_kernel<<<n_groups, kEntropyThreads, 0, st>>>(ghist, nbins,
                                                  (double)w.rows * w.cols * w.group, out);
   e = cudaGetLastError();
   return e == cudaSuccess ? GR_OK : fail(GR_ERR_CUDA, "entropy: %s", cudaGetErrorString(e));

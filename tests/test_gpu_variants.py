@@ -134,3 +134,25 @@ def test_padded_window_same_bits(n, a, S, pairs):
         torch.cuda.synchronize()
         plan.device_status()
     np.testing.assert_array_equal(got.cpu().numpy()[..., :n], want.cpu().numpy())
+
+
+@pytest.mark.parametrize("lo,hi,nbins", [(-0.5, 1.5, 7), (0.0, 1.0, 1023), (-1e-3, 3e-3, 10000),
+                                         (0.0, 1e-30, 5), (-1e35, 1e35, 11)])
+def test_entropy_bins_at_their_edges(lo, hi, nbins):
+    """Pixels on and next to every bin edge, zeros of both signs, denormals, infinities, NaN and
+    the largest values: the counts of the float32 quotient truncated as a host cast does."""
+    inv = np.float32(np.float32(hi) - np.float32(lo)) / np.float32(nbins)
+    edges = (np.float32(lo) + np.arange(-2, nbins + 3, dtype=np.float32) * inv).astype(np.float32)
+    x = np.concatenate([edges, np.nextafter(edges, np.float32(np.inf)),
+                        np.nextafter(edges, np.float32(-np.inf)),
+                        np.float32([0.0, -0.0, 1e-45, -1e-45, np.inf, -np.inf, np.nan, 3e38, -3e38])])
+    x = np.resize(x, (2, 9, (x.size + 17) // 18)).astype(np.float32)
+    with np.errstate(all="ignore"):
+        f = ((x - np.float32(lo)) / inv).astype(np.float32)
+    f = f[np.isfinite(f) & (np.abs(f) < 2.0 ** 31)]
+    k = np.trunc(f).astype(np.int64)
+    counts = np.bincount(k[(k >= 0) & (k <= nbins)], minlength=nbins + 1)
+    p = counts[counts > 0] / x.size
+    want = -(p * np.log2(p)).sum()
+    got = G.entropy(_dev(x), lo, hi, nbins, group=2).cpu().numpy()
+    assert abs(float(got[0]) - want) <= 1e-6 * max(1.0, want)  # a float32 result
