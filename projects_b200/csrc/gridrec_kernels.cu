@@ -257,17 +257,10 @@ __device__ __forceinline__ void fft_reg(float2 (&v)[16], float2* buf, int N, int
 // The same transform with N a compile-time constant: pass radices, strides,
 // twiddle steps and swizzle offsets fold into constants (fft_reg computes them
 // at run time).  Instantiated for N = 256 .. 8192.
-template <int R, int S, int N, int Ns, bool LAST>
-__device__ __forceinline__ void fft_pass_t(float2 (&v)[16], float2* buf, int tid, const float2* lo,
-                                           const float2* hi) {
-  constexpr int B = 16 / R, NR = N / R, nthr = N / 16, tstep = N / (Ns * R);
-  static_assert(NR % 16 == 0 && Ns % 16 == 0, "offsets that keep the swizzle's low bits");
-#pragma unroll
-  for (int i = 0; i < B; ++i) {
-    const int j = tid + i * nthr;
-#pragma unroll
-    for (int r = 0; r < R; ++r) v[i * R + r] = buf[swz_at(j, r * NR) + r * NR];
-  }
+template <int R, int S, int N, int Ns>
+__device__ __forceinline__ void fft_butterflies_t(float2 (&v)[16], int tid, const float2* lo,
+                                                  const float2* hi) {
+  constexpr int B = 16 / R, nthr = N / 16, tstep = N / (Ns * R);
 #pragma unroll
   for (int i = 0; i < B; ++i) {
     const int j = tid + i * nthr;
@@ -302,6 +295,20 @@ __device__ __forceinline__ void fft_pass_t(float2 (&v)[16], float2* buf, int tid
     }
     dftR<R, S>(&v[i * R]);
   }
+}
+
+template <int R, int S, int N, int Ns, bool LAST>
+__device__ __forceinline__ void fft_pass_t(float2 (&v)[16], float2* buf, int tid, const float2* lo,
+                                           const float2* hi) {
+  constexpr int B = 16 / R, NR = N / R, nthr = N / 16;
+  static_assert(NR % 16 == 0 && Ns % 16 == 0, "offsets that keep the swizzle's low bits");
+#pragma unroll
+  for (int i = 0; i < B; ++i) {
+    const int j = tid + i * nthr;
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[i * R + r] = buf[swz_at(j, r * NR) + r * NR];
+  }
+  fft_butterflies_t<R, S, N, Ns>(v, tid, lo, hi);
   if constexpr (!LAST) {
     __syncthreads();
 #pragma unroll
@@ -336,6 +343,43 @@ __device__ __forceinline__ void fft_reg_t(float2 (&v)[16], float2* buf, int tid,
     for (int r = 0; r < 16; ++r) buf[swz(tid * 16 + r)] = v[r];
     __syncthreads();
     fft_passes_t<S, N, 16>(v, buf, tid, lo, hi);
+  }
+}
+
+// The same transform with the exchanges through N floats instead of N complex values: the
+// real parts, then the imaginary parts.  Twice the barriers, half the shared memory.  swz's
+// low bits spread floats over the banks as they do complex values (lines 32 / G floats
+// apart modulo 32, so that the G lines of a warp's threads take banks of their own).
+template <int S, int N, int Ns>
+__device__ __forceinline__ void fft_passes_split_t(float2 (&v)[16], float* buf, int tid, const float2* lo,
+                                                   const float2* hi) {
+  if constexpr (Ns < N) {
+    constexpr int rem = N / Ns, R = rem >= 16 ? 16 : rem, B = 16 / R, NR = N / R, nthr = N / 16;
+    constexpr int Rp = 16, Nsp = Ns / Rp;  // radix and span of the pass before (always 16)
+    static_assert(NR % 16 == 0, "offsets that keep the swizzle's low bits");
+    const int k = tid & (Nsp - 1), base = (tid - k) * Rp + k;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      if (Nsp > 1 || c == 1) __syncthreads();  // every thread has read buf
+#pragma unroll
+      for (int r = 0; r < 16; ++r) {
+        const int at = Nsp == 1 ? swz(base + r) : swz_at(base, r * Nsp) + r * Nsp;
+        buf[at] = c ? v[r].y : v[r].x;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < B; ++i) {
+        const int j = tid + i * nthr;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const float x = buf[swz_at(j, r * NR) + r * NR];
+          if (c) v[i * R + r].y = x;
+          else v[i * R + r].x = x;
+        }
+      }
+    }
+    fft_butterflies_t<R, S, N, Ns>(v, tid, lo, hi);
+    fft_passes_split_t<S, N, Ns * R>(v, buf, tid, lo, hi);
   }
 }
 
@@ -1921,69 +1965,65 @@ __global__ void __launch_bounds__(MAXT, 1024 / MAXT)
 }
 
 // The column FFT with persistent CTAs (as many as fit per SM): strip s = blockIdx.x + i gridDim.x
-// of G columns lands by TMA in buffer i % 2 while the previous strip is transformed
-// from the other, so the copy latency that the one-strip kernel waits out is hidden.
-// A buffer is refilled once every thread is done with it (its FFT exchange writes are
-// ordered before the copy by a proxy fence and a barrier).  Waits are bounded: on a
-// timeout the CTA records the error word, waits (bounded) for its copies in flight and
-// leaves.  Same transform, same results as cols_tma_kernel.
+// of G columns lands by TMA while the strip before it is transformed: once every thread
+// has its 16 values in registers the landing buffer is free for the next strip, and the
+// transform exchanges its values through a buffer of half the size, real and imaginary
+// parts in turn.  Waits are bounded: on a timeout the CTA records the error word, waits
+// (bounded) for its copy in flight and leaves.  Same transform, same results as
+// cols_tma_kernel.  Bound by its phases, which one CTA per SM does not overlap with each
+// other (shared-memory exchanges, butterflies), and by DRAM: at 4096 x 4096 66 us a pair
+// for 268 MB read and written, 87 with one strip of 2 columns per CTA, whose 16-byte rows use
+// half a sector.
 template <int MAXT, int NT, bool WIN>
-__global__ void __launch_bounds__(MAXT, 512 / MAXT > 0 ? 512 / MAXT : 1)
+__global__ void __launch_bounds__(MAXT, 1024 / MAXT)
     cols_ring_kernel(const __grid_constant__ CUtensorMap tmap, ColArgs a, int G, int box_rows) {
   extern __shared__ __align__(128) float2 sm[];
-  const int M = NT ? NT : a.M;
-  const int nthr = M >> 4;
+  constexpr int M = NT, nthr = NT >> 4;
   const int per_pair = M / G, total = per_pair * a.pairs;
-  const int lstride = G * M + 16;  // landing buffer: [row][g], + 16 for the exchange stride
   float2* tw = sm;
-  float2* land0 = sm + kTwSlots;
-  uint64_t* bar = reinterpret_cast<uint64_t*>(land0 + 2 * lstride);
+  float2* land = sm + kTwSlots;  // [row][g]
+  float* xch = reinterpret_cast<float*>(land + (size_t)G * M);
+  uint64_t* bar = reinterpret_cast<uint64_t*>(xch + (size_t)G * M + 32);
   const int g = threadIdx.x % G, tid = threadIdx.x / G;
   const unsigned bytes = (unsigned)(G * M) * (unsigned)sizeof(float2);
-  auto issue = [&](int s, int b) {  // one thread
+  auto issue = [&](int s) {  // one thread
     const int pair = s / per_pair, q0 = (s - pair * per_pair) * G;
-    mbar_expect_tx(&bar[b], bytes);
+    mbar_expect_tx(bar, bytes);
     for (int r = 0; r < M; r += box_rows)
-      tma_load_2d(land0 + (size_t)b * lstride + (size_t)r * G, &tmap, 2 * q0, pair * M + r, &bar[b]);
+      tma_load_2d(land + (size_t)r * G, &tmap, 2 * q0, pair * M + r, bar);
   };
   if (threadIdx.x == 0) {
-    mbar_init(&bar[0], 1);
-    mbar_init(&bar[1], 1);
+    mbar_init(bar, 1);
     fence_mbar_init();
   }
-  __syncthreads();  // the barriers are initialised before any thread polls them
-  if (threadIdx.x == 0) {
-    if ((int)blockIdx.x < total) issue(blockIdx.x, 0);
-    if ((int)(blockIdx.x + gridDim.x) < total) issue(blockIdx.x + gridDim.x, 1);
-  }
+  __syncthreads();  // the barrier is initialised before any thread polls it
+  if (threadIdx.x == 0 && (int)blockIdx.x < total) issue(blockIdx.x);
   load_twiddles(tw, a.tw, M);
-  int i = 0;
-  for (int s = blockIdx.x; s < total; s += gridDim.x, ++i) {
-    const int b = i & 1;
-    const unsigned ph = (unsigned)(i >> 1) & 1u;
-    float2* land = land0 + (size_t)b * lstride;
-    const bool ok = mbar_wait(&bar[b], ph);
-    if (__syncthreads_or(!ok)) {
+  unsigned ph = 0;
+  for (int s = blockIdx.x; s < total; s += gridDim.x) {
+    const bool ok = mbar_wait(bar, ph);
+    if (__syncthreads_or(!ok)) {  // (also: every thread has left the strip before)
       if (threadIdx.x == 0) {
         atomicExch(a.err, 1);
-        mbar_wait(&bar[b], ph);  // this strip's copy
-        if (s + (int)gridDim.x < total) mbar_wait(&bar[b ^ 1], (unsigned)((i + 1) >> 1) & 1u);
+        mbar_wait(bar, ph);
       }
       __syncthreads();
       return;
     }
+    ph ^= 1u;
     float2 v[16];
 #pragma unroll
     for (int r = 0; r < 16; ++r) v[r] = land[(tid + r * nthr) * G + g];
-    __syncthreads();  // inputs read before the landing buffer becomes the exchange buffer
-    fft_line<-1, NT>(v, land + g * (M + 16 / G), M, tid, nthr, tw, tw + 64);
+    __syncthreads();  // every thread has its values: the landing buffer is free
+    if (threadIdx.x == 0 && s + (int)gridDim.x < total) {
+      fence_proxy_async();
+      issue(s + gridDim.x);
+    }
+    dft16<-1>(v);
+    fft_passes_split_t<-1, NT, 16>(v, xch + g * (M + 32 / G), tid, tw, tw + 64);
     const int pair = s / per_pair, q0 = (s - pair * per_pair) * G;
     float2* Hp = a.H + (size_t)pair * M * M + q0 + g;
     store_column<NT, WIN>(a, Hp, v, M, tid, nthr);
-    // every thread's exchange accesses of this buffer come before the copy that refills it
-    fence_proxy_async();
-    __syncthreads();
-    if (threadIdx.x == 0 && s + 2 * (int)gridDim.x < total) issue(s + 2 * gridDim.x, b);
   }
 }
 
@@ -2147,12 +2187,14 @@ void add_fft_kernels(std::vector<const void*>& f) {
   f.push_back((const void*)cols_tma_kernel<512, NT, true>);
   f.push_back((const void*)cols_tma_kernel<1024, NT, false>);
   f.push_back((const void*)cols_tma_kernel<1024, NT, true>);
-  f.push_back((const void*)cols_ring_kernel<256, NT, false>);
-  f.push_back((const void*)cols_ring_kernel<256, NT, true>);
-  f.push_back((const void*)cols_ring_kernel<512, NT, false>);
-  f.push_back((const void*)cols_ring_kernel<512, NT, true>);
-  f.push_back((const void*)cols_ring_kernel<1024, NT, false>);
-  f.push_back((const void*)cols_ring_kernel<1024, NT, true>);
+  if constexpr (NT > 0) {
+    f.push_back((const void*)cols_ring_kernel<256, NT, false>);
+    f.push_back((const void*)cols_ring_kernel<256, NT, true>);
+    f.push_back((const void*)cols_ring_kernel<512, NT, false>);
+    f.push_back((const void*)cols_ring_kernel<512, NT, true>);
+    f.push_back((const void*)cols_ring_kernel<1024, NT, false>);
+    f.push_back((const void*)cols_ring_kernel<1024, NT, true>);
+  }
   f.push_back((const void*)rows_kernel<256, NT>);
   f.push_back((const void*)rows_kernel<512, NT>);
   f.push_back((const void*)fbp_filter_kernel<256, NT>);
@@ -2353,8 +2395,18 @@ cudaError_t launch_grid_tc(const GridArgs& a, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-int cols_group(int M) {
-  int g = 8192 / M;  // G * M / 16 <= 512 threads; G = 4 (32-byte rows) at M = 2048
+// Default form of the column FFT.  us per pair, one strip per CTA (G columns) against the
+// persistent kernel: M = 4096 86.5 (G = 2; 84.8 with 4) against 66.3 (G = 4); M = 2048 14.9 (G =
+// 4; 18.0 with 8) against 14.4 (G = 8; 17.7 with 4) for 32 pairs, 17.4 against 17.0 for 4,
+// even for one; M = 1024 3.5 against 3.9, 512 1.2 against 1.4 (G = 8).  At M = 8192 no
+// persistent form has strips wide enough: 519 with G = 2, 931 with 1, 600 persistent.
+int cols_ring_default(int M) { return M == 2048 || M == 4096; }
+
+// Columns per CTA: up to 512 threads of M / 16 a column, 1024 where narrower strips would
+// leave the 32-byte sectors of a row half used (M = 8192) and for the persistent kernel,
+// whose one CTA per SM takes them all.
+int cols_group(int M, int ring) {
+  const int g = (ring || M >= 8192 ? 16384 : 8192) / M;
   return g < 1 ? 1 : (g > 8 ? 8 : g);
 }
 
@@ -2376,7 +2428,7 @@ static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 
 template <bool WIN>
 static cudaError_t launch_cols_t(const ColArgs& a, cudaStream_t s) {
-  const int G = a.G > 0 ? a.G : cols_group(a.M);
+  const int G = a.G > 0 ? a.G : cols_group(a.M, a.ring);
   const int threads = G * (a.M / 16);
   PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
   if (a.err && encode && G >= 2 && a.M >= 16 && ((uintptr_t)a.H % 16) == 0) {
@@ -2394,21 +2446,20 @@ static cudaError_t launch_cols_t(const ColArgs& a, cudaStream_t s) {
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int ring_smem = (kTwSlots + 2 * (G * a.M + 16)) * (int)sizeof(float2) + 2 * (int)sizeof(uint64_t);
-    if (r == CUDA_SUCCESS && a.ring && ring_smem <= optin) {
+    const int ring_smem = (kTwSlots + G * a.M) * (int)sizeof(float2) + (G * a.M + 32) * (int)sizeof(float) +
+                          (int)sizeof(uint64_t);
+    if (r == CUDA_SUCCESS && a.ring && a.M >= 256 && ring_smem <= optin) {
       const int total = (a.M / G) * a.pairs;
       // persistent: as many CTAs as fit on the SMs at once
 #define GR_COLR(NT)                                                                              \
-  {                                                                                              \
-    const void* fn = threads <= 256 ? (const void*)cols_ring_kernel<256, NT, WIN>                     \
-                     : threads <= 512 ? (const void*)cols_ring_kernel<512, NT, WIN>                   \
-                                      : (const void*)cols_ring_kernel<1024, NT, WIN>;                 \
+  if constexpr (NT > 0) {                                                                        \
+    const auto fn = threads <= 256 ? cols_ring_kernel<256, NT, WIN>                              \
+                    : threads <= 512 ? cols_ring_kernel<512, NT, WIN>                            \
+                                     : cols_ring_kernel<1024, NT, WIN>;                          \
     int per_sm = 0;                                                                              \
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, ring_smem);              \
     const int blocks = std::min(total, std::max(per_sm, 1) * std::max(sms, 1));                  \
-    if (threads <= 256) cols_ring_kernel<256, NT, WIN><<<blocks, threads, ring_smem, s>>>(map, a, G, box_rows); \
-    else if (threads <= 512) cols_ring_kernel<512, NT, WIN><<<blocks, threads, ring_smem, s>>>(map, a, G, box_rows); \
-    else cols_ring_kernel<1024, NT, WIN><<<blocks, threads, ring_smem, s>>>(map, a, G, box_rows);      \
+    fn<<<blocks, threads, ring_smem, s>>>(map, a, G, box_rows);                                  \
   }
       GR_DISPATCH_N(a.M, GR_COLR)
 #undef GR_COLR
@@ -2438,7 +2489,11 @@ static cudaError_t launch_cols_t(const ColArgs& a, cudaStream_t s) {
 #undef GR_COL
   return cudaGetLastError();
 }
-cudaError_t launch_cols(const ColArgs& a, cudaStream_t s) {
+cudaError_t launch_cols(const ColArgs& args, cudaStream_t s) {
+  ColArgs a = args;
+  // by default the persistent kernel wants two strips per SM (one pair at M = 2048: 194.9
+  // us a call with it, 194.4 without)
+  if (a.G <= 0 && a.ring && (long)(a.M / cols_group(a.M, 1)) * a.pairs < 2 * 148) a.ring = 0;
   return a.rows < a.M ? launch_cols_t<true>(a, s) : launch_cols_t<false>(a, s);
 }
 

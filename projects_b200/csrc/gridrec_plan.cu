@@ -177,8 +177,8 @@ struct Plan {
   // gridding by groups of pairs (grid_group_kernel), with the sums in the order of the tile
   // kernel's list and of the 16-pair kernel's
   GroupList g_tiles, g_wide;
-  int cols_G = 0;                   // column-FFT group width (0 = cols_group(M); autotuned)
-  int cols_ring = 0;                // 1: persistent double-buffered column FFT (autotuned)
+  int cols_G = 0;                   // column-FFT group width (0 = cols_group(M, ring); autotuned)
+  int cols_ring = 0;                // 1: persistent column FFT (cols_ring_default(M); autotuned)
   // gridding kernel of full chunks (max_pairs pairs) in the default mode, chosen by the
   // autotuner or gr_plan_set_tuning: 0 tiles, 1 16-pair, 3 32-pair (-1: by chunk size)
   int tuned_kernel = -1;
@@ -1401,6 +1401,7 @@ int gr::plan_create_ex(const gr_params* prm, const Pswf* pswf, float (*filter_fn
   p->pdim = (int)pdim;
   p->J = (int)(pdim / 2);
   p->M = (int)M;
+  p->cols_ring = cols_ring_default(p->M);
   p->M02 = (int)M02;
   p->M0 = (int)geo.M0;
   p->sampl = geo.sampl;
@@ -1816,7 +1817,7 @@ int gr_plan_tuning(const gr_plan* p, int* item_cap, int* cols_group_width) {
   // the item cap of the work list a full chunk grids with
   const bool wl4x8 = gr::use_wide(p, p->max_pairs) || gr::use_w32(p, p->max_pairs);
   if (item_cap) *item_cap = wl4x8 ? p->w_item_cap : p->item_cap;
-  if (cols_group_width) *cols_group_width = p->cols_G > 0 ? p->cols_G : gr::cols_group(p->M);
+  if (cols_group_width) *cols_group_width = p->cols_G > 0 ? p->cols_G : gr::cols_group(p->M, p->cols_ring);
   return GR_OK;
 }
 

@@ -117,7 +117,8 @@ def test_network_gradients_ragged_shapes(shape):
         assert err < 2e-2, (a, err)
 
 
-@pytest.mark.parametrize("n,a,S,pairs", [(8, 5, 1, 1), (33, 20, 3, 1), (64, 45, 5, 2), (100, 60, 4, 4)])
+@pytest.mark.parametrize("n,a,S,pairs", [(8, 5, 1, 1), (33, 20, 3, 1), (64, 45, 5, 2), (100, 60, 4, 4),
+                                           (600, 9, 3, 2), (1030, 6, 3, 1)])
 def test_padded_window_same_bits(n, a, S, pairs):
     """The padded reconstruction transforms and writes its centre window only: the bits of the
     whole image reconstructed from the padded rows, then cropped (odd widths, an odd last
@@ -156,3 +157,23 @@ def test_entropy_bins_at_their_edges(lo, hi, nbins):
     want = -(p * np.log2(p)).sum()
     got = G.entropy(_dev(x), lo, hi, nbins, group=2).cpu().numpy()
     assert abs(float(got[0]) - want) <= 1e-6 * max(1.0, want)  # a float32 result
+
+
+@pytest.mark.parametrize("n,ring_group", [(200, 8), (512, 8), (600, 8), (1100, 4), (2100, 4), (4100, 2)])
+def test_persistent_columns_same_bits(n, ring_group):
+    """The persistent column FFT at M = 256 .. 8192 (widest strips of each) against one strip
+    per block on the same input."""
+    a, S = 7, 3
+    rng = np.random.default_rng(n)
+    sinos = _dev(rng.uniform(0.0, 2.0, (S, a, n)).astype(np.float32))
+    outs = []
+    with G.Plan(n, a, ph.angles_deg(a), filter=G.FILTER_HANN, max_pairs=1) as plan:
+        for g, ring in ((0, None), (2, False), (ring_group, True)):
+            plan.set_tuning(cols_group=g, cols_ring=ring)
+            o = torch.full((S, plan.M0, max(plan.M0, n)), float("nan"), device="cuda")
+            plan.reconstruct_batch(sinos, o)
+            torch.cuda.synchronize()
+            plan.device_status()
+            outs.append(o.cpu().numpy()[:, :, :plan.M0])
+    np.testing.assert_array_equal(outs[0], outs[1])
+    np.testing.assert_array_equal(outs[2], outs[1])
