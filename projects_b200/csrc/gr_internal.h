@@ -134,6 +134,11 @@ struct SpectraArgs {
   // (launch_dark_log), so that a sample costs one load and one logarithm; null: the
   // flat and dark rows above are read per sample
   const float2* dl = nullptr;
+  // sub-pixel shift and half padding of the rows on the way (see PaddedInput): n_det is
+  // then the length of the given rows
+  bool padded = false;
+  const float* shift = nullptr;
+  float shift_const = 0.f;
 };
 
 struct PhaseArgs {
@@ -183,6 +188,18 @@ struct GridArgs {
 // columns col0 .. col0 + cols - 1, written from the start of the output rows.
 struct ImageWindow {
   int row0, rows, col0, cols;
+};
+
+// Float rows of n values to be shifted and half padded (gr_shift_pad's values) to the
+// plan's width: pair p's slices at s1 / s2 + p * pair_stride, shifted by shift[p]
+// (shift_const where shift is null).
+struct PaddedInput {
+  const float* s1;
+  const float* s2;
+  long pair_stride;
+  int n;
+  const float* shift;
+  float shift_const;
 };
 
 struct ColArgs {
@@ -246,7 +263,9 @@ int plan_create_ex(const gr_params* p, const Pswf* pswf, float (*filter_fn)(floa
 int plan_shape(const gr_plan* p, int* n_det, int* n_ang, int* M0, int* max_pairs, int* device);
 // Grow-only device scratch owned by the plan (the slice-pipeline entry points).
 int plan_scratch(gr_plan* p, size_t bytes, void** out);
-int plan_reconstruct(gr_plan* p, const gr_batch_desc* b, const ImageWindow* win, cudaStream_t st);
+int plan_reconstruct(gr_plan* p, const gr_batch_desc* b, cudaStream_t st);
+int plan_reconstruct_padded(gr_plan* p, const PaddedInput& in, int n_slices, float* outs, long out_stride,
+                            const ImageWindow& win, cudaStream_t st);
 
 // Makes `dev` current for the scope and restores the caller's device after.
 struct DeviceGuard {

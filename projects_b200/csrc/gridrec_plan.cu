@@ -999,7 +999,7 @@ cudaEvent_t next_event(Plan* p) {
 int launch_chunk(Plan* p, int pairs, int n_valid, int slice_base, const void* s1,
                  const void* s2, long in_pair_stride, gr_dtype dt, const float* centers,
                  const float* flat, const float* dark, long flat_stride, float* o1, float* o2,
-                 long out_pair_stride, long out_stride, const ImageWindow* win, cudaStream_t st) {
+                 long out_pair_stride, long out_stride, const ImageWindow* win, cudaStream_t st, const PaddedInput* pad = nullptr) {
   const ImageWindow full{0, p->M0, 0, p->M0};
   const ImageWindow& w = win ? *win : full;
   GR_MARK();
@@ -1032,6 +1032,12 @@ int launch_chunk(Plan* p, int pairs, int n_valid, int slice_base, const void* s1
                  p->d_tw_p, p->n_det, p->n_ang, p->pdim, p->J, pairs, p->d_roi_off,
                  w32 ? kW32Pairs : ((wide || tc) ? kWidePairs : (grp > 1 ? grp : 0)), p->d_err};
   if (dl) sa.dl = p->d_dl;
+  if (pad) {
+    sa.padded = true;
+    sa.n_det = pad->n;
+    sa.shift = pad->shift;
+    sa.shift_const = pad->shift_const;
+  }
   GR_CUDA(launch_spectra(sa, dt, st));
   GR_MARK();
   const GridArgs ga = tc ? grid_args_tc(p, pairs)
@@ -1071,12 +1077,11 @@ size_t dtype_size(gr_dtype dt) {
   return 0;
 }
 
-// out_cols: the columns written of an image.
-int validate_batch(const Plan* p, const gr_batch_desc* b, int out_cols) {
+int validate_batch(const Plan* p, const gr_batch_desc* b) {
   if (!b || b->n_slices < 1 || !b->sinos || !b->outs)
     return fail(GR_ERR_ARG, "batch: n_slices >= 1, sinos and outs are required");
-  if (b->out_stride < out_cols)
-    return fail(GR_ERR_ARG, "out_stride %ld < M0 %d", b->out_stride, out_cols);
+  if (b->out_stride < p->M0)
+    return fail(GR_ERR_ARG, "out_stride %ld < M0 %d", b->out_stride, p->M0);
   if (dtype_size(b->dtype) == 0) return fail(GR_ERR_ARG, "unknown dtype %d", (int)b->dtype);
   if ((b->dtype == GR_DTYPE_U16_RAW || b->dtype == GR_DTYPE_U16_LINEAR) && (!b->flat || !b->dark))
     return fail(GR_ERR_ARG, "raw uint16 dtypes need flat and dark rows");
@@ -1278,15 +1283,14 @@ int plan_scratch(gr_plan* p, size_t bytes, void** out) {
   return GR_OK;
 }
 
-// gr_reconstruct_batch of a window of the images (within M0 x M0; null: all of it).
-int plan_reconstruct(gr_plan* p, const gr_batch_desc* b, const ImageWindow* win, cudaStream_t st) {
+int plan_reconstruct(gr_plan* p, const gr_batch_desc* b, cudaStream_t st) {
   if (!p) return fail(GR_ERR_ARG, "null plan");
-  int rc = validate_batch(p, b, win ? win->cols : p->M0);
+  int rc = validate_batch(p, b);
   if (rc) return rc;
   DeviceGuard g(p->device);
   const size_t es = dtype_size(b->dtype);
   const long slice_in = (long)p->n_ang * p->n_det;
-  const long slice_out = (long)(win ? win->rows : p->M0) * b->out_stride;
+  const long slice_out = (long)p->M0 * b->out_stride;
   const int n_pairs = (b->n_slices + 1) / 2;
   for (int c0 = 0; c0 < n_pairs; c0 += p->max_pairs) {
     const int pairs = std::min(p->max_pairs, n_pairs - c0);
@@ -1296,7 +1300,29 @@ int plan_reconstruct(gr_plan* p, const gr_batch_desc* b, const ImageWindow* win,
     float* ob = b->outs + (size_t)s0 * slice_out;
     rc = launch_chunk(p, pairs, n_valid, s0, base, base + slice_in * es, 2 * slice_in,
                       b->dtype, b->centers, b->flat, b->dark, b->flat_stride, ob, ob + slice_out,
-                      2 * slice_out, b->out_stride, win, st);
+                      2 * slice_out, b->out_stride, nullptr, st);
+    if (rc) return rc;
+  }
+  return GR_OK;
+}
+
+// Padded reconstruction of the given rows; only the window of the images is written
+// (out_stride >= its columns).
+int plan_reconstruct_padded(gr_plan* p, const PaddedInput& in, int n_slices, float* outs, long out_stride,
+                            const ImageWindow& win, cudaStream_t st) {
+  DeviceGuard g(p->device);
+  const long slice_out = (long)win.rows * out_stride;
+  const int n_pairs = (n_slices + 1) / 2;
+  for (int c0 = 0; c0 < n_pairs; c0 += p->max_pairs) {
+    const int pairs = std::min(p->max_pairs, n_pairs - c0);
+    PaddedInput chunk = in;
+    chunk.s1 += c0 * in.pair_stride;
+    chunk.s2 += c0 * in.pair_stride;
+    if (chunk.shift) chunk.shift += c0;
+    float* ob = outs + (size_t)(2 * c0) * slice_out;
+    const int rc = launch_chunk(p, pairs, std::min(2 * pairs, n_slices - 2 * c0), 2 * c0, chunk.s1,
+                                chunk.s2, in.pair_stride, GR_DTYPE_F32, nullptr, nullptr, nullptr, 0, ob,
+                                ob + slice_out, 2 * slice_out, out_stride, &win, st, &chunk);
     if (rc) return rc;
   }
   return GR_OK;
@@ -1885,13 +1911,13 @@ int gr_reconstruct_pair_host(gr_plan* p, const float* sino1, const float* sino2,
 }
 
 int gr_reconstruct_batch(gr_plan* p, const gr_batch_desc* b, void* stream) {
-  return gr::plan_reconstruct(p, b, nullptr, (cudaStream_t)stream);
+  return gr::plan_reconstruct(p, b, (cudaStream_t)stream);
 }
 
 int gr_reconstruct_host(gr_plan* p, const gr_batch_desc* b, void* stream) {
   using namespace gr;
   if (!p) return fail(GR_ERR_ARG, "null plan");
-  int rc = validate_batch(p, b, p->M0);
+  int rc = validate_batch(p, b);
   if (rc) return rc;
   DeviceGuard g(p->device);
   cudaStream_t st = (cudaStream_t)stream;
@@ -2146,7 +2172,7 @@ int gr_graph_create(const gr_graph_item* items, int n_items, gr_graph** out) {
     if (!p) return fail(GR_ERR_ARG, "graph: item %d has no plan", i);
     if (p->device != dev) return fail(GR_ERR_ARG, "graph: all plans must be on one device");
     if (p->timing) return fail(GR_ERR_ARG, "graph: disable stage timing before capture");
-    int rc = validate_batch(p, &items[i].batch, p->M0);
+    int rc = validate_batch(p, &items[i].batch);
     if (rc) return rc;
     if (std::find(plans.begin(), plans.end(), p) == plans.end()) plans.push_back(p);
   }

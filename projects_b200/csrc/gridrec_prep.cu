@@ -1092,27 +1092,10 @@ int gr_reconstruct_padded(gr_plan* plan, const float* sinos, int n_slices, int n
                 off + n_det, M0);
   DeviceGuard guard(dev);
   cudaStream_t st = (cudaStream_t)stream;
-  const int chunk = std::min(n_slices, 2 * max_pairs);
-  Carve c;
-  c.take<float>((size_t)chunk * n_ang * pn);
-  if ((rc = plan_scratch(plan, c.off + 256, (void**)&c.base))) return rc;
-  c.off = 0;
-  float* sp = c.take<float>((size_t)chunk * n_ang * pn);
-  const ImageWindow win{off, n_det, off, n_det};  // the crop: only it is transformed and written
-  for (int s0 = 0; s0 < n_slices; s0 += chunk) {
-    const int ns = std::min(chunk, n_slices - s0);
-    launch_shift_pad(n_ang, ns, st, sinos + (size_t)s0 * n_ang * n_det, (long)n_ang * n_det, ns,
-                     nullptr, 1, xoffset, sp, n_det, pn);
-    if ((rc = check_launch("padded: shift/pad"))) return rc;
-    gr_batch_desc b{};
-    b.n_slices = ns;
-    b.dtype = GR_DTYPE_F32;
-    b.sinos = sp;
-    b.outs = outs + (size_t)s0 * n_det * out_stride;
-    b.out_stride = out_stride;
-    if ((rc = plan_reconstruct(plan, &b, &win, st))) return rc;
-  }
-  return GR_OK;
+  // shifted and padded as the spectra are formed; only the crop is transformed and written
+  const long slice_in = (long)n_ang * n_det;
+  const PaddedInput in{sinos, sinos + slice_in, 2 * slice_in, n_det, nullptr, xoffset};
+  return plan_reconstruct_padded(plan, in, n_slices, outs, out_stride, {off, n_det, off, n_det}, st);
 }
 
 int gr_center_search(gr_plan* plan, const float* sino1, const float* sino2, int n_det, int n_ang,
@@ -1134,7 +1117,6 @@ int gr_center_search(gr_plan* plan, const float* sino1, const float* sino2, int 
   DeviceGuard guard(dev);
   cudaStream_t st = (cudaStream_t)stream;
   const int chunk = std::min(n_cand, max_pairs);  // candidates per batch (one pair each)
-  const long slice_in = (long)n_ang * n_det;
   const long slice_rec = (long)n_det * n_det;
   const ImageWindow win{off, n_det, off, n_det};  // the crop: only it is transformed and written
   Carve c;
@@ -1143,38 +1125,23 @@ int gr_center_search(gr_plan* plan, const float* sino1, const float* sino2, int 
       if ((rc = plan_scratch(plan, c.off + 256, (void**)&c.base))) return rc;
       c.off = 0;
     }
-    c.take<float>(2 * slice_in);
-    c.take<float>((size_t)2 * chunk * n_ang * pn);
     c.take<float>((size_t)2 * chunk * slice_rec);
     c.take<float>(n_cand);
     c.take<unsigned>((size_t)chunk * (nbins + 1));
     c.take<float>(n_cand);
   }
   c.off = 0;
-  float* pr = c.take<float>(2 * slice_in);
-  float* sp = c.take<float>((size_t)2 * chunk * n_ang * pn);
   float* rec = c.take<float>((size_t)2 * chunk * slice_rec);
   float* xo = c.take<float>(n_cand);
   unsigned* gh = c.take<unsigned>((size_t)chunk * (nbins + 1));
   float* sc = c.take<float>(n_cand);
-  cudaError_t e = cudaMemcpyAsync(pr, sino1, slice_in * sizeof(float), cudaMemcpyDeviceToDevice, st);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(pr + slice_in, sino2, slice_in * sizeof(float), cudaMemcpyDeviceToDevice,
-                        st);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(xo, shifts, n_cand * sizeof(float), cudaMemcpyHostToDevice, st);
+  cudaError_t e = cudaMemcpyAsync(xo, shifts, n_cand * sizeof(float), cudaMemcpyHostToDevice, st);
   if (e != cudaSuccess) return cuda_fail(e, "centre search: copies");
   for (int c0 = 0; c0 < n_cand; c0 += chunk) {
     const int nc = std::min(chunk, n_cand - c0);
-    launch_shift_pad(n_ang, 2 * nc, st, pr, slice_in, 2, xo + c0, 2, 0.f, sp, n_det, pn);
-    if ((rc = check_launch("centre search: shift/pad"))) return rc;
-    gr_batch_desc b{};
-    b.n_slices = 2 * nc;
-    b.dtype = GR_DTYPE_F32;
-    b.sinos = sp;
-    b.outs = rec;
-    b.out_stride = n_det;
-    if ((rc = plan_reconstruct(plan, &b, &win, st))) return rc;
+    // every pair of the chunk is the given pair of slices, with the candidate's shift
+    const PaddedInput in{sino1, sino2, 0, n_det, xo + c0, 0.f};
+    if ((rc = plan_reconstruct_padded(plan, in, 2 * nc, rec, n_det, win, st))) return rc;
     Window w{rec, n_det, slice_rec, 2 * slice_rec, n_det, n_det, 2};
     if ((rc = launch_entropy(w, nc, hist_lo, hist_hi, nbins, gh, sc + c0, st))) return rc;
   }
@@ -1187,15 +1154,8 @@ int gr_center_search(gr_plan* plan, const float* sino1, const float* sino2, int 
     if (scores[k] < scores[bi]) bi = k;
   if (best) *best = bi;
   if (best_images) {
-    launch_shift_pad(n_ang, 2, st, pr, slice_in, 2, xo + bi, 2, 0.f, sp, n_det, pn);
-    if ((rc = check_launch("centre search: shift/pad"))) return rc;
-    gr_batch_desc b{};
-    b.n_slices = 2;
-    b.dtype = GR_DTYPE_F32;
-    b.sinos = sp;
-    b.outs = best_images;
-    b.out_stride = n_det;
-    if ((rc = plan_reconstruct(plan, &b, &win, st))) return rc;
+    const PaddedInput in{sino1, sino2, 0, n_det, xo + bi, 0.f};
+    if ((rc = plan_reconstruct_padded(plan, in, 2, best_images, n_det, win, st))) return rc;
   }
   return GR_OK;
 }

@@ -120,16 +120,18 @@ def test_network_gradients_ragged_shapes(shape):
 @pytest.mark.parametrize("n,a,S,pairs", [(8, 5, 1, 1), (33, 20, 3, 1), (64, 45, 5, 2), (100, 60, 4, 4),
                                            (600, 9, 3, 2), (1030, 6, 3, 1)])
 def test_padded_window_same_bits(n, a, S, pairs):
-    """The padded reconstruction transforms and writes its centre window only: the bits of the
-    whole image reconstructed from the padded rows, then cropped (odd widths, an odd last
-    slice, several chunks, output rows longer than the window stay untouched beyond it)."""
+    """The padded reconstruction shifts and pads as it forms the spectra and transforms and
+    writes its centre window only: the bits of the whole image reconstructed from the
+    padded rows, then cropped (rows aligned and not, odd widths, an odd last slice, several
+    chunks)."""
     th = ph.angles_deg(a)
     rng = np.random.default_rng(n + S)
     sinos = _dev(rng.uniform(0.0, 2.0, (S, a, n)).astype(np.float32))
+    shift = 0.75 if S != 3 else -1.5 - 2 * n  # taps inside the row, all beyond its end
     with G.Plan(2 * n, a, th, filter=G.FILTER_HANN, max_pairs=pairs) as plan:
-        got = G.reconstruct_padded(plan, sinos, 0.75)
+        got = G.reconstruct_padded(plan, sinos, shift)
         whole = torch.empty((S, plan.M0, max(plan.M0, 2 * n)), device="cuda")
-        padded = G.shift_pad(sinos, torch.full((S,), 0.75), out_width=2 * n)
+        padded = G.shift_pad(sinos, torch.full((S,), shift), out_width=2 * n)
         plan.reconstruct_batch(padded, whole)
         want = G.crop_center(whole, n, n // 2)
         torch.cuda.synchronize()
