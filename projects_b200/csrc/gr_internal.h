@@ -63,11 +63,16 @@ struct alignas(32) TapRec {
   unsigned pad;
 };
 constexpr int kGrpMinBlocks = 4;
+// Lanes over which a bundle spreads the rows of an item for one pair: 4 of one row each for
+// two pairs (4 items a bundle; 16 items of 4 rows cost more table lookups per step taken:
+// 88 against 105 us a pair at 2048 x 1500, 30 against 33 at 1024 x 720), else 1 (4 pairs: 64
+// against 58 at 2048 x 1500; one pair: 40 against 36 at 512 x 360).
+constexpr int grp_row_split(int G) { return G == 2 ? 4 : 1; }
 // It grids chunks of up to kGroupPairs pairs by default (gr_params.wide_grid = 0), those of
 // one pair only where the list has at most kGroupOneItems sub-tiles (M <= 1024).  Per pair
 // against the kernel that took the chunk otherwise (the tile kernel up to 6 pairs, the
 // 16-pair kernel above), us at 1024 x 720 and 2048 x 1500: 8 pairs 12.2 / 19.7 and 35.3 /
-// 71.0, 6 pairs 17.5 / 29.0 and 53.6 / 89.7, 4 pairs 20 / 31 and 58 / 95, 2 pairs 33 / 57 and 108 /
+// 71.0, 6 pairs 17.5 / 29.0 and 53.6 / 89.7, 4 pairs 20 / 31 and 58 / 95, 2 pairs 30 / 57 and 88 /
 // 110, one pair 60 / 97 and 205 / 133 (32 items of a bundle for one pair cost more table
 // lookups than the tile kernel's pass over them).  For 9 to 16 pairs two groups cost what the
 // 16-pair kernel does, for more the 32-pair kernel is faster (31 a pair).

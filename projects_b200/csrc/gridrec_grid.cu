@@ -15,13 +15,13 @@ namespace gr {
 // The same gather as grid_kernel -- the work-list geometry, tap set and
 // nearest-neighbour weights of gridrec.cu:546-566 -- for chunks of a few slice pairs.
 // A work item is one kWideRows x kWideCols (4 x 8) sub-tile of H and the samples whose
-// taps reach it.  A warp grids for G pairs either a bundle of Q = 32 / G items of similar
-// length at once -- lane q * G + p holds pair p's cells of item q in registers -- or one
-// long item, lane q * G + p holding pair p's G cells q * G .. of it:
+// taps reach it.  A warp grids for G pairs either a bundle of Q = 32 / (G RS) items of similar
+// length at once -- RS lanes hold pair p's cells of item q in registers, 4 / RS rows each --
+// or one long item, lane q * G + p holding pair p's G cells q * G .. of it:
 // * no shared-memory read-modify-write, no atomics, no idle lanes for few pairs; per sample
 //   a tap adds w_c (w_r value) by packed FMAs over pairs of columns, real and imaginary
 //   parts apart, so that the column weights are used as they lie in shared memory.
-// * a bundle reads a sample's 12 weights once for 32 cells of its lane, a long item once for
+// * a bundle reads a sample's weights once for 32 cells of its lane (RS = 1), a long item once for
 //   G cells: about a quarter slower per sample at G = 8, but a long item's samples pass 3 to
 //   4 times as fast, and no warp holds one when the others have ended.
 // * the geometry depends on the plan only: tap_record_kernel computes, once per work list, a
@@ -159,17 +159,24 @@ struct GrpCell2 {
   float2 re, im;
 };
 
-// One sample: x_r = w_r * value, then acc += w_c x_r; wts: the weights of rows 0..3,
-// then columns 0..7.
-__device__ __forceinline__ void grp_apply(GrpCell2 (&acc)[kWideRows][kWideCols / 2], float2 v,
-                                          const unsigned char* wts) {
+// One sample on this lane's R rows: x_r = w_r * value, then acc += w_c x_r; wts: the weights
+// of rows 0..3, then columns 0..7; row0: the first of the lane's rows.
+template <int R>
+__device__ __forceinline__ void grp_apply(GrpCell2 (&acc)[R][kWideCols / 2], float2 v,
+                                          const unsigned char* wts, int row0) {
   const float4* d = reinterpret_cast<const float4*>(wts);
-  const float4 rw = d[0], c0 = d[1], c1 = d[2];
-  const float wr[4] = {rw.x, rw.y, rw.z, rw.w};
+  float wr[4];
+  if (R == 4) {
+    const float4 rw = d[0];
+    wr[0] = rw.x, wr[1] = rw.y, wr[2] = rw.z, wr[3] = rw.w;
+  } else {
+    wr[0] = reinterpret_cast<const float*>(wts)[row0];
+  }
+  const float4 c0 = d[1], c1 = d[2];
   const float2 wc[4] = {make_float2(c0.x, c0.y), make_float2(c0.z, c0.w), make_float2(c1.x, c1.y),
                         make_float2(c1.z, c1.w)};
 #pragma unroll
-  for (int r = 0; r < 4; ++r) {
+  for (int r = 0; r < R; ++r) {
     const float xr = __fmul_rn(wr[r], v.x), xi = __fmul_rn(wr[r], v.y);
     const float2 x2 = make_float2(xr, xr), y2 = make_float2(xi, xi);
 #pragma unroll
@@ -229,9 +236,11 @@ __device__ __forceinline__ void grp_store(float2* o, int row, int q0, const floa
   }
 }
 
-template <int G>
+template <int G, int RS>
 __global__ void __launch_bounds__(kGrpWarps * 32, kGrpMinBlocks) grid_group_kernel(GridArgs a) {
-  constexpr int Q = 32 / G, TR = kWideRows, TC = kWideCols;
+  constexpr int TR = kWideRows, TC = kWideCols;
+  constexpr int LI = G * RS, Q = 32 / LI, R = TR / RS;  // lanes per item of a bundle, items, rows per lane
+  constexpr int S1 = LI;                                // steps of a bundle's batch
   extern __shared__ __align__(16) unsigned char smg[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float* tbl = reinterpret_cast<float*>(smg);  // the table, then a zero
@@ -241,9 +250,10 @@ __global__ void __launch_bounds__(kGrpWarps * 32, kGrpMinBlocks) grid_group_kern
   if (lane < kGrpRow / 16)
     *reinterpret_cast<uint4*>(wb + kGrpZeroRow * kGrpRow + lane * 16) = make_uint4(0u, 0u, 0u, 0u);
   __syncthreads();
-  const int p = lane & (G - 1), q = lane / G;    // this lane's pair and item (long item: cells)
+  const int p = lane & (G - 1), q = lane / LI;   // this lane's pair and item
+  const int row0 = lane / G % RS * R;            // and the first of its rows
   const int rq = lane % Q, rt = lane / Q;        // item and step whose record it expands
-  const int crow = q / (TC / G), ccol = q % (TC / G) * G;  // its cells of a long item
+  const int crow = lane / G / (TC / G), ccol = lane / G % (TC / G) * G;  // its cells of a long item
   // the list begins with the n_long long items
   const unsigned total = (unsigned)a.n_long + (unsigned)(a.n_items - a.n_long + Q - 1) / Q;
   const unsigned char* spec = reinterpret_cast<const unsigned char*>(a.spec) + p * 32;
@@ -270,19 +280,22 @@ __global__ void __launch_bounds__(kGrpWarps * 32, kGrpMinBlocks) grid_group_kern
   unsigned rec[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};  // this lane's record of the next batch
   float2* vals = reinterpret_cast<float2*>(wb + kGrpWtBytes);
   int vbuf = 0;  // which of the two value buffers holds the next batch
-  // A batch is G steps of the items of a bundle, or 32 samples of a long item.
+  // A batch is S1 steps of the items of a bundle, or 32 samples of a long item: 32 records.
   // rb, rn: first record and count of the item whose record this lane expands (the long
   // item, or item rq).
   auto load_rec = [&](int kind, int rb, int rn, int tb) {
     const int t = tb + (kind == 2 ? lane : rt);
     if (t < rn) ldg256(rec, a.rec + rb + t);
   };
-  // this lane's values: pair p of the samples whose records lanes q, Q + q, ... hold
+  // pair p of the samples whose records lanes lane / G, 32 / G + lane / G, ... hold: step i / Q
+  // of item i % Q for the record of lane i, or sample i of a long item
   auto load_values = [&](int kind, int cnt, int tb) {
+    const int n = RS == 1 ? cnt : __shfl_sync(0xffffffffu, cnt, lane / G % Q * LI);
 #pragma unroll
     for (int k = 0; k < G; ++k) {
-      const unsigned pl = __shfl_sync(0xffffffffu, rec[6], k * Q + q);
-      if (tb + (kind == 2 ? k * Q + q : k) < cnt)
+      const int i = k * (32 / G) + lane / G;
+      const unsigned pl = __shfl_sync(0xffffffffu, rec[6], i);
+      if (tb + (kind == 2 ? i : i / Q) < n)
         cp_async8(vals + (vbuf * G + k) * 32 + lane, spec + (size_t)(pl >> 2) * (G * 32) + (pl & 3u) * 8);
     }
     cp_async_commit();
@@ -292,7 +305,7 @@ __global__ void __launch_bounds__(kGrpWarps * 32, kGrpMinBlocks) grid_group_kern
   int kind = take(it);
   if (kind == 0) return;
   int cnt = it.run_end - it.run_begin;
-  int rb = __shfl_sync(0xffffffffu, it.run_begin, rq * G), rn = __shfl_sync(0xffffffffu, cnt, rq * G);
+  int rb = __shfl_sync(0xffffffffu, it.run_begin, rq * LI), rn = __shfl_sync(0xffffffffu, cnt, rq * LI);
   load_rec(kind, rb, rn, 0);
   load_values(kind, cnt, 0);
   for (;;) {
@@ -301,7 +314,7 @@ __global__ void __launch_bounds__(kGrpWarps * 32, kGrpMinBlocks) grid_group_kern
     const int ncnt = nit.run_end - nit.run_begin;
     // A sub-tile that no sample reaches has an empty item: its cells are written as zeros.
     const int nt = max(1, __reduce_max_sync(0xffffffffu, cnt));
-    const int S = kind == 2 ? 32 : G;
+    const int S = kind == 2 ? 32 : S1;
     // start of a batch: this batch's weights (lane i expands the record it holds), the
     // next batch's records; its values, later, when those are there
     auto begin = [&](int tb) {
@@ -316,8 +329,8 @@ __global__ void __launch_bounds__(kGrpWarps * 32, kGrpMinBlocks) grid_group_kern
       }
       const bool last = tb + S >= nt;
       if (last) {  // the next batch is the next bundle's first
-        rb = __shfl_sync(0xffffffffu, nit.run_begin, rq * G);
-        rn = __shfl_sync(0xffffffffu, ncnt, rq * G);
+        rb = __shfl_sync(0xffffffffu, nit.run_begin, rq * LI);
+        rn = __shfl_sync(0xffffffffu, ncnt, rq * LI);
       }
       load_rec(last ? nkind : kind, rb, rn, last ? 0 : tb + S);
       __syncwarp();
@@ -358,41 +371,41 @@ __global__ void __launch_bounds__(kGrpWarps * 32, kGrpMinBlocks) grid_group_kern
         grp_store<G>(Ht + (size_t)crow * a.M + ccol, tu * TR + crow, tv * TC + ccol, re, im);
       }
     } else {
-      GrpCell2 acc[TR][TC / 2];
+      GrpCell2 acc[R][TC / 2];
 #pragma unroll
-      for (int r = 0; r < TR; ++r)
+      for (int r = 0; r < R; ++r)
 #pragma unroll
         for (int c = 0; c < TC / 2; ++c) acc[r][c].re = acc[r][c].im = make_float2(0.f, 0.f);
-      for (int tb = 0; tb < nt; tb += G) {
+      for (int tb = 0; tb < nt; tb += S1) {
         begin(tb);
-        const float2* vv = vals + (vbuf ^ 1) * G * 32 + lane;
+        const float2* vv = vals + (vbuf ^ 1) * G * 32 + q * G + p;
         const unsigned char* d = wb + q * kGrpRow;
-        const int n = min(G, nt - tb), half = n >> 1;
+        const int n = min(S1, nt - tb), half = n >> 1;
         auto step = [&](int t) {
           const bool in = tb + t < cnt;
-          grp_apply(acc, in ? vv[t * 32] : make_float2(0.f, 0.f),
-                    in ? d + t * Q * kGrpRow : wb + kGrpZeroRow * kGrpRow);
+          grp_apply<R>(acc, in ? vv[t * Q * G] : make_float2(0.f, 0.f),
+                       in ? d + t * Q * kGrpRow : wb + kGrpZeroRow * kGrpRow, row0);
         };
         for (int t = 0; t < half; ++t) step(t);
         middle(tb);
         for (int t = half; t < n; ++t) step(t);
-        __syncwarp();  // the weights are read before they are replaced
+        __syncwarp();  // weights and values are read before they are replaced
       }
       if (slot >= 0) {
 #pragma unroll
-        for (int r = 0; r < TR; ++r)
+        for (int r = 0; r < R; ++r)
 #pragma unroll
           for (int c = 0; c < TC / 2; ++c) {
-            part[(r * TC + 2 * c) * G] = make_float2(acc[r][c].re.x, acc[r][c].im.x);
-            part[(r * TC + 2 * c + 1) * G] = make_float2(acc[r][c].re.y, acc[r][c].im.y);
+            part[((row0 + r) * TC + 2 * c) * G] = make_float2(acc[r][c].re.x, acc[r][c].im.x);
+            part[((row0 + r) * TC + 2 * c + 1) * G] = make_float2(acc[r][c].re.y, acc[r][c].im.y);
           }
       } else if (slot == -1 && p < a.pairs) {
 #pragma unroll
-        for (int r = 0; r < TR; ++r) {
+        for (int r = 0; r < R; ++r) {
           float2 re[TC / 2], im[TC / 2];
 #pragma unroll
           for (int c = 0; c < TC / 2; ++c) re[c] = acc[r][c].re, im[c] = acc[r][c].im;
-          grp_store<TC>(Ht + (size_t)r * a.M, tu * TR + r, tv * TC, re, im);
+          grp_store<TC>(Ht + (size_t)(row0 + r) * a.M, tu * TR + row0 + r, tv * TC, re, im);
         }
       }
     }
@@ -437,24 +450,25 @@ cudaError_t launch_tap_records(const GridArgs& a, int subs, int spw, int* counts
 
 // The kernels whose shared memory may exceed the default limit (init_kernel_attributes).
 void add_grid_kernels(std::vector<const void*>& f) {
-  f.push_back((const void*)grid_group_kernel<8>);
-  f.push_back((const void*)grid_group_kernel<4>);
-  f.push_back((const void*)grid_group_kernel<2>);
-  f.push_back((const void*)grid_group_kernel<1>);
+  f.push_back((const void*)grid_group_kernel<8, grp_row_split(8)>);
+  f.push_back((const void*)grid_group_kernel<4, grp_row_split(4)>);
+  f.push_back((const void*)grid_group_kernel<2, grp_row_split(2)>);
+  f.push_back((const void*)grid_group_kernel<1, grp_row_split(1)>);
 }
 
 template <int G>
 static cudaError_t launch_grid_group_g(const GridArgs& a, cudaStream_t s) {
+  constexpr int RS = grp_row_split(G), Q = 32 / (G * RS);
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int smem = grp_table_bytes(a.ltbl) + kGrpWarps * grp_warp_bytes<G>();
   int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, grid_group_kernel<G>, kGrpWarps * 32, smem);
-  const long bundles = a.n_long + (a.n_items - a.n_long + 32 / G - 1) / (32 / G);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, grid_group_kernel<G, RS>, kGrpWarps * 32, smem);
+  const long bundles = a.n_long + (a.n_items - a.n_long + Q - 1) / Q;
   const long want = (bundles + kGrpWarps - 1) / kGrpWarps;
   const int blocks = (int)std::min<long>(want, (long)std::max(per_sm, 1) * sms);
-  grid_group_kernel<G><<<blocks, kGrpWarps * 32, smem, s>>>(a);
+  grid_group_kernel<G, RS><<<blocks, kGrpWarps * 32, smem, s>>>(a);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess || a.n_split_tiles == 0) return e;
   split_reduce_group_kernel<<<a.n_split_tiles, 32 * G, 0, s>>>(a, G);
