@@ -2546,9 +2546,10 @@ static cudaError_t launch_cols_t(const ColArgs& a, cudaStream_t s) {
 }
 cudaError_t launch_cols(const ColArgs& args, cudaStream_t s) {
   ColArgs a = args;
-  // by default the persistent kernel wants two strips per SM (one pair at M = 2048: 194.9
-  // us a call with it, 194.4 without)
-  if (a.G <= 0 && a.ring && (long)(a.M / cols_group(a.M, 1)) * a.pairs < 2 * 148) a.ring = 0;
+  // by default the persistent kernel wants four strips per SM, for its last round to weigh
+  // little (M = 2048, us a pair: one pair 24.8 with and without, two 20.8 against 19.4, four
+  // 17.0 against 17.4)
+  if (a.G <= 0 && a.ring && (long)(a.M / cols_group(a.M, 1)) * a.pairs < 4 * 148) a.ring = 0;
   return a.rows < a.M ? launch_cols_t<true>(a, s) : launch_cols_t<false>(a, s);
 }
 
