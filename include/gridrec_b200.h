@@ -282,13 +282,13 @@ int gr_plan_tuning(const gr_plan* plan, int* item_cap, int* cols_group);
  * 16-pair, 3 32-pair, as gr_plan_grid_kernel reports; -1: by chunk size; only in the
  * default mode and among the kernels the plan holds records for), item_cap of that
  * kernel's work list (0: keep), cols_group (1, 2, 4, 8; 0: keep) and cols_ring (1:
- * the persistent double-buffered column FFT where its two landing buffers fit in
- * shared memory, 0: one strip per CTA, -1: keep).  GR_ERR_ARG for an option the plan
+ * the persistent column FFT, whose next strip lands during the transform, where its
+ * buffers fit in shared memory, 0: one strip per CTA, -1: keep).  GR_ERR_ARG for an option the plan
  * cannot run, or while a gr_graph holds the plan. */
 int gr_plan_set_tuning(gr_plan* plan, int grid_kernel, int item_cap, int cols_group,
                        int cols_ring);
 /* The full tuning: gridding kernel of a full chunk, its item cap, column group width
- * and whether the column FFT runs persistent and double-buffered. */
+ * and whether the column FFT runs persistent. */
 int gr_plan_tuning_ex(const gr_plan* plan, int* grid_kernel, int* item_cap, int* cols_group,
                       int* cols_ring);
 

@@ -319,7 +319,7 @@ class Plan:
         """Pins a tuning: grid_kernel ('tiles', 'wide', 'wide32' or None for the
         choice by chunk size) for full chunks, its work list's item cap (0: keep),
         the column-FFT group width (0: keep) and cols_ring (True: persistent
-        double-buffered column FFT, False: one strip per CTA, None: keep)."""
+        column FFT, False: one strip per CTA, None: keep)."""
         k = -1 if grid_kernel is None else self.GRID_KERNEL_CODES[grid_kernel]
         ring = -1 if cols_ring is None else int(bool(cols_ring))
         _check(lib().gr_plan_set_tuning(self._h, k, int(item_cap), int(cols_group), ring),
