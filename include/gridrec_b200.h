@@ -323,7 +323,9 @@ int gr_graph_destroy(gr_graph* graph);
 
 /* Ring suppression <- RingCorrectionSinogram   gridrec/GPU/tomo_recon.cpp:3905-3972
  * (the reference runs 20 rounds with RING_COEFF 1.0, tomo_recon.h:63).  In place on
- * n_slices sinograms; workspace: gr_ring_workspace_bytes() bytes of device memory. */
+ * n_slices sinograms; workspace: gr_ring_workspace_bytes() bytes of device memory, which
+ * never fall as a size grows (a buffer for the largest stack serves smaller ones).  A
+ * slice's bits do not depend on the other slices of the call. */
 size_t gr_ring_workspace_bytes(int n_slices, int n_det, int n_ang);
 int gr_ring_removal(float* sinos, int n_slices, int n_det, int n_ang, float ring_coeff,
                     int iterations, void* workspace, void* stream);

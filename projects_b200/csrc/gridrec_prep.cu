@@ -77,33 +77,26 @@ __global__ void ring_rowmean_kernel(const float* data, float* rowmean, int n_det
   if (threadIdx.x == 0) rowmean[(size_t)s * n_ang + i] = acc / n_det;
 }
 
-__device__ __forceinline__ float slice_gmean(const float* rm, int n_ang, float* red) {
+// g, the mean of a slice's row means.  Summed in FP64: an error of g scales the whole slice in
+// every round (20 rounds' error against float64 at 1024 x 720 x 16: 3.5e-7 with FP32 sums of g,
+// 2.2e-7).
+__device__ __forceinline__ float slice_gmean(const float* rm, int n_ang) {
   __shared__ float g_s;
-  float acc = 0.f;
+  __shared__ double red[32];
+  double acc = 0.0;
+#pragma unroll 8
   for (int i = threadIdx.x; i < n_ang; i += blockDim.x) acc += rm[i];
-  acc = block_sum(acc, red);
-  if (threadIdx.x == 0) g_s = acc / n_ang;
+  acc = block_sum_d(acc, red);
+  if (threadIdx.x == 0) g_s = (float)(acc / n_ang);
   __syncthreads();
   return g_s;
 }
 
-// Whether some chunk of slice s has a row of mean 0 that is not all zero (flags: one per
-// chunk of every slice).  Called by the whole block.
-__device__ __forceinline__ bool slice_flagged(const int* flags, int R) {
-  bool f = false;
-  for (int q = threadIdx.x; q < R; q += blockDim.x) f = f || flags[q] != 0;
-  return __syncthreads_or(f);
-}
-
-// flags given: only for slices with a flagged chunk (the others' partials are there).
 __global__ void ring_colpart_kernel(const float* data, const float* rowmean, float* part,
-                                    float* gmean, int n_det, int n_ang, int rows_per_chunk,
-                                    const int* flags) {
-  __shared__ float red[32];
+                                    float* gmean, int n_det, int n_ang, int rows_per_chunk) {
   const int r = blockIdx.y, s = blockIdx.z, R = gridDim.y;
-  if (flags && !slice_flagged(flags + (size_t)s * R, R)) return;
   const float* rm = rowmean + (size_t)s * n_ang;
-  const float g = slice_gmean(rm, n_ang, red);
+  const float g = slice_gmean(rm, n_ang);
   if (threadIdx.x == 0 && blockIdx.x == 0 && r == 0) gmean[s] = g;
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= n_det) return;
@@ -121,21 +114,17 @@ __global__ void ring_colpart_kernel(const float* data, const float* rowmean, flo
 // Column means c_j = g / n_ang * sum_q part[q][j] (32 columns x 16 chunk
 // strides per block).  scaled = 1: partials already include g (first round,
 // sums of v); scaled = 0: partials are sums of x / r_i and g, the mean of the
-// row means, is formed here and recorded for the next update.  flags given: scaled for
-// the slices that ring_colpart_kernel did.
+// row means, is formed here and recorded for the next update.
 constexpr int kColStrides = 16;
 
 __global__ void __launch_bounds__(32 * kColStrides) ring_colmean_kernel(const float* part, const float* rowmean,
                                                           float* colmean, float* gmean, int n_det,
-                                                          int n_ang, int R, int scaled,
-                                                          const int* flags) {
-  __shared__ float red[32];
+                                                          int n_ang, int R, int scaled) {
   __shared__ float acc_s[kColStrides][33];
   const int s = blockIdx.y;
   float g = 1.f;
-  if (flags) scaled = slice_flagged(flags + (size_t)s * R, R);
   if (!scaled) {
-    g = slice_gmean(rowmean + (size_t)s * n_ang, n_ang, red);
+    g = slice_gmean(rowmean + (size_t)s * n_ang, n_ang);
     if (threadIdx.x == 0 && blockIdx.x == 0) gmean[s] = g;
   }
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
@@ -269,32 +258,44 @@ __device__ __forceinline__ float div_by(float a, float b, float y) {
 constexpr int ring_threads(int n_det) { return n_det <= 2048 ? 128 : 256; }
 constexpr int ring_blocks(int threads) { return threads == 128 ? 5 : 2; }
 
+// Column sums of the vector kernels: a thread adds kRingGroup rows in FP32, then adds that sum
+// to an FP64 one that starts at kRingSum0, rounding down.  While a column's sum of x / r stays
+// below 2^21 in magnitude, every such addition keeps the multiples of 2^-30 below the sum
+// (kRingSum0 + sum lies in [2^22, 2^23), one binade), so the additions are exact in any order:
+// how a slice's rows are divided among blocks, which follows from the slices of the call, does
+// not show in its bits.  (Sums beyond that are FP64 sums of the usual kind.)
+constexpr int kRingGroup = 4;
+constexpr double kRingSum0 = 6291456.0;  // 1.5 * 2^22
+
 // The same round on rows of whole aligned 16-byte pieces: thread t of NT owns the pieces
 // t, t + NT, ... of a row (KV of them), so a row of 2048 costs four loads and four stores
 // per thread, the work per row (means, reciprocals, exchanges) is shared by 16 samples
 // of a thread, and rows whose mean and data are in div_by's range divide by one
 // reciprocal.  kFirst: the data may be negative (the first round), where the row mean
 // does not bound the samples and every division is the general one.  kStart: no update,
-// only the input's row means and column partials, with a flag per chunk for a row of mean
-// 0 that is not all zero (its samples enter the column means unscaled: the general
-// column pass redoes such slices).
-// Bound: DRAM once a call's slices exceed L2, then issue (50 % active).  16 slices of
-// 2048 x 1500: 62 us per round for 393 MB read and written against 101 us for the scalar
-// kernel (32 instructions per sample there, 17 here); 20 rounds 2.40 -> 1.48 ms with the
-// start pass (38 us for two passes of 97 and 109) and the backward rounds (65 -> 62 us per
-// round, part of the data still being in L2).  One slice 0.88 -> 0.36 ms.  256 threads of
-// half the pieces cost 74 us per round, groups of slices that fit L2 more than one wave
-// of all slices (80 MB groups 2.30 ms for the call).
+// only the input's row means and column partials, with a flag per block for a row of mean
+// 0 that is not all zero (its samples enter the column means unscaled:
+// ring_first_colmean_kernel does such slices).
+// Bound: DRAM once a call's slices exceed L2, then issue (17 instructions per sample, and
+// 50 per thread and row group for the FP64 sums).  16 slices of 2048 x 1500: 67.7 us per
+// round for 393 MB read and written, and 7.0 for the means; 20 rounds 2.42 -> 1.48 ms against
+// the scalar kernels, one slice 0.89 -> 0.35 ms.  (Column sums kept in FP32 over a block's rows
+// take 64.3 us per round, but their bits follow the number of slices of the call; FP32 sums over
+// fixed chunks of 8, 12 or 16 rows 1.74, 1.60 and 1.71 ms for the 20 rounds; writing a block's
+// only or last group without the shared copy 69.2 us.)  4 slices of 3000 x 1200, which fit L2:
+// 0.71 ms, 0.64 with FP32 sums.  256 threads of half the pieces cost 74 us per round, groups of
+// slices that fit L2 more than one wave of all slices (80 MB groups 2.30 ms for the call).
 enum RingMode { kStart, kFirst, kLater };
 template <int NT, int KV, int RB, RingMode kMode>
 __global__ void __launch_bounds__(NT, ring_blocks(NT)) ring_round_vec_kernel(
-    float* data, float* rowmean, const float* colmean, const float* gmean, float* part, int n_det,
-    int n_ang, int rows_per_chunk, float coeff, bool backward, int* flags) {
-  constexpr int NW = NT / 32;
+    float* data, float* rowmean, const float* colmean, const float* gmean, const float* cscale,
+    double* part, int n_det, int n_ang, int rows_per_block, float coeff, bool backward, int* flags) {
+  constexpr int NW = NT / 32, GB = kRingGroup / RB;  // batches of RB rows in a group
   __shared__ __align__(16) float red[2][RB][NW];
+  __shared__ double2 colsum[KV * 2][NT];  // a thread's own columns: pairs 2 k and 2 k + 1
   const int r = blockIdx.x, s = blockIdx.y, R = gridDim.x;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const float g = kMode == kStart ? 0.f : gmean[s];
+  const float g = kMode == kStart ? 0.f : gmean[s], cs = kMode == kStart ? 0.f : cscale[s];
   const float* c = colmean + (size_t)s * n_det;
   float d[KV][4], acc[KV][4];
   bool odd_row = false;
@@ -305,17 +306,19 @@ __global__ void __launch_bounds__(NT, ring_blocks(NT)) ring_round_vec_kernel(
       const int j = 4 * (threadIdx.x + k * NT) + e;
       float t = 0.f;
       if (kMode != kStart && j > 0 && j < n_det - 1) t = c[j] - (c[j - 1] + c[j] + c[j + 1]) / 3.f;
-      d[k][e] = __fmul_rn(t, coeff);
+      d[k][e] = __fmul_rn(__fmul_rn(t, cs), coeff);
       acc[k][e] = 0.f;
     }
+#pragma unroll
+  for (int k = 0; k < 2 * KV; ++k) colsum[k][threadIdx.x] = make_double2(kRingSum0, kRingSum0);
   float* rm = rowmean + (size_t)s * n_ang;
-  const int i0 = r * rows_per_chunk, i1 = min(n_ang, i0 + rows_per_chunk);
+  const int i0 = r * rows_per_block, i1 = min(n_ang, i0 + rows_per_block);
   const bool g_ok = !(kMode != kLater) && g >= 0x1p-40f && g <= 0x1p40f;
   // odd rounds walk the rows backwards: what the previous round wrote last is in L2
   const int nb = (i1 - i0 + RB - 1) / RB;
   int buf = 0;
   for (int t = 0; t < nb; ++t, buf ^= 1) {
-    const int ib = i0 + (backward ? nb - 1 - t : t) * RB;
+    const int bt = backward ? nb - 1 - t : t, ib = i0 + bt * RB;
     float4 y[RB][KV];
     float ri[RB], sum[RB];
     // all loads of the RB rows first, so they are in flight together
@@ -405,17 +408,104 @@ __global__ void __launch_bounds__(NT, ring_blocks(NT)) ring_round_vec_kernel(
         }
       }
     }
+    if (backward ? bt % GB == 0 : (bt % GB == GB - 1 || t == nb - 1)) {  // a group's last rows
+#pragma unroll
+      for (int k = 0; k < 2 * KV; ++k) {
+        float* g2 = &acc[k / 2][k % 2 * 2];
+        double2 c2 = colsum[k][threadIdx.x];
+        c2.x = __dadd_rd(c2.x, (double)g2[0]);
+        c2.y = __dadd_rd(c2.y, (double)g2[1]);
+        colsum[k][threadIdx.x] = c2;
+        g2[0] = g2[1] = 0.f;
+      }
+    }
   }
 #pragma unroll
-  for (int k = 0; k < KV; ++k) {
-    const int q = threadIdx.x + k * NT;
+  for (int k = 0; k < 2 * KV; ++k) {
+    const int q = threadIdx.x + k / 2 * NT;
+    const double2 c2 = colsum[k][threadIdx.x];
     if (4 * q < n_det)
-      reinterpret_cast<float4*>(part + ((size_t)s * R + r) * n_det)[q] =
-          make_float4(acc[k][0], acc[k][1], acc[k][2], acc[k][3]);
+      reinterpret_cast<double2*>(part + ((size_t)s * R + r) * n_det)[2 * q + k % 2] =
+          make_double2(c2.x - kRingSum0, c2.y - kRingSum0);
   }
   if (kMode == kStart) {
     const bool any = __syncthreads_or(odd_row);
     if (threadIdx.x == 0) flags[(size_t)s * R + r] = any;
+  }
+}
+
+// Whether some block of a slice met a row of mean 0 that is not all zero.  Called by the
+// whole block.
+__device__ __forceinline__ bool slice_flagged(const int* flags, int R) {
+  bool f = false;
+  for (int q = threadIdx.x; q < R; q += blockDim.x) f = f || flags[q] != 0;
+  return __syncthreads_or(f);
+}
+
+// Means of the vector kernels.  A block takes COLS columns in STR strides: colmean_j = sum_q
+// part[q][j] / n_ang (exact sums: any split gives the same bits), the factor g of the column
+// mean being left to the reader (cscale).  The last block of a slice forms g, the mean of its
+// row means, meanwhile.  flags given (after the start pass): no column means and a factor 1
+// for flagged slices.
+template <int COLS, int STR>
+__global__ void __launch_bounds__(COLS * STR) ring_colmean_vec_kernel(
+    const double* part, const float* rowmean, float* colmean, float* gmean, float* cscale, int n_det,
+    int n_ang, int R, const int* flags) {
+  __shared__ double acc_s[STR][COLS + 1];
+  const int s = blockIdx.y;
+  const bool flagged = flags && slice_flagged(flags + (size_t)s * R, R);
+  if (blockIdx.x == gridDim.x - 1) {
+    const float g = slice_gmean(rowmean + (size_t)s * n_ang, n_ang);
+    if (threadIdx.x == 0) gmean[s] = g, cscale[s] = flagged ? 1.f : g;
+    return;
+  }
+  if (flagged) return;
+  const int tx = threadIdx.x % COLS, ty = threadIdx.x / COLS;
+  const int j0 = blockIdx.x * COLS;
+  double acc = 0.0;
+  if (j0 + tx < n_det) {
+    const double* p = part + (size_t)s * R * n_det + j0 + tx;
+#pragma unroll 8
+    for (int q = ty; q < R; q += STR) acc += p[(size_t)q * n_det];
+  }
+  acc_s[ty][tx] = acc;
+  __syncthreads();
+  const int j = j0 + threadIdx.x / STR;  // STR lanes per column
+  double c = acc_s[threadIdx.x % STR][threadIdx.x / STR];
+#pragma unroll
+  for (int o = STR / 2; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+  if (threadIdx.x % STR == 0 && j < n_det) colmean[(size_t)s * n_det + j] = (float)(c / n_ang);
+}
+
+// First column means of flagged slices (those of the start pass leave out what a row of mean
+// 0 adds): ring_colpart_kernel's and ring_colmean_kernel's sums in one pass.
+__global__ void __launch_bounds__(32 * kColStrides) ring_first_colmean_kernel(
+    const float* data, const float* rowmean, float* colmean, int n_det, int n_ang, int R,
+    const int* flags) {
+  __shared__ float acc_s[kColStrides][33];
+  const int s = blockIdx.y;
+  if (!slice_flagged(flags + (size_t)s * R, R)) return;
+  const float* rm = rowmean + (size_t)s * n_ang;
+  const float g = slice_gmean(rm, n_ang);
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int j = blockIdx.x * 32 + tx;
+  float acc = 0.f;
+  if (j < n_det)
+    for (int q = ty; q * kRingRows < n_ang; q += kColStrides) {
+      float p = 0.f;
+      for (int i = q * kRingRows; i < min(n_ang, (q + 1) * kRingRows); ++i) {
+        const float x = data[((size_t)s * n_ang + i) * n_det + j];
+        const float ri = rm[i];
+        p += ri != 0.f ? __fdiv_rn(__fmul_rn(x, g), ri) : x;
+      }
+      acc += p;
+    }
+  acc_s[ty][tx] = acc;
+  __syncthreads();
+  if (ty == 0 && j < n_det) {
+    float c = 0.f;
+    for (int q = 0; q < kColStrides; ++q) c += acc_s[q][tx];
+    colmean[(size_t)s * n_det + j] = c / n_ang;
   }
 }
 
@@ -885,28 +975,36 @@ void launch_ring_round(dim3 grid, cudaStream_t st, float* x, float* rm, const fl
 // round -1: the start pass.
 template <int NT, int KV, int RB>
 void launch_ring_round_vec(int round, int rows, dim3 grid, cudaStream_t st, float* x, float* rm,
-                           const float* c, const float* g, float* part, int n_det, int n_ang,
-                           float coeff, int* flags) {
+                           const float* c, const float* g, const float* cs, double* part, int n_det,
+                           int n_ang, float coeff, int* flags) {
   if (round < 0)
-    ring_round_vec_kernel<NT, KV, RB, kStart><<<grid, NT, 0, st>>>(x, rm, c, g, part, n_det, n_ang,
+    ring_round_vec_kernel<NT, KV, RB, kStart><<<grid, NT, 0, st>>>(x, rm, c, g, cs, part, n_det, n_ang,
                                                                    rows, coeff, false, flags);
   else if (round == 0)
-    ring_round_vec_kernel<NT, KV, RB, kFirst><<<grid, NT, 0, st>>>(x, rm, c, g, part, n_det, n_ang,
+    ring_round_vec_kernel<NT, KV, RB, kFirst><<<grid, NT, 0, st>>>(x, rm, c, g, cs, part, n_det, n_ang,
                                                                    rows, coeff, true, flags);
   else
     ring_round_vec_kernel<NT, KV, RB, kLater><<<grid, NT, 0, st>>>(
-        x, rm, c, g, part, n_det, n_ang, rows, coeff, (round & 1) == 0, flags);
+        x, rm, c, g, cs, part, n_det, n_ang, rows, coeff, (round & 1) == 0, flags);
 }
 
 constexpr int kRingRB = 2;  // rows at once at 2048 and 4096 columns, twice that below
 
-// Rows per chunk on rows of whole 16-byte pieces: one wave of blocks over the GPU, in
-// equal chunks of whole row groups.
+// Rows per block on rows of whole 16-byte pieces: one wave of blocks over the GPU, in equal
+// parts of whole row groups.
+constexpr int ring_wave(int n_det) { return ring_blocks(ring_threads(n_det)) * 148; }
 int ring_rows_vec(int n_slices, int n_det, int n_ang) {
-  const long waves = ring_blocks(ring_threads(n_det)) * 148L;
-  const int rows = (int)(((long)n_ang * n_slices + waves - 1) / waves);
-  const int chunks = (n_ang + rows - 1) / rows;
-  return ((n_ang + chunks - 1) / chunks + 2 * kRingRB - 1) / (2 * kRingRB) * (2 * kRingRB);
+  const long wave = ring_wave(n_det);
+  const int rows = (int)(((long)n_ang * n_slices + wave - 1) / wave);
+  const int parts = (n_ang + rows - 1) / rows;
+  return ((n_ang + parts - 1) / parts + kRingGroup - 1) / kRingGroup * kRingGroup;
+}
+// The most partials that a call with up to n_slices slices of up to these sizes writes: at most
+// one per row group and slice, and a slice's parts are at most its share of the widest wave,
+// rounded up.
+size_t ring_parts_vec(int n_slices, int n_ang) {
+  const size_t groups = (size_t)n_slices * ((n_ang + kRingGroup - 1) / kRingGroup);
+  return std::min(groups, (size_t)std::max(ring_wave(1), ring_wave(4096)) + n_slices);
 }
 }  // namespace
 }  // namespace gr
@@ -917,10 +1015,11 @@ extern "C" {
 
 size_t gr_ring_workspace_bytes(int n_slices, int n_det, int n_ang) {
   if (n_slices < 1 || n_det < 1 || n_ang < 1) return 0;
-  const int rows = std::min(kRingRows, ring_rows_vec(n_slices, n_det, n_ang));
-  const size_t R = (n_ang + rows - 1) / rows;  // chunk partials of either kind of rows
-  const size_t floats = (size_t)n_slices * ((size_t)n_ang + R * (n_det + 1) + n_det + 1) + 4;
-  return floats * sizeof(float);
+  // column partials of either kind of rows, each with its flag; never less for smaller sizes
+  const size_t vec = ring_parts_vec(n_slices, n_ang) * ((size_t)n_det * sizeof(double) + sizeof(int));
+  const size_t scalar = (size_t)n_slices * ring_chunks(n_ang) * n_det * sizeof(float);
+  const size_t means = (size_t)n_slices * ((size_t)n_ang + n_det + 2) * sizeof(float);
+  return std::max(vec, scalar) + means + 16;
 }
 
 int gr_ring_removal(float* sinos, int n_slices, int n_det, int n_ang, float ring_coeff,
@@ -937,9 +1036,11 @@ int gr_ring_removal(float* sinos, int n_slices, int n_det, int n_ang, float ring
   const bool vec = bx <= 16 && n_det % 4 == 0 && (reinterpret_cast<uintptr_t>(sinos) & 15) == 0;
   const int rows = vec ? ring_rows_vec(n_slices, n_det, n_ang) : kRingRows;
   const int R = (n_ang + rows - 1) / rows;
-  // the chunk partials first, on a 16-byte boundary
-  float* part = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(workspace) + 15) & ~uintptr_t(15));
-  float* rowmean = part + (size_t)n_slices * R * n_det;
+  // the column partials first, on a 16-byte boundary
+  void* parts = reinterpret_cast<void*>((reinterpret_cast<uintptr_t>(workspace) + 15) & ~uintptr_t(15));
+  float* part = static_cast<float*>(parts);
+  double* part_vec = static_cast<double*>(parts);
+  float* rowmean = part + (size_t)n_slices * R * n_det * (vec ? 2 : 1);
   float* colmean = rowmean + (size_t)n_slices * n_ang;
   float* gmean = colmean + (size_t)n_slices * n_det;
   const int kpt = bx <= 1 ? 1 : bx <= 2 ? 2 : bx <= 4 ? 4 : bx <= 8 ? 8 : 16;
@@ -951,29 +1052,39 @@ int gr_ring_removal(float* sinos, int n_slices, int n_det, int n_ang, float ring
     float* pt = part;
     float* cm = colmean;
     float* gm = gmean;
-    int* flags = reinterpret_cast<int*>(gmean + n_slices);
+    float* cscale = gmean + n_slices;  // this and the flags: of the vector kernels
+    int* flags = reinterpret_cast<int*>(cscale + n_slices);
     auto vec_round = [&](int m) {
       const dim3 grid(R, ns);
       auto* fn = n_det <= 512    ? launch_ring_round_vec<128, 1, 2 * kRingRB>
                  : n_det <= 1024 ? launch_ring_round_vec<128, 2, 2 * kRingRB>
                  : n_det <= 2048 ? launch_ring_round_vec<128, 4, kRingRB>
                                  : launch_ring_round_vec<256, 4, kRingRB>;
-      fn(m, rows, grid, st, x, rm, cm, gm, pt, n_det, n_ang, ring_coeff, flags);
+      fn(m, rows, grid, st, x, rm, cm, gm, cscale, part_vec, n_det, n_ang, ring_coeff, flags);
+    };
+    auto vec_means = [&](const int* fl) {
+      // (one slice: few blocks and many partials, 24 loads in a row with 8 strides)
+      if (R > 200)
+        ring_colmean_vec_kernel<16, 32><<<dim3((n_det + 15) / 16 + 1, ns), 512, 0, st>>>(
+            part_vec, rm, cm, gm, cscale, n_det, n_ang, R, fl);
+      else
+        ring_colmean_vec_kernel<32, 8><<<dim3((n_det + 31) / 32 + 1, ns), 256, 0, st>>>(
+            part_vec, rm, cm, gm, cscale, n_det, n_ang, R, fl);
     };
     if (vec) {
       vec_round(-1);
+      vec_means(flags);
+      ring_first_colmean_kernel<<<dim3(cx, ns), cthreads, 0, st>>>(x, rm, cm, n_det, n_ang, R, flags);
     } else {
       ring_rowmean_kernel<<<dim3(n_ang, ns), kPrepThreads, 0, st>>>(x, rm, n_det, n_ang);
-      flags = nullptr;
+      ring_colpart_kernel<<<dim3(bx, R, ns), kPrepThreads, 0, st>>>(x, rm, pt, gm, n_det, n_ang, rows);
+      ring_colmean_kernel<<<dim3(cx, ns), cthreads, 0, st>>>(pt, rm, cm, gm, n_det, n_ang, R, 1);
     }
-    ring_colpart_kernel<<<dim3(bx, R, ns), kPrepThreads, 0, st>>>(x, rm, pt, gm, n_det, n_ang, rows,
-                                                                  flags);
-    ring_colmean_kernel<<<dim3(cx, ns), cthreads, 0, st>>>(pt, rm, cm, gm, n_det, n_ang, R, 1, flags);
     for (int m = 0; m < iterations; ++m) {
       if (vec) {
         vec_round(m);
         if (m + 1 < iterations)
-          ring_colmean_kernel<<<dim3(cx, ns), cthreads, 0, st>>>(pt, rm, cm, gm, n_det, n_ang, R, 0, nullptr);
+          vec_means(nullptr);
       } else if (fused) {
         const dim3 grid(R, ns);
         switch (kpt) {
@@ -984,14 +1095,13 @@ int gr_ring_removal(float* sinos, int n_slices, int n_det, int n_ang, float ring
           default: launch_ring_round<16, 2>(grid, st, x, rm, cm, gm, pt, n_det, n_ang, ring_coeff);
         }
         if (m + 1 < iterations)
-          ring_colmean_kernel<<<dim3(cx, ns), cthreads, 0, st>>>(pt, rm, cm, gm, n_det, n_ang, R, 0, nullptr);
+          ring_colmean_kernel<<<dim3(cx, ns), cthreads, 0, st>>>(pt, rm, cm, gm, n_det, n_ang, R, 0);
       } else {
         // Rows wider than 4096: separate update and column passes.
         if (m > 0) {
           ring_colpart_kernel<<<dim3(bx, R, ns), kPrepThreads, 0, st>>>(x, rm, pt, gm, n_det,
-                                                                        n_ang, kRingRows, nullptr);
-          ring_colmean_kernel<<<dim3(cx, ns), cthreads, 0, st>>>(pt, rm, cm, gm, n_det, n_ang, R, 1,
-                                                                 nullptr);
+                                                                        n_ang, kRingRows);
+          ring_colmean_kernel<<<dim3(cx, ns), cthreads, 0, st>>>(pt, rm, cm, gm, n_det, n_ang, R, 1);
         }
         ring_update_kernel<<<dim3(n_ang, ns), kPrepThreads, 0, st>>>(x, rm, cm, gm, n_det, n_ang,
                                                                      ring_coeff);

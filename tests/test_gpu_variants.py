@@ -179,3 +179,43 @@ def test_persistent_columns_same_bits(n, ring_group):
             outs.append(o.cpu().numpy()[:, :, :plan.M0])
     np.testing.assert_array_equal(outs[0], outs[1])
     np.testing.assert_array_equal(outs[2], outs[1])
+
+
+@pytest.mark.parametrize("n,a,S", [(8, 5, 9), (512, 37, 40), (1024, 97, 12), (2048, 61, 50), (4096, 35, 24),
+                                   (1021, 50, 3)])
+def test_ring_slice_bits_do_not_depend_on_the_stack(n, a, S):
+    """A slice alone, in a pair and in the whole stack (blocks of 4 rows up to many) gives the
+    same bits, with a row of mean 0 that is not all zero in one slice."""
+    rng = np.random.default_rng(n + S)
+    x = rng.uniform(0.0, 2.0, (S, a, n)).astype(np.float32)
+    x[rng.uniform(size=x.shape) < 0.04] = 0.0
+    x[1, 1, ::2], x[1, 1, 1::2] = 0.5, -0.5 if n % 2 == 0 else 0.0
+    whole = G.ring_removal(_dev(x), 1.0, 4).cpu().numpy()
+    for s in (0, 1, S - 2, S - 1):
+        np.testing.assert_array_equal(G.ring_removal(_dev(x[s:s + 1]), 1.0, 4).cpu().numpy()[0], whole[s])
+    np.testing.assert_array_equal(G.ring_removal(_dev(x[:2]), 1.0, 4).cpu().numpy(), whole[:2])
+
+
+@pytest.mark.parametrize("n", [12, 516, 1020, 2044, 4092])
+def test_ring_quotients_correctly_rounded(n):
+    """Rounds without column correction (coefficient 0) on rows of two samples, whose sum has
+    one rounding in any order: every value is RN(RN(x g) / r), bit for bit, whether the row
+    divides by its reciprocal or not (means beyond 2^40, products below 2^-60)."""
+    rng = np.random.default_rng(n)
+    S, a = 2, 700
+    x = np.zeros((S, a, n), np.float32)
+    for s in range(S):
+        for i in range(a):
+            j = rng.choice(n, 2, replace=False)
+            x[s, i, j] = (2.0 ** rng.uniform(-20, 20, 2)).astype(np.float32)
+            if i % 50 == 0:
+                x[s, i, j[0]] = np.float32(2.0 ** rng.uniform(-100, -55))
+            if s == 1 and i % 50 == 1:
+                x[s, i, j] = (2.0 ** rng.uniform(52, 60, 2)).astype(np.float32)
+    got = G.ring_removal(_dev(x), 0.0, 3).cpu().numpy()
+    for _ in range(3):
+        r = np.float32(x.sum(axis=2, dtype=np.float64)) / np.float32(n)
+        g = np.float32(r.astype(np.float64).mean(axis=1))
+        x = (x * g[:, None, None]) / r[:, :, None]
+    assert x.dtype == np.float32
+    np.testing.assert_array_equal(got, x)

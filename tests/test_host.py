@@ -408,3 +408,27 @@ def test_on_stream_leaves_the_current_stream_for_none_and_raw_handles():
     assert isinstance(G._on_stream(None), contextlib.nullcontext)
     assert isinstance(G._on_stream(0), contextlib.nullcontext)
     assert isinstance(G._on_stream(12345), contextlib.nullcontext)
+
+
+def _falls(size, steps):
+    """The (smaller, larger) neighbours along each axis at which size() falls."""
+    bad = []
+    for axis in range(len(steps)):
+        for at in range(len(steps[axis]) - 1):
+            for rest in np.ndindex(*[len(s) for k, s in enumerate(steps) if k != axis]):
+                rest = [s[i] for s, i in zip([s for k, s in enumerate(steps) if k != axis], rest)]
+                lo, hi = list(rest), list(rest)
+                lo.insert(axis, steps[axis][at])
+                hi.insert(axis, steps[axis][at + 1])
+                if size(*lo) > size(*hi):
+                    bad.append((tuple(lo), tuple(hi)))
+    return bad
+
+
+def test_ring_workspace_never_falls_as_a_dimension_grows():
+    """A buffer sized once for the largest stack serves every smaller one: the call takes no
+    size, so it would write past the end of a buffer that a smaller stack needs more of."""
+    f = G.lib().gr_ring_workspace_bytes
+    slices = list(range(1, 42)) + [63, 64, 65, 255, 256, 739, 740, 741, 1500, 4096]
+    bad = _falls(f, (slices, [9, 512, 1024, 1028, 2047, 2048, 2052, 4096, 4100], [1, 3, 4, 5, 37, 720, 1500, 1501, 6000]))
+    assert not bad, bad[:5]
