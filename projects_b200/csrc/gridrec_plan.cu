@@ -487,6 +487,12 @@ bool group_tiles_possible(const Plan* p) {
          (p->max_pairs > 1 || (long)p->M * p->M / (kWideRows * kWideCols) <= kGroupOneItems);
 }
 bool group_wide_possible(const Plan* p) { return p->wide_mode == 0 && p->max_pairs >= kWideMinPairs; }
+// The group that a chunk of `pairs` pairs grids as, and the largest one of this plan's chunks
+// (whether or not its records are there yet).
+int group_size(int pairs) { return pairs <= 2 ? pairs : (pairs <= 4 ? 4 : 8); }
+int group_size_max(const Plan* p) {
+  return group_tiles_possible(p) ? group_size(std::min(p->max_pairs, kGroupPairs)) : 1;
+}
 
 void drop_group_list(Plan* p, GroupList* g) {
   dev_free(p, &g->d_items);
@@ -572,7 +578,7 @@ int install_group_list(Plan* p, GroupList* out, const WorkList& wl, const Item* 
                                      wl.splits[t].nsplit, subs));
         }
     const size_t slots = (size_t)std::max(wl.n_slots * subs, 1);
-    const size_t cells = slots * kGroupPairs * (kWideRows * kWideCols / 2);
+    const size_t cells = slots * group_size_max(p) * (kWideRows * kWideCols / 2);
     e = cudaMemcpy(d_at, base.data(), n * sizeof(int), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = launch_tap_records(g, subs, spw, nullptr, d_at, out->d_rec, 0);
     if (e == cudaSuccess) e = cudaStreamSynchronize(0);
@@ -821,11 +827,10 @@ bool use_wide(const Plan* p, int pairs) {
 const GroupList* group_list(const Plan* p, int pairs) {
   if (pairs > kGroupPairs || p->wide_mode != 0 || use_w32(p, pairs)) return nullptr;
   const GroupList* g = use_wide(p, pairs) ? &p->g_wide : &p->g_tiles;
-  if (!g->ready || (pairs == 1 && (long)p->M * p->M / (kWideRows * kWideCols) > kGroupOneItems)) return nullptr;
+  if (!g->ready || group_size(pairs) > p->spec_pairs) return nullptr;
+  if (pairs == 1 && (long)p->M * p->M / (kWideRows * kWideCols) > kGroupOneItems) return nullptr;
   return g;
 }
-int group_size(int pairs) { return pairs <= 2 ? pairs : (pairs <= 4 ? 4 : 8); }
-
 GridArgs grid_args_tc(const Plan* p, int pairs) {
   GridArgs g{p->d_spec, p->d_H, p->d_t_scratch, p->d_queue, p->d_t_items, nullptr,
              p->d_t_split_list, p->t_split_tiles, p->d_dir, p->d_wtbl, p->t_items, pairs,
@@ -1500,9 +1505,11 @@ int gr::plan_create_ex(const gr_params* prm, const Pswf* pswf, float (*filter_fn
     return rc;
   }
   const size_t P = (size_t)p->max_pairs;
-  // the 16- and 32-pair kernels' spectra layouts hold whole groups of pairs
-  const size_t G_spec = p->x_ready ? kW32Pairs
-                        : ((p->w_items || p->t_items) ? kWidePairs : (p->g_tiles.ready ? kGroupPairs : 1));
+  // the spectra layouts of the 16- and 32-pair kernels and of gridding by groups hold whole
+  // groups of pairs (by what the plan may come to run: a list that is left out now may be
+  // there after a change of the tuning)
+  const size_t G_spec =
+      p->x_ready ? kW32Pairs : ((p->w_items || p->t_items) ? kWidePairs : group_size_max(p));
   const size_t P_spec = (P + G_spec - 1) / G_spec * G_spec;
   p->spec_pairs = (int)P_spec;
   if ((rc = dev_alloc(p, &p->d_spec, P_spec * p->n_ang * 2 * p->J)) ||

@@ -219,3 +219,21 @@ def test_ring_quotients_correctly_rounded(n):
         x = (x * g[:, None, None]) / r[:, :, None]
     assert x.dtype == np.float32
     np.testing.assert_array_equal(got, x)
+
+
+def test_plan_holds_spectra_for_its_own_groups():
+    """A plan's spectra hold the group that its largest chunk grids as (1, 2, 4, 4, 8, 8 pairs
+    for plans of 1 to 6), no more and no less: its bytes against those of a plan of the same
+    pairs without groups, whose spectra hold exactly its pairs."""
+    n, a = 256, 30
+    th = ph.angles_deg(a)
+    pair = a * 2 * 128 * 8  # one pair's spectra: two half lines of 128 complex values per angle
+    records = set()
+    for pairs, group in ((1, 1), (2, 2), (3, 4), (4, 4), (5, 8), (6, 8)):
+        size = {}
+        for mode in (0, -1):
+            with G.Plan(n, a, th, max_pairs=pairs, wide_grid=mode) as plan:
+                size[mode] = plan.device_bytes()
+        # (the list's scratch: 32 complex cells of a group)
+        records.add(size[0] - size[-1] - (group - pairs) * pair - group * 32 * 8)
+    assert len(records) == 1, records
