@@ -598,10 +598,26 @@ int install_group_list(Plan* p, GroupList* out, const WorkList& wl, const Item* 
   return GR_OK;
 }
 
+// The records for gridding by groups in the order of the tile list `wl`.
+int install_group_tiles(Plan* p, const WorkList& wl) {
+  if (!group_tiles_possible(p)) return GR_OK;
+  const int nt = p->ntaps <= 3 ? 3 : (p->ntaps <= 4 ? 4 : kMaxTaps);  // grid_kernel's lanes per sample
+  return install_group_list(p, &p->g_tiles, wl, p->d_items, p->d_runs, (kTile / kWideRows) * (kTile / kWideCols),
+                            32 / nt);
+}
+// And in the order of the 16-pair kernel's list.
+int install_group_wide(Plan* p, const WorkList& wl) {
+  if (!group_wide_possible(p)) return GR_OK;
+  return install_group_list(p, &p->g_wide, wl, p->d_w_items, p->d_w_runs, 1, 32);
+}
+
 // Builds the work list with the given item cap and (re)places it on the
-// device; grows the split-tile scratch when needed.
-int install_work_list(Plan* p, int item_cap) {
-  WorkList wl;
+// device; grows the split-tile scratch when needed.  The optional group records, which may
+// take what memory is left, come last: here, or with `later` by the caller, who gets the list.
+int install_work_list(Plan* p, int item_cap, WorkList* later = nullptr) {
+  WorkList local;
+  WorkList& wl = later ? *later : local;
+  drop_group_list(p, &p->g_tiles);
   build_work_list(p->M, p->J, p->L, p->n_ang, p->dxy, &wl, item_cap);
   std::vector<int4> split_list;
   for (size_t t = 0; t < wl.splits.size(); ++t)
@@ -631,10 +647,7 @@ int install_work_list(Plan* p, int item_cap) {
   p->total_samples = wl.total;
   p->n_split_tiles = (int)split_list.size();
   p->item_cap = item_cap;
-  if (!group_tiles_possible(p)) return GR_OK;
-  const int nt = p->ntaps <= 3 ? 3 : (p->ntaps <= 4 ? 4 : kMaxTaps);  // grid_kernel's lanes per sample
-  return install_group_list(p, &p->g_tiles, wl, p->d_items, p->d_runs, (kTile / kWideRows) * (kTile / kWideCols),
-                            32 / nt);
+  return later ? GR_OK : install_group_tiles(p, wl);
 }
 
 // Whether chunks of this plan can use the 16-pair kernel (its weights) or the
@@ -647,9 +660,12 @@ bool w32_possible(const Plan* p) {
 }
 
 // The 16- and 32-pair kernels' work list (4 x 8 sub-tiles), placed on the device
-// with the records of whichever of the two kernels the plan can use.
-int install_work_list_wide(Plan* p, int item_cap) {
-  WorkList wl;
+// with the records of whichever of the two kernels the plan can use; `later` as for
+// install_work_list.  (In a plan without larger chunks the group records take the place of
+// the weights, which are larger: they come first, and the weights only without them.)
+int install_work_list_wide(Plan* p, int item_cap, WorkList* later = nullptr) {
+  WorkList local;
+  WorkList& wl = later ? *later : local;
   build_work_list(p->M, p->J, p->L, p->n_ang, p->dxy, &wl, item_cap, kListWide);
   std::vector<int4> split_list;
   for (size_t t = 0; t < wl.splits.size(); ++t)
@@ -668,10 +684,8 @@ int install_work_list_wide(Plan* p, int item_cap) {
   if (n_rec > (size_t)INT_MAX) return fail(GR_ERR_UNSUPPORTED, "work list too large");
   // the 32-pair kernel's records: per run an index block of n * 12 16-bit indices,
   // padded to whole 16-byte units (its bulk copies move whole units)
-  // (a plan whose chunks of 7 and 8 pairs grid by groups and has no larger ones needs no
-  // weights)
-  const bool need32 = w32_possible(p);
-  if (group_wide_possible(p)) drop_group_list(p, &p->g_wide);
+  const bool need32 = w32_possible(p), groups_only = p->max_pairs <= kGroupPairs;
+  drop_group_list(p, &p->g_wide);
   std::vector<int2> rinfo;
   size_t n_units = 0;
   if (need32) {
@@ -694,10 +708,8 @@ int install_work_list_wide(Plan* p, int item_cap) {
   if ((rc = upload(p, &p->d_w_items, wl.items)) || (rc = upload(p, &p->d_w_runs, wl.runs)) ||
       (rc = upload(p, &p->d_w_split_list, split_list)))
     return rc;
-  if (group_wide_possible(p) &&
-      (rc = install_group_list(p, &p->g_wide, wl, p->d_w_items, p->d_w_runs, 1, 32)))
-    return rc;
-  const bool need16 = wide16_possible(p) && !(p->g_wide.ready && p->max_pairs <= kGroupPairs);
+  if (groups_only && (rc = install_group_wide(p, wl))) return rc;
+  const bool need16 = wide16_possible(p) && !(groups_only && p->g_wide.ready);
   if ((need16 && ((rc = upload(p, &p->d_w_meta, meta)) ||
                   (rc = dev_alloc(p, &p->d_w_wts, std::max<size_t>(n_rec, 1) * kWideRec)))))
     return rc;
@@ -751,7 +763,7 @@ int install_work_list_wide(Plan* p, int item_cap) {
   p->w_slots = wl.n_slots;
   p->w_split_tiles = (int)split_list.size();
   p->w_item_cap = item_cap;
-  return GR_OK;
+  return later || groups_only ? GR_OK : install_group_wide(p, wl);
 }
 
 // The tensor-core kernel's work list: 16 x 8 sub-tiles; each item's runs
@@ -1495,12 +1507,13 @@ int gr::plan_create_ex(const gr_params* prm, const Pswf* pswf, float (*filter_fn
       return rc;
     }
   }
+  WorkList wl, wl_wide;
   if ((rc = upload(p, &p->d_wtbl, fw)) || (rc = upload(p, &p->d_winv, fi)) ||
       (rc = upload(p, &p->d_filt, filt)) || (rc = upload(p, &p->d_tw_p, twiddles((int)pdim))) ||
       (rc = upload(p, &p->d_tw_m, twiddles((int)M))) || (rc = upload(p, &p->d_dir, dirs)) ||
-      (rc = install_work_list(p, kItemCap)) ||
+      (rc = install_work_list(p, kItemCap, &wl)) ||
       (p->wide_mode == 2 && (rc = install_work_list_tc(p, kItemCapT))) ||
-      ((wide16_possible(p) || w32_possible(p)) && (rc = install_work_list_wide(p, kItemCapW)))) {
+      ((wide16_possible(p) || w32_possible(p)) && (rc = install_work_list_wide(p, kItemCapW, &wl_wide)))) {
     gr_plan_destroy(p);
     return rc;
   }
@@ -1516,7 +1529,10 @@ int gr::plan_create_ex(const gr_params* prm, const Pswf* pswf, float (*filter_fn
       (rc = dev_alloc(p, &p->d_H, P * (size_t)M * M)) ||
       (rc = dev_alloc(p, &p->d_pq, P * p->J)) ||
       (rc = dev_alloc(p, &p->d_dl, 2 * P * (size_t)p->n_det)) ||
-      (rc = dev_alloc(p, &p->d_queue, 1)) || (rc = dev_alloc(p, &p->d_err, 1))) {
+      (rc = dev_alloc(p, &p->d_queue, 1)) || (rc = dev_alloc(p, &p->d_err, 1)) ||
+      // then the records that are left out where they do not fit
+      (p->max_pairs > kGroupPairs && (rc = install_group_wide(p, wl_wide))) ||
+      (rc = install_group_tiles(p, wl))) {
     gr_plan_destroy(p);
     return rc;
   }

@@ -237,3 +237,49 @@ def test_plan_holds_spectra_for_its_own_groups():
         # (the list's scratch: 32 complex cells of a group)
         records.add(size[0] - size[-1] - (group - pairs) * pair - group * 32 * 8)
     assert len(records) == 1, records
+
+
+@pytest.mark.parametrize("pairs,chunk", [(3, 3), (6, 6), (12, 8)])
+def test_plan_where_the_group_records_do_not_fit(pairs, chunk):
+    """On a GPU with room for a plan's buffers but not for its optional group records, the plan
+    is made without them and gives the same bits; records that come with a later change of the
+    tuning, when there is room, grid the same chunks by groups within the plan's buffers."""
+    n, a = 512, 2000
+    th = ph.angles_deg(a)
+    S = 2 * chunk - 1
+    rng = np.random.default_rng(pairs)
+    sinos = _dev(rng.uniform(0.0, 2.0, (S, a, n)).astype(np.float32))
+
+    def images(plan):
+        o = torch.full((S, plan.M0, n), float("nan"), device="cuda")
+        plan.reconstruct_batch(sinos, o)
+        torch.cuda.synchronize()
+        plan.device_status()
+        return o.cpu().numpy()[:, :, :plan.M0]
+
+    def make():
+        return G.Plan(n, a, th, filter=G.FILTER_HANN, max_pairs=pairs)
+
+    with make() as plan:
+        want, whole = images(plan), plan.device_bytes()
+        cap = plan.set_tuning("tiles" if pairs < 7 else "wide", 600)["item_cap"]
+        tuned = images(plan)
+    with G.Plan(n, a, th, filter=G.FILTER_HANN, max_pairs=pairs, wide_grid=-1) as plan:
+        bare = plan.device_bytes()
+    torch.cuda.empty_cache()
+    list_bytes = 30 << 20  # well under one list of records (32 bytes each, more than 2 a sample)
+    assert whole - bare > list_bytes and 2 * n * a * 32 > list_bytes
+    # room for everything but the last list of records, less half of that
+    room = whole - list_bytes // 2
+    filler = torch.empty(torch.cuda.mem_get_info()[0] - room, dtype=torch.uint8, device="cuda")
+    try:
+        plan = make()
+        short = plan.device_bytes()
+    finally:
+        del filler
+        torch.cuda.empty_cache()
+    with plan:
+        assert short < whole - list_bytes, (short, whole)
+        np.testing.assert_array_equal(images(plan), want)
+        assert plan.set_tuning("tiles" if pairs < 7 else "wide", 600)["item_cap"] == cap
+        np.testing.assert_array_equal(images(plan), tuned)
