@@ -77,6 +77,7 @@ constexpr int grp_row_split(int G) { return G == 2 ? 4 : 1; }
 // lookups than the tile kernel's pass over them).  For 9 to 16 pairs two groups cost what the
 // 16-pair kernel does, for more the 32-pair kernel is faster (31 a pair).
 constexpr int kGroupPairs = 8;
+constexpr int kGridYMax = 65535;  // blocks along a grid's y
 constexpr int kGroupOneItems = 1 << 15;
 
 // The tensor-core gridding kernel (grid_tc_kernel): a CTA accumulates a

@@ -482,16 +482,18 @@ void build_work_list(int M, int J, double L, int n_ang, const std::vector<double
 
 // Whether chunks of this plan can grid by groups of pairs in the order of the tile kernel
 // (1 .. 6 pairs) or of the 16-pair kernel (7 and 8 pairs).
+// (One pair only of more than kGridYMax angles: the interleaved spectra of several take the
+// angle as their grid's y.)
 bool group_tiles_possible(const Plan* p) {
-  return p->wide_mode == 0 &&
-         (p->max_pairs > 1 || (long)p->M * p->M / (kWideRows * kWideCols) <= kGroupOneItems);
+  if (p->wide_mode != 0) return false;
+  return p->max_pairs > 1 ? p->n_ang <= kGridYMax : (long)p->M * p->M / (kWideRows * kWideCols) <= kGroupOneItems;
 }
 bool group_wide_possible(const Plan* p) { return p->wide_mode == 0 && p->max_pairs >= kWideMinPairs; }
 // The group that a chunk of `pairs` pairs grids as, and the largest one of this plan's chunks
 // (whether or not its records are there yet).
 int group_size(int pairs) { return pairs <= 2 ? pairs : (pairs <= 4 ? 4 : 8); }
 int group_size_max(const Plan* p) {
-  return group_tiles_possible(p) ? group_size(std::min(p->max_pairs, kGroupPairs)) : 1;
+  return p->wide_mode == 0 ? group_size(std::min(p->max_pairs, kGroupPairs)) : 1;
 }
 
 void drop_group_list(Plan* p, GroupList* g) {

@@ -283,3 +283,21 @@ def test_plan_where_the_group_records_do_not_fit(pairs, chunk):
         np.testing.assert_array_equal(images(plan), want)
         assert plan.set_tuning("tiles" if pairs < 7 else "wide", 600)["item_cap"] == cap
         np.testing.assert_array_equal(images(plan), tuned)
+
+
+@pytest.mark.parametrize("S", [2, 3, 8])
+def test_more_angles_than_a_grid_has_rows(S):
+    """Chunks of 1 to 4 pairs of 65,600 angles: the tile kernel, whose spectra take the angle as
+    the grid's x, as with wide_grid = -1."""
+    n, a = 16, 65600
+    th = ph.angles_deg(a)
+    sinos = _dev(np.random.default_rng(S).uniform(0.0, 2.0, (S, a, n)).astype(np.float32))
+    outs = []
+    for mode in (0, -1):
+        with G.Plan(n, a, th, filter=G.FILTER_HANN, max_pairs=4, wide_grid=mode) as plan:
+            o = torch.full((S, plan.M0, n), float("nan"), device="cuda")
+            plan.reconstruct_batch(sinos, o)
+            torch.cuda.synchronize()
+            plan.device_status()
+            outs.append(o.cpu().numpy()[:, :, :plan.M0])
+    np.testing.assert_array_equal(outs[0], outs[1])
