@@ -381,7 +381,7 @@ int gr_entropy(const float* images, int n_groups, int group, int rows, int cols,
  * every slice shifted by xoffset and half padded to the plan's width (the plan is
  * made for 2 n_det detector pixels and n_ang angles), reconstructed in pairs, and
  * cropped to n_det x n_det (rows of out_stride floats, slices n_det * out_stride
- * apart).  Allocates its intermediates (stream-ordered). */
+ * apart).  Uses the plan's own buffers only. */
 int gr_reconstruct_padded(gr_plan* plan, const float* sinos, int n_slices, int n_det, int n_ang,
                           float xoffset, float* outs, long out_stride, void* stream);
 
@@ -391,7 +391,8 @@ int gr_reconstruct_padded(gr_plan* plan, const float* sinos, int n_slices, int n
  * both n_det x n_det crops are scored together with the histogram entropy
  * [hist_lo, hist_hi] in nbins bins, and scores[c] (host) receives the score.
  * *best = first index of the minimum score.  best_images (optional, device,
- * 2 x n_det x n_det) receives the pair at the best shift.  Synchronises `stream`. */
+ * 2 x n_det x n_det) receives the pair at the best shift, in stream order.  Synchronises
+ * `stream` once the scores are there; sino1 and sino2 are not read after the call. */
 int gr_center_search(gr_plan* plan, const float* sino1, const float* sino2, int n_det, int n_ang,
                      const float* shifts, int n_cand, float hist_lo, float hist_hi, int nbins,
                      float* scores, int* best, float* best_images, void* stream);

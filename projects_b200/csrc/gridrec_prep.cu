@@ -1228,6 +1228,9 @@ int gr_center_search(gr_plan* plan, const float* sino1, const float* sino2, int 
   cudaStream_t st = (cudaStream_t)stream;
   const int chunk = std::min(n_cand, max_pairs);  // candidates per batch (one pair each)
   const long slice_rec = (long)n_det * n_det;
+  // The best images may still be on their way when the call returns: they are made from a copy,
+  // so that the caller's rows are not read after that.
+  const size_t kept = best_images ? (size_t)n_ang * n_det : 0;
   const ImageWindow win{off, n_det, off, n_det};  // the crop: only it is transformed and written
   Carve c;
   for (int pass = 0; pass < 2; ++pass) {
@@ -1235,17 +1238,25 @@ int gr_center_search(gr_plan* plan, const float* sino1, const float* sino2, int 
       if ((rc = plan_scratch(plan, c.off + 256, (void**)&c.base))) return rc;
       c.off = 0;
     }
+    c.take<float>(kept);
+    c.take<float>(kept);
     c.take<float>((size_t)2 * chunk * slice_rec);
     c.take<float>(n_cand);
     c.take<unsigned>((size_t)chunk * (nbins + 1));
     c.take<float>(n_cand);
   }
   c.off = 0;
+  float* kept1 = c.take<float>(kept);
+  float* kept2 = c.take<float>(kept);
   float* rec = c.take<float>((size_t)2 * chunk * slice_rec);
   float* xo = c.take<float>(n_cand);
   unsigned* gh = c.take<unsigned>((size_t)chunk * (nbins + 1));
   float* sc = c.take<float>(n_cand);
   cudaError_t e = cudaMemcpyAsync(xo, shifts, n_cand * sizeof(float), cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess && kept)
+    e = cudaMemcpyAsync(kept1, sino1, kept * sizeof(float), cudaMemcpyDeviceToDevice, st);
+  if (e == cudaSuccess && kept)
+    e = cudaMemcpyAsync(kept2, sino2, kept * sizeof(float), cudaMemcpyDeviceToDevice, st);
   if (e != cudaSuccess) return cuda_fail(e, "centre search: copies");
   for (int c0 = 0; c0 < n_cand; c0 += chunk) {
     const int nc = std::min(chunk, n_cand - c0);
@@ -1264,7 +1275,7 @@ int gr_center_search(gr_plan* plan, const float* sino1, const float* sino2, int 
     if (scores[k] < scores[bi]) bi = k;
   if (best) *best = bi;
   if (best_images) {
-    const PaddedInput in{sino1, sino2, 0, n_det, xo + bi, 0.f};
+    const PaddedInput in{kept1, kept2, 0, n_det, xo + bi, 0.f};
     if ((rc = plan_reconstruct_padded(plan, in, 2, best_images, n_det, win, st))) return rc;
   }
   return GR_OK;

@@ -301,3 +301,28 @@ def test_more_angles_than_a_grid_has_rows(S):
             plan.device_status()
             outs.append(o.cpu().numpy()[:, :, :plan.M0])
     np.testing.assert_array_equal(outs[0], outs[1])
+
+
+def test_center_search_leaves_the_sinograms_to_the_caller():
+    """The images of the best shift are those of the sinograms as they were passed, also where
+    the caller overwrites them on another stream as soon as the call has returned."""
+    n, a = 1000, 2400
+    rng = np.random.default_rng(4)
+    x = rng.uniform(0.0, 2.0, (2, a, n)).astype(np.float32)
+    shifts = np.float32([-0.5, 0.5])
+    side = torch.cuda.Stream()
+    with G.Plan(2 * n, a, ph.angles_deg(a), filter=G.FILTER_HANN) as plan:
+        s = _dev(x)
+        scores, best, want = G.center_search(plan, s[0], s[1], shifts, -1.0, 3.0, 500, want_images=True)
+        torch.cuda.synchronize()
+        other = torch.full_like(s, 7.0)
+        for _ in range(3):
+            s.copy_(torch.from_numpy(x))
+            torch.cuda.synchronize()
+            with torch.cuda.stream(side):
+                again = G.center_search(plan, s[0], s[1], shifts, -1.0, 3.0, 500, want_images=True, stream=side)
+            s.copy_(other)  # on the current stream, not ordered after `side`
+            torch.cuda.synchronize()
+            assert again[1] == best
+            np.testing.assert_array_equal(again[0], scores)
+            assert torch.equal(again[2], want)
