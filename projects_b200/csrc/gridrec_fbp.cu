@@ -128,11 +128,6 @@ __global__ void __launch_bounds__(kBpThreads) fbp_backproject_kernel(const float
 template <int S, int R>
 cudaError_t launch_backproject_r(const float* filt, const float2* cs, float* recon, int n, int n_ang,
                                  bool finite, int groups, int smem, cudaStream_t st) {
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(fbp_backproject_kernel<S, R>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-  }
   const dim3 grid((n + kBpTile - 1) / kBpTile, (n + 8 * R - 1) / (8 * R), groups);
   fbp_backproject_kernel<S, R><<<grid, kBpThreads, smem, st>>>(filt, cs, recon, n, n_ang, finite);
   return cudaGetLastError();
@@ -148,6 +143,22 @@ cudaError_t launch_backproject(const float* filt, const float2* cs, float* recon
   return t * t * groups >= 4 * 148
              ? launch_backproject_r<S, 4>(filt, cs, recon, n, n_ang, finite, groups, smem, st)
              : launch_backproject_r<S, 1>(filt, cs, recon, n, n_ang, finite, groups, smem, st);
+}
+
+// Lets every form of the backprojection use `smem` bytes of shared memory.
+cudaError_t allow_backproject_smem(int smem) {
+  if (smem <= 48 * 1024) return cudaSuccess;
+  const void* forms[] = {(const void*)fbp_backproject_kernel<4, 4>, (const void*)fbp_backproject_kernel<4, 1>,
+                         (const void*)fbp_backproject_kernel<2, 4>, (const void*)fbp_backproject_kernel<2, 1>,
+                         (const void*)fbp_backproject_kernel<1, 4>, (const void*)fbp_backproject_kernel<1, 1>};
+  for (const void* f : forms) {
+    const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) {
+      cudaGetLastError();  // not left behind for the next call's launch check
+      return e;
+    }
+  }
+  return cudaSuccess;
 }
 
 // Slices backprojected together: 4, then 2, then 1 of what is left of a call's chunk.
@@ -247,20 +258,22 @@ int gr_fbp_reconstruct(gr_fbp* f, const float* sinos, int n_slices, float* recon
   const int n = f->n;
   const size_t slice_in = (size_t)f->n_ang * n, slice_out = (size_t)n * n;
   const int smem_bp = f->n_ang * (int)sizeof(float2);
+  // too many angles for their table: refused before anything runs
+  cudaError_t e = allow_backproject_smem(smem_bp);
+  if (e != cudaSuccess)
+    return fail(GR_ERR_UNSUPPORTED, "fbp: %d angles: %s", f->n_ang, cudaGetErrorString(e));
   for (int s0 = 0; s0 < n_slices;) {
     // whole groups of one size, as many as the filtered-row buffer holds
     const int S = bp_group(std::min(f->max_slices, n_slices - s0));
     const int groups = std::min(f->max_slices, n_slices - s0) / S;
     FbpFilterArgs fa{sinos + s0 * slice_in, f->d_filt, f->d_lut, f->d_tw, n, f->n_ang, groups * S, S};
-    cudaError_t e = launch_fbp_filter(fa, st);
+    e = launch_fbp_filter(fa, st);
     if (e != cudaSuccess) return fail(GR_ERR_CUDA, "fbp filter: %s", cudaGetErrorString(e));
     float* out = recons + s0 * slice_out;
     e = S == 4 ? launch_backproject<4>(f->d_filt, f->d_cs, out, n, f->n_ang, f->finite, groups, smem_bp, st)
         : S == 2 ? launch_backproject<2>(f->d_filt, f->d_cs, out, n, f->n_ang, f->finite, groups, smem_bp, st)
                  : launch_backproject<1>(f->d_filt, f->d_cs, out, n, f->n_ang, f->finite, groups, smem_bp, st);
-    if (e != cudaSuccess)
-      return fail(smem_bp > 48 * 1024 ? GR_ERR_UNSUPPORTED : GR_ERR_CUDA, "fbp: %d angles: %s",
-                  f->n_ang, cudaGetErrorString(e));
+    if (e != cudaSuccess) return fail(GR_ERR_CUDA, "fbp backprojection: %s", cudaGetErrorString(e));
     s0 += groups * S;
   }
   return GR_OK;

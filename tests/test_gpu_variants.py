@@ -326,3 +326,19 @@ def test_center_search_leaves_the_sinograms_to_the_caller():
             assert again[1] == best
             np.testing.assert_array_equal(again[0], scores)
             assert torch.equal(again[2], want)
+
+
+def test_fbp_too_many_angles_refused_and_nothing_left_behind():
+    """More angles than the shared-memory table holds: refused as unsupported before anything
+    runs, and the next call is not told of it; more than the default table limit: run."""
+    n = 16
+    x = _dev(np.random.default_rng(0).uniform(0.0, 2.0, (1, 30000, n)).astype(np.float32))
+    many = G.FBP(n, 30000, ph.angles_deg(30000), max_slices=1)
+    some = G.FBP(n, 7000, ph.angles_deg(7000), max_slices=1)
+    for _ in range(2):
+        with pytest.raises(G.GrError, match="UNSUPPORTED"):
+            many.reconstruct(x)
+        got = some.reconstruct(x[:, :7000].contiguous()).cpu().numpy()[0]
+        assert ph.rel_l2(got, O.port_optimized_fbp(x[0, :7000].cpu().numpy(), ph.angles_deg(7000))) < 1e-5
+    many.close()
+    some.close()
