@@ -250,7 +250,10 @@ int gr_worklist_export(const gr_params* p, int* n_items, int* n_runs, int* tiles
 int gr_worklist_export_wide(const gr_params* p, int* n_items, int* n_runs, int* tiles_v,
                             int* items, int* runs, int* splits, int cap_items, int cap_runs);
 /* *wide = 0 (tile kernel), 1 (16-pair kernel), 2 (tensor-core kernel) or 3 (32-pair
- * kernel) for a chunk of `pairs` pairs. */
+ * kernel) for a chunk of `pairs` pairs.  It names the order of summation, and so the bits: by
+ * default a chunk of 2 to 8 pairs, or of one pair up to M = 1024, grids by groups of pairs, on
+ * the same work list and with the same bits as the kernel named, which grids it where the
+ * group's records do not fit the GPU's memory. */
 int gr_plan_grid_kernel(const gr_plan* plan, int pairs, int* wide);
 
 /* Text of the last error recorded on this thread (never NULL). */
@@ -282,13 +285,15 @@ int gr_plan_tuning(const gr_plan* plan, int* item_cap, int* cols_group);
  * 16-pair, 3 32-pair, as gr_plan_grid_kernel reports; -1: by chunk size; only in the
  * default mode and among the kernels the plan holds records for), item_cap of that
  * kernel's work list (0: keep), cols_group (1, 2, 4, 8; 0: keep) and cols_ring (1:
- * the persistent column FFT, whose next strip lands during the transform, where its
- * buffers fit in shared memory, 0: one strip per CTA, -1: keep).  GR_ERR_ARG for an option the plan
- * cannot run, or while a gr_graph holds the plan. */
+ * the persistent column FFT, whose next strip lands during the transform, for chunks of any
+ * size, where M >= 256, strips are two columns or wider and its buffers fit in shared memory;
+ * 0: one strip per CTA; -1: keep).  GR_ERR_ARG for an option the plan cannot run, or while a
+ * gr_graph holds the plan. */
 int gr_plan_set_tuning(gr_plan* plan, int grid_kernel, int item_cap, int cols_group,
                        int cols_ring);
-/* The full tuning: gridding kernel of a full chunk, its item cap, column group width
- * and whether the column FFT runs persistent. */
+/* The full tuning: gridding kernel of a full chunk (as gr_plan_grid_kernel reports), its item
+ * cap, the column group width and whether the column FFT runs persistent: as tuned or
+ * pinned, else what a full chunk runs by default. */
 int gr_plan_tuning_ex(const gr_plan* plan, int* grid_kernel, int* item_cap, int* cols_group,
                       int* cols_ring);
 

@@ -213,8 +213,9 @@ struct ColArgs {
   const float2* tw;      // two-level twiddle table for M
   int M, pairs;
   int* err;              // device error word for bounded-wait timeouts (null: plain loads)
-  int G = 0;             // columns per CTA (0: cols_group(M, ring))
-  int ring = 0;          // 1: persistent CTAs, next strip landing (cols_ring_kernel)
+  int G = 0;             // columns per CTA (0: by cols_form)
+  int ring = -1;         // 1: persistent CTAs, next strip landing (cols_ring_kernel), 0: a strip per
+                         // CTA, -1: by cols_form
   // rows of H that are read afterwards: row iu with (iu + shift) mod M in [row0, row0 + rows)
   int shift = 0, row0 = 0, rows = 1 << 30;
 };
@@ -313,8 +314,12 @@ cudaError_t launch_grid_w32(const GridArgs& a, cudaStream_t s);
 cudaError_t launch_grid_group(const GridArgs& a, int G, cudaStream_t s);
 cudaError_t launch_tap_records(const GridArgs& a, int subs, int spw, int* counts, const int* base,
                                TapRec* rec, cudaStream_t s);
-int cols_group(int M, int ring);
-int cols_ring_default(int M);
+// The form in which launch_cols transforms: a width and a form asked for, or the default ones
+// (0, -1) for so many pairs.
+struct ColForm {
+  int G, ring;
+};
+ColForm cols_form(int M, int pairs, int G, int ring);
 cudaError_t launch_cols(const ColArgs& a, cudaStream_t s);
 cudaError_t launch_rows(const RowArgs& a, cudaStream_t s);
 cudaError_t launch_wait_probe(int* err, int limit, cudaStream_t s);

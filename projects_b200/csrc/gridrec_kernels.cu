@@ -2454,12 +2454,12 @@ cudaError_t launch_grid_tc(const GridArgs& a, cudaStream_t s) {
 // 4; 18.0 with 8) against 14.4 (G = 8; 17.7 with 4) for 32 pairs, 17.4 against 17.0 for 4,
 // even for one; M = 1024 3.5 against 3.9, 512 1.2 against 1.4 (G = 8).  At M = 8192 no
 // persistent form has strips wide enough: 519 with G = 2, 931 with 1, 600 persistent.
-int cols_ring_default(int M) { return M == 2048 || M == 4096; }
+static bool cols_ring_default(int M) { return M == 2048 || M == 4096; }
 
 // Columns per CTA: up to 512 threads of M / 16 a column, 1024 where narrower strips would
 // leave the 32-byte sectors of a row half used (M = 8192) and for the persistent kernel,
 // whose one CTA per SM takes them all.
-int cols_group(int M, int ring) {
+static int cols_group(int M, int ring) {
   const int g = (ring || M >= 8192 ? 16384 : 8192) / M;
   return g < 1 ? 1 : (g > 8 ? 8 : g);
 }
@@ -2480,9 +2480,27 @@ static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
   return fn;
 }
 
+static int cols_ring_smem(int M, int G) {
+  return (kTwSlots + G * M) * (int)sizeof(float2) + (G * M + 32) * (int)sizeof(float) + (int)sizeof(uint64_t);
+}
+
+// By default the persistent kernel wants four strips per SM, for its last round to weigh little
+// (M = 2048, us a pair: one pair 24.8 with and without, two 20.8 against 19.4, four 17.0
+// against 17.4).  It transforms lines of 256 and more (the exchanges of shorter ones are not
+// compiled), in strips of at least two columns whose buffers fit.
+ColForm cols_form(int M, int pairs, int G, int ring) {
+  const int Gr = G > 0 ? G : cols_group(M, 1);
+  if (ring < 0) ring = cols_ring_default(M) && (long)(M / Gr) * pairs >= 4 * 148;
+  int optin = 0, dev = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (ring && (M < 256 || Gr < 2 || cols_ring_smem(M, Gr) > optin)) ring = 0;
+  return {G > 0 ? G : cols_group(M, ring), ring};
+}
+
 template <bool WIN>
 static cudaError_t launch_cols_t(const ColArgs& a, cudaStream_t s) {
-  const int G = a.G > 0 ? a.G : cols_group(a.M, a.ring);
+  const int G = a.G;
   const int threads = G * (a.M / 16);
   PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
   if (a.err && encode && G >= 2 && a.M >= 16 && ((uintptr_t)a.H % 16) == 0) {
@@ -2496,13 +2514,11 @@ static cudaError_t launch_cols_t(const ColArgs& a, cudaStream_t s) {
     CUresult r = encode(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, (void*)a.H, dims, strides, box,
                         estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    int optin = 0, dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int ring_smem = (kTwSlots + G * a.M) * (int)sizeof(float2) + (G * a.M + 32) * (int)sizeof(float) +
-                          (int)sizeof(uint64_t);
-    if (r == CUDA_SUCCESS && a.ring && a.M >= 256 && ring_smem <= optin) {
+    if (r == CUDA_SUCCESS && a.ring) {
+      int dev = 0, sms = 0;
+      cudaGetDevice(&dev);
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+      const int ring_smem = cols_ring_smem(a.M, G);
       const int total = (a.M / G) * a.pairs;
       // persistent: as many CTAs as fit on the SMs at once
 #define GR_COLR(NT)                                                                              \
@@ -2545,10 +2561,9 @@ static cudaError_t launch_cols_t(const ColArgs& a, cudaStream_t s) {
 }
 cudaError_t launch_cols(const ColArgs& args, cudaStream_t s) {
   ColArgs a = args;
-  // by default the persistent kernel wants four strips per SM, for its last round to weigh
-  // little (M = 2048, us a pair: one pair 24.8 with and without, two 20.8 against 19.4, four
-  // 17.0 against 17.4)
-  if (a.G <= 0 && a.ring && (long)(a.M / cols_group(a.M, 1)) * a.pairs < 4 * 148) a.ring = 0;
+  const ColForm f = cols_form(a.M, a.pairs, a.G, a.ring);
+  a.G = f.G;
+  a.ring = f.ring;
   return a.rows < a.M ? launch_cols_t<true>(a, s) : launch_cols_t<false>(a, s);
 }
 

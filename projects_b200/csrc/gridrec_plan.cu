@@ -177,8 +177,9 @@ struct Plan {
   // gridding by groups of pairs (grid_group_kernel), with the sums in the order of the tile
   // kernel's list and of the 16-pair kernel's
   GroupList g_tiles, g_wide;
-  int cols_G = 0;                   // column-FFT group width (0 = cols_group(M, ring); autotuned)
-  int cols_ring = 0;                // 1: persistent column FFT (cols_ring_default(M); autotuned)
+  // column-FFT group width and whether it runs persistent, as autotuned or asked for (0, -1:
+  // by cols_form for each chunk)
+  int cols_G = 0, cols_ring = -1;
   // gridding kernel of full chunks (max_pairs pairs) in the default mode, chosen by the
   // autotuner or gr_plan_set_tuning: 0 tiles, 1 16-pair, 3 32-pair (-1: by chunk size)
   int tuned_kernel = -1;
@@ -1446,7 +1447,6 @@ int gr::plan_create_ex(const gr_params* prm, const Pswf* pswf, float (*filter_fn
   p->pdim = (int)pdim;
   p->J = (int)(pdim / 2);
   p->M = (int)M;
-  p->cols_ring = cols_ring_default(p->M);
   p->M02 = (int)M02;
   p->M0 = (int)geo.M0;
   p->sampl = geo.sampl;
@@ -1742,7 +1742,7 @@ int gr_plan_autotune(gr_plan* p, void* stream) {
   };
   cudaMemsetAsync(p->d_spec, 0, (size_t)p->spec_pairs * p->n_ang * 2 * p->J * sizeof(float2), st);
   cudaMemsetAsync(p->d_H, 0, (size_t)pairs * p->M * p->M * sizeof(float2), st);
-  Tuned best{kernels[0], p->item_cap, p->w_item_cap, 0, 0};
+  Tuned best{kernels[0], p->item_cap, p->w_item_cap, p->cols_G, p->cols_ring};
   float best_t = 1e30f;
   int best_cap_t = p->item_cap, best_cap_w = p->w_item_cap, rc = GR_OK;
   float best_tt = 1e30f, best_tw = 1e30f;
@@ -1859,7 +1859,11 @@ int gr_plan_tuning_ex(const gr_plan* p, int* grid_kernel, int* item_cap, int* co
     const int pr = p->max_pairs;
     *grid_kernel = gr::use_tc(p, pr) ? 2 : (gr::use_w32(p, pr) ? 3 : (gr::use_wide(p, pr) ? 1 : 0));
   }
-  if (cols_ring) *cols_ring = p->cols_ring;
+  if (cols_ring) {
+    gr::DeviceGuard g(p->device);
+    *cols_ring = p->cols_ring >= 0 ? p->cols_ring
+                                   : gr::cols_form(p->M, p->max_pairs, p->cols_G, p->cols_ring).ring;
+  }
   return gr_plan_tuning(p, item_cap, cols_group);
 }
 
@@ -1868,7 +1872,10 @@ int gr_plan_tuning(const gr_plan* p, int* item_cap, int* cols_group_width) {
   // the item cap of the work list a full chunk grids with
   const bool wl4x8 = gr::use_wide(p, p->max_pairs) || gr::use_w32(p, p->max_pairs);
   if (item_cap) *item_cap = wl4x8 ? p->w_item_cap : p->item_cap;
-  if (cols_group_width) *cols_group_width = p->cols_G > 0 ? p->cols_G : gr::cols_group(p->M, p->cols_ring);
+  if (cols_group_width) {
+    gr::DeviceGuard g(p->device);
+    *cols_group_width = gr::cols_form(p->M, p->max_pairs, p->cols_G, p->cols_ring).G;
+  }
   return GR_OK;
 }
 

@@ -277,7 +277,8 @@ class Plan:
 
     def grid_kernel(self, pairs=None) -> str:
         """'wide32' (32 pairs per warp), 'wide' (16 pairs per warp), 'tensor'
-        (tcgen05) or 'tiles' for a chunk of `pairs` pairs."""
+        (tcgen05) or 'tiles' for a chunk of `pairs` pairs: the kernel whose work list and
+        bits the chunk has (chunks of up to 8 pairs grid by groups of pairs in its order)."""
         w = C.c_int()
         _check(lib().gr_plan_grid_kernel(self._h, int(pairs or self.max_pairs), C.byref(w)),
                "gr_plan_grid_kernel")
@@ -319,7 +320,7 @@ class Plan:
         """Pins a tuning: grid_kernel ('tiles', 'wide', 'wide32' or None for the
         choice by chunk size) for full chunks, its work list's item cap (0: keep),
         the column-FFT group width (0: keep) and cols_ring (True: persistent
-        column FFT, False: one strip per CTA, None: keep)."""
+        column FFT from M = 256, False: one strip per CTA, None: keep)."""
         k = -1 if grid_kernel is None else self.GRID_KERNEL_CODES[grid_kernel]
         ring = -1 if cols_ring is None else int(bool(cols_ring))
         _check(lib().gr_plan_set_tuning(self._h, k, int(item_cap), int(cols_group), ring),

@@ -342,3 +342,31 @@ def test_fbp_too_many_angles_refused_and_nothing_left_behind():
         assert ph.rel_l2(got, O.port_optimized_fbp(x[0, :7000].cpu().numpy(), ph.angles_deg(7000))) < 1e-5
     many.close()
     some.close()
+
+
+@pytest.mark.parametrize("n,pairs,group,ring", [(2048, 1, 4, False), (2048, 2, 4, False), (2048, 3, 8, True),
+                                                (1024, 4, 8, False), (4096, 1, 4, True), (8192, 1, 2, False)])
+def test_column_form_reported_and_pinned(n, pairs, group, ring):
+    """The tuning names the column FFT that a full chunk runs by default (persistent from
+    four strips per SM at M = 2048 and 4096), and keeps what is pinned, also a persistent
+    form without a width for a chunk of few strips: the same bits."""
+    a = 3
+    S = 2 * pairs
+    sinos = _dev(np.random.default_rng(n).uniform(0.0, 2.0, (S, a, n)).astype(np.float32))
+    with G.Plan(n, a, ph.angles_deg(a), filter=G.FILTER_HANN, max_pairs=pairs) as plan:
+        def images():
+            o = torch.full((S, plan.M0, max(plan.M0, n)), float("nan"), device="cuda")
+            plan.reconstruct_batch(sinos, o)
+            torch.cuda.synchronize()
+            plan.device_status()
+            return o[:, :, :plan.M0]
+
+        t = plan.tuning()
+        assert (t["cols_group"], t["cols_ring"]) == (group, ring)
+        want = images()
+        t = plan.set_tuning(cols_ring=True)
+        assert (t["cols_group"], t["cols_ring"]) == (min(8, 16384 // n), True)
+        assert torch.equal(images(), want)
+        t = plan.set_tuning(cols_ring=False)
+        assert (t["cols_group"], t["cols_ring"]) == (2 if n == 8192 else min(8, 8192 // n), False)
+        assert torch.equal(images(), want)
