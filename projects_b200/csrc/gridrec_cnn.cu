@@ -1004,6 +1004,7 @@ extern "C" {
 int gr_cnn_param_count(void) { return kCnnParams; }
 
 size_t gr_cnn_workspace_bytes(int n_img, int h, int w) {
+  if (n_img < 1 || h < 1 || w < 1) return 0;
   const size_t px = (size_t)n_img * h * w;
   // h1, h2, gz1, gz2 (bf16 x 16) + gy (f32) + block partials + loss partials
   return 4 * px * kC * 2 + px * 4 + (size_t)wg_blocks(n_img, h, w) * kCnnParams * 4 + 1024 * 8 + 1024;

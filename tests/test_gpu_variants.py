@@ -370,3 +370,12 @@ def test_column_form_reported_and_pinned(n, pairs, group, ring):
         t = plan.set_tuning(cols_ring=False)
         assert (t["cols_group"], t["cols_ring"]) == (2 if n == 8192 else min(8, 8192 // n), False)
         assert torch.equal(images(), want)
+
+
+def test_network_refuses_an_empty_minibatch():
+    from projects_b200 import learned as L
+    net = L.CorrectionNet(L.init_params(1))
+    for shape in ((0, 8, 8), (2, 0, 8), (2, 8, 0)):
+        x = torch.empty(shape, device="cuda")
+        with pytest.raises(G.GrError, match="GR_ERR_ARG"):
+            net.loss_and_grads(x, x)

@@ -432,3 +432,12 @@ def test_ring_workspace_never_falls_as_a_dimension_grows():
     slices = list(range(1, 42)) + [63, 64, 65, 255, 256, 739, 740, 741, 1500, 4096]
     bad = _falls(f, (slices, [9, 512, 1024, 1028, 2047, 2048, 2052, 4096, 4100], [1, 3, 4, 5, 37, 720, 1500, 1501, 6000]))
     assert not bad, bad[:5]
+
+
+def test_network_workspace_of_an_empty_minibatch_is_nothing():
+    """The size query of a size that the calls refuse, as the Python class makes it before the
+    call: 0, not an arithmetic fault."""
+    from projects_b200 import learned as L
+    f = L._lib().gr_cnn_workspace_bytes
+    assert [f(0, 8, 8), f(1, 0, 8), f(1, 8, 0), f(-1, 8, 8)] == [0, 0, 0, 0]
+    assert f(1, 1, 1) > 0
