@@ -437,7 +437,8 @@ int gr_fbp_destroy(gr_fbp* fbp);
  * float32).  params: gr_cnn_param_count() floats, layout w1[9][16], b1[16],
  * w2[9][16][16], b2[16], w3[9][16], b3.  conv2 runs on BF16 tensor cores with FP32
  * accumulation; hidden activations are stored as BF16.  The workspace
- * (gr_cnn_workspace_bytes) keeps the forward activations that gr_cnn_backward uses:
+ * (gr_cnn_workspace_bytes, which never falls as a size grows and is 0 for a size below 1)
+ * keeps the forward activations that gr_cnn_backward uses:
  * call backward after forward on the same images and workspace.  gr_cnn_backward
  * writes the mean-squared-loss gradient to grads and the loss to *loss (synchronises
  * when loss is non-NULL); gr_cnn_adam applies one Adam step (step counts from 1). */

@@ -420,6 +420,12 @@ int wg_segments(int n_img, int h, int w) { return strip_segments(n_img, h, w, kW
 long wg_blocks(int n_img, int h, int w) {
   return (long)n_img * ((w + kWgW - 1) / kWgW) * wg_segments(n_img, h, w);
 }
+// The most blocks of a call of up to these sizes: wg_blocks falls where a strip more leaves
+// room for fewer segments of each.
+size_t wg_blocks_bound(int n_img, int h, int w) {
+  const size_t strips = (size_t)n_img * ((w + kWgW - 1) / kWgW);
+  return std::max(strips, std::min(strips * h, (size_t)kWgBlocks * 148));
+}
 
 __device__ __forceinline__ void cp_async_zfill4(void* dst, const void* src, bool ok) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(smem_u32(dst)), "l"(src),
@@ -1007,7 +1013,7 @@ size_t gr_cnn_workspace_bytes(int n_img, int h, int w) {
   if (n_img < 1 || h < 1 || w < 1) return 0;
   const size_t px = (size_t)n_img * h * w;
   // h1, h2, gz1, gz2 (bf16 x 16) + gy (f32) + block partials + loss partials
-  return 4 * px * kC * 2 + px * 4 + (size_t)wg_blocks(n_img, h, w) * kCnnParams * 4 + 1024 * 8 + 1024;
+  return 4 * px * kC * 2 + px * 4 + wg_blocks_bound(n_img, h, w) * kCnnParams * 4 + 1024 * 8 + 1024;
 }
 
 size_t gr_cnn_forward_workspace_bytes(int n_img, int h, int w) {

@@ -441,3 +441,12 @@ def test_network_workspace_of_an_empty_minibatch_is_nothing():
     f = L._lib().gr_cnn_workspace_bytes
     assert [f(0, 8, 8), f(1, 0, 8), f(1, 8, 0), f(-1, 8, 8)] == [0, 0, 0, 0]
     assert f(1, 1, 1) > 0
+
+
+def test_network_workspace_never_falls_as_a_dimension_grows():
+    """As for ring removal: one buffer for the largest minibatch."""
+    from projects_b200 import learned as L
+    f = L._lib().gr_cnn_workspace_bytes
+    images = list(range(1, 30)) + [55, 56, 74, 75, 111, 112, 148, 149, 221, 222, 223, 224, 443, 444, 445, 900]
+    bad = _falls(f, (images, [1, 2, 3, 16, 32, 64, 65, 300], [1, 32, 63, 64, 65, 128, 129, 512]))
+    assert not bad, bad[:5]
