@@ -390,31 +390,43 @@ __global__ void cnn_conv3_bwd_kernel(const float* params, const float* gy,
 }
 
 // Weight gradients of all three layers on the tensor cores, contracted over pixels.
-// A block of 4 warps walks down a strip of kWgW columns, 16 pixels of the row per warp;
-// per row and warp (mma.m16n8k16, K = the 16 pixels q, FP32 accumulators kept for the
-// whole strip segment):
-//   dW2[tap][co][ci] = sum_q gz2[q][co] h1[q + off][ci]   A = gz2^T, B = h1 shifted, 18 MMAs
+// A block of 4 warps walks down a strip of kWgW columns, 64 pixels of a row in four groups
+// q of 16 (mma.m16n8k16, K = the 16 pixels):
+//   dW2[tap][co][ci] = sum_q gz2[q][co] h1[q + off][ci]   A = gz2^T, B = h1 shifted
 //   dW1[tap][co]     = sum_q gz1[q][co] x[q + off]         A = gz1^T, B = x's taps and a one
 //   dW3[tap][ci]     = sum_q gy[q - off] h2[q][ci]         A = gy's taps, B = h2
 //   db2[co] = sum gz2, db1 (the column of ones of dW1's B), db3 = sum gy
 // gz1, gz2, h1 and h2 are BF16 already, so their products are exact; the FP32 operands x
-// and gy enter as three BF16 parts each, which add up to the FP32 value.  Rows arrive by
-// cp.async a row ahead into rings (three rows of h1, x and gy are in use); pixels lie 48
-// bytes apart, so that the eight 16-byte rows of an ldmatrix fall on distinct banks.
+// and gy enter as three BF16 parts each, which add up to the FP32 value.
+// The tensor core cuts off what its FP32 accumulator cannot hold instead of rounding, so
+// a sum kept in the accumulator loses up to 2^-24 of itself with every MMA (7e-6 of the
+// gradients at 4 x 1024 x 1024, 6e-5 at 4096 x 4096).  Every MMA therefore starts from zero;
+// its 16 pixels are added to a sum in registers (rounded to nearest), and those sums of at
+// most 128 additions to FP64 sums in shared memory every kWgFlush rows.  A warp takes two
+// taps of dW2 for the whole row, and tap 8, dW1, dW3 and the biases for its own group of 16
+// pixels, so that its sums fit the registers.
+// Rows arrive by cp.async a row ahead into rings (three rows of h1, x and gy are in use);
+// pixels lie 48 bytes apart, so that the eight 16-byte rows of an ldmatrix fall on distinct
+// banks.
 // Bound: the latency of a row's exchanges (one row of 64 pixels per barrier), then DRAM
-// (136 bytes per pixel).  4 x 1024 x 1024: 232 us and 5 us for the reduction of 384 blocks,
-// against 2179 us on the CUDA cores and 1444 us for the reduction of 32768 segments.
+// (136 bytes per pixel).  4 x 1024 x 1024: 247 us and 6 us for the reduction of 384 blocks,
+// error against the exact contraction of the same operands 2.4e-8 to 2.9e-8; 237 us and
+// up to 8e-6 with the sums kept in the accumulators; 2179 us on the CUDA cores and 1444 us for the
+// reduction of 32768 segments, 2.4e-8 to 2.9e-8.
 constexpr int kWgW = kStW, kWgThreads = 128, kWgBlocks = 3;  // blocks per SM
+constexpr int kWgFlush = 32;                                 // rows: 4 additions each
 constexpr int kWgPx = kStPx;
 constexpr int kWgHalo = kWgW + 2;
+// A warp's FP64 sums: dW2 of its two taps and of tap 8, then those of its own pixels.
+constexpr int kWgOwn = 3 * kC * kC;  // dW1, db1, dW3, db2, db3
+constexpr int kWgOwnB1 = kWgOwn + 9 * kC, kWgOwnW3 = kWgOwnB1 + kC, kWgOwnB2 = kWgOwnW3 + 9 * kC;
+constexpr int kWgOwnB3 = kWgOwnB2 + kC, kWgSums = kWgOwnB3 + 1;
 struct WgSmem {
   alignas(16) unsigned char h1[4][kWgHalo * kWgPx];        // ring over rows y - 1 .. y + 2
   alignas(16) unsigned char g1[2][kWgW * kWgPx], g2[2][kWgW * kWgPx], h2[2][kWgW * kWgPx];
   float x[4][kWgHalo], gy[4][kWgHalo];
+  double sums[kWgThreads / 32][kWgSums];
 };
-
-static_assert(sizeof(WgSmem) <= 48 * 1024 && sizeof(WgSmem) >= kCnnParams * sizeof(float),
-              "default shared-memory limit; the sums fit over the rings");
 
 int wg_segments(int n_img, int h, int w) { return strip_segments(n_img, h, w, kWgBlocks); }
 long wg_blocks(int n_img, int h, int w) {
@@ -454,6 +466,20 @@ __device__ __forceinline__ void split3(float a, float b, unsigned (&o)[3]) {
   }
 }
 
+// The MMA from zero: d = a b.
+__device__ __forceinline__ void mma_bf16_zero(float (&d)[4], const unsigned (&a)[4], unsigned b0,
+                                              unsigned b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
+      "{%8,%9}, {%10,%10,%10,%10};\n"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
+__device__ __forceinline__ void add4(float (&s)[4], const float (&d)[4]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) s[i] = __fadd_rn(s[i], d[i]);
+}
+
 __global__ void __launch_bounds__(kWgThreads, kWgBlocks) cnn_wgrad_kernel(
     const float* x, const float* gy, const __nv_bfloat16* h1, const __nv_bfloat16* h2,
     const __nv_bfloat16* gz1, const __nv_bfloat16* gz2, float* part, int h, int w, int segs) {
@@ -491,18 +517,25 @@ __global__ void __launch_bounds__(kWgThreads, kWgBlocks) cnn_wgrad_kernel(
       cp_async_zfill16(sm.h2[slot] + o, reinterpret_cast<const unsigned char*>(h2) + p, ok);
     }
   };
-  float a2[9][2][4], a1[2][4], a3[2][4], ab[4];
+  // this warp's FP32 sums: dW2 of taps 2 warp, 2 warp + 1 and 8 (two n = 8 tiles each), dW1,
+  // dW3, db2, db3
+  float a2[3][2][4], a1[2][4], a3[2][4], ab[4], b3 = 0.f;
+  auto clear = [&]() {
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < 4; ++i) {
 #pragma unroll
-    for (int n = 0; n < 2; ++n) {
+      for (int n = 0; n < 2; ++n) {
 #pragma unroll
-      for (int tap = 0; tap < 9; ++tap) a2[tap][n][i] = 0.f;
-      a1[n][i] = a3[n][i] = 0.f;
+        for (int k = 0; k < 3; ++k) a2[k][n][i] = 0.f;
+        a1[n][i] = a3[n][i] = 0.f;
+      }
+      ab[i] = 0.f;
     }
-    ab[i] = 0.f;
-  }
-  float b3 = 0.f;
+    b3 = 0.f;
+  };
+  clear();
+  double* sums = sm.sums[warp];
+  for (int i = lane; i < kWgSums; i += 32) sums[i] = 0.0;
   const unsigned one2 = lane < 4 ? 0x3f803f80u : 0u;  // B column 0 of ones
   load_halo_row(y0 - 1);
   load_halo_row(y0);
@@ -510,41 +543,59 @@ __global__ void __launch_bounds__(kWgThreads, kWgBlocks) cnn_wgrad_kernel(
   load_row(y0);
   asm volatile("cp.async.commit_group;\n" ::: "memory");
   const int g = lane >> 2, t = lane & 3;
-  const int q0 = warp * 16;  // this warp's pixels of the row
+  const int q0 = warp * 16;  // this warp's own pixels of the row
+  __syncwarp();              // its sums are zero for all its lanes
   for (int y = y0; y < y1; ++y) {
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();  // row y and its neighbours are there for every thread, row y - 2 is free
     if (y + 1 < y1) {
       load_halo_row(y + 2);
       load_row(y + 1);
     }
     asm volatile("cp.async.commit_group;\n" ::: "memory");
-    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-    __syncthreads();  // row y and its neighbours are there for every thread
     unsigned fa[4], fb[4];
-    ldm_t(fa, sm.g2[y & 1] + q0 * kWgPx, lane);
-    mma_bf16(ab, fa, one2, one2);
+    float d[4], small[4];
+    // dW2 of tap `tap` over the 16 pixels at q, whose gz2 fa holds
+    auto tap_sums = [&](float (&s)[2][4], int tap, int q) {
+      ldm_t(fb, sm.h1[(y + tap_dy(tap)) & 3] + (q + 1 + tap_dx(tap)) * kWgPx, lane);
 #pragma unroll
-    for (int tap = 0; tap < 9; ++tap) {
-      ldm_t(fb, sm.h1[(y + tap_dy(tap)) & 3] + (q0 + 1 + tap_dx(tap)) * kWgPx, lane);
-      mma_bf16(a2[tap][0], fa, fb[0], fb[2]);
-      mma_bf16(a2[tap][1], fa, fb[1], fb[3]);
+      for (int n = 0; n < 2; ++n) {
+        mma_bf16_zero(d, fa, fb[n], fb[n + 2]);
+        add4(s[n], d);
+      }
+    };
+#pragma unroll
+    for (int q = 0; q < kWgW; q += 16) {
+      ldm_t(fa, sm.g2[y & 1] + q * kWgPx, lane);
+      tap_sums(a2[0], 2 * warp, q);
+      tap_sums(a2[1], 2 * warp + 1, q);
     }
-    // dW1: B column n = tap (n = 9: ones); this lane's columns g and g + 8
+    ldm_t(fa, sm.g2[y & 1] + q0 * kWgPx, lane);
+    tap_sums(a2[2], 8, q0);
+    mma_bf16_zero(d, fa, one2, one2);
+    add4(ab, d);
+    // dW1: B column n = tap (n = 9: ones); this lane's columns g and g + 8.  The two
+    // small parts share an accumulator, the largest has its own.
     ldm_t(fa, sm.g1[y & 1] + q0 * kWgPx, lane);
     {
       const float* r = sm.x[(y + g / 3 - 1) & 3] + q0 + g % 3;  // x[q + off(g)], halo offset in
       unsigned lo[3], hi[3];
       split3(r[2 * t], r[2 * t + 1], lo);
       split3(r[2 * t + 8], r[2 * t + 9], hi);
-#pragma unroll
-      for (int k = 0; k < 3; ++k) mma_bf16(a1[0], fa, lo[k], hi[k]);
+      mma_bf16_zero(small, fa, lo[2], hi[2]);
+      mma_bf16(small, fa, lo[1], hi[1]);
+      mma_bf16_zero(d, fa, lo[0], hi[0]);
+      add4(d, small);
+      add4(a1[0], d);
       const float* r8 = sm.x[(y + 1) & 3] + q0 + 2;             // tap 8
       split3(r8[2 * t], r8[2 * t + 1], lo);
       split3(r8[2 * t + 8], r8[2 * t + 9], hi);
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        const unsigned one = g == 1 && k == 0 ? 0x3f803f80u : 0u;
-        mma_bf16(a1[1], fa, g == 0 ? lo[k] : one, g == 0 ? hi[k] : one);
-      }
+      const unsigned one = g == 1 ? 0x3f803f80u : 0u;
+      mma_bf16_zero(small, fa, g == 0 ? lo[2] : 0u, g == 0 ? hi[2] : 0u);
+      mma_bf16(small, fa, g == 0 ? lo[1] : 0u, g == 0 ? hi[1] : 0u);
+      mma_bf16_zero(d, fa, g == 0 ? lo[0] : one, g == 0 ? hi[0] : one);
+      add4(d, small);
+      add4(a1[1], d);
     }
     // dW3: A row m = tap; this lane's rows g and g + 8 (tap 8 for g = 0)
     ldm_t(fb, sm.h2[y & 1] + q0 * kWgPx, lane);
@@ -557,42 +608,57 @@ __global__ void __launch_bounds__(kWgThreads, kWgBlocks) cnn_wgrad_kernel(
       split3(r8[2 * t], r8[2 * t + 1], lo8);
       split3(r8[2 * t + 8], r8[2 * t + 9], hi8);
 #pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        const unsigned a[4] = {lo[k], g == 0 ? lo8[k] : 0u, hi[k], g == 0 ? hi8[k] : 0u};
-        mma_bf16(a3[0], a, fb[0], fb[2]);
-        mma_bf16(a3[1], a, fb[1], fb[3]);
+      for (int n = 0; n < 2; ++n) {
+#pragma unroll
+        for (int k = 2; k >= 0; --k) {
+          const unsigned a[4] = {lo[k], g == 0 ? lo8[k] : 0u, hi[k], g == 0 ? hi8[k] : 0u};
+          if (k == 2) mma_bf16_zero(small, a, fb[n], fb[n + 2]);
+          else if (k == 1) mma_bf16(small, a, fb[n], fb[n + 2]);
+          else mma_bf16_zero(d, a, fb[n], fb[n + 2]);
+        }
+        add4(d, small);
+        add4(a3[n], d);
       }
       if (lane < 16) b3 += sm.gy[y & 3][q0 + 1 + lane];
     }
-    __syncthreads();  // the rings' oldest rows are read before they are refilled
-  }
-  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-  // the four warps' sums in warp order, in shared memory over the rings
-  float* acc = reinterpret_cast<float*>(smw);
-  for (int o = 16; o > 0; o >>= 1) b3 += __shfl_xor_sync(0xffffffffu, b3, o);
-  for (int k = 0; k < kWgThreads / 32; ++k) {
-    __syncthreads();
-    if (warp != k) continue;
-    auto put = [&](int i, float v) { acc[i] = k == 0 ? v : acc[i] + v; };
+    if ((y - y0) % kWgFlush == kWgFlush - 1 || y == y1 - 1) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int row = g + (i >> 1) * 8, col = 2 * t + (i & 1);
+      for (int i = 0; i < 4; ++i) {
+        const int row = g + (i >> 1) * 8, col = 2 * t + (i & 1);
 #pragma unroll
-      for (int n = 0; n < 2; ++n) {
+        for (int n = 0; n < 2; ++n) {
 #pragma unroll
-        for (int tap = 0; tap < 9; ++tap) put(kW2 + (tap * kC + row) * kC + n * 8 + col, a2[tap][n][i]);
-        const int tap1 = n * 8 + col;                      // a1: row = co, column = tap
-        if (tap1 < 9) put(kW1 + tap1 * kC + row, a1[n][i]);
-        if (tap1 == 9) put(kB1 + row, a1[n][i]);
-        if (row < 9) put(kW3 + row * kC + n * 8 + col, a3[n][i]);  // a3: row = tap, column = ci
+          for (int k = 0; k < 3; ++k) sums[(k * kC + row) * kC + n * 8 + col] += a2[k][n][i];
+          const int tap1 = n * 8 + col;                      // a1: row = co, column = tap
+          if (tap1 < 9) sums[kWgOwn + tap1 * kC + row] += a1[n][i];
+          if (tap1 == 9) sums[kWgOwnB1 + row] += a1[n][i];
+          if (row < 9) sums[kWgOwnW3 + row * kC + n * 8 + col] += a3[n][i];  // a3: row = tap, column = ci
+        }
+        if (col == 0) sums[kWgOwnB2 + row] += ab[i];
       }
-      if (col == 0) put(kB2 + row, ab[i]);
+      double s = b3;
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (lane == 0) sums[kWgOwnB3] += s;
+      clear();
     }
-    if (lane == 0) put(kB3, b3);
   }
   __syncthreads();
+  // the block's sums, those that every warp holds in warp order
   float* out = part + ((size_t)im * gridDim.x + blockIdx.x) * kCnnParams;
-  for (int i = tid; i < kCnnParams; i += kWgThreads) out[i] = acc[i];
+  auto all = [&](int i) { return (float)(((sm.sums[0][i] + sm.sums[1][i]) + sm.sums[2][i]) + sm.sums[3][i]); };
+  constexpr int kTap = kC * kC;
+  for (int i = tid; i < 8 * kTap; i += kWgThreads)
+    out[kW2 + i] = (float)sm.sums[i / (2 * kTap)][i % (2 * kTap)];
+  for (int i = tid; i < kTap; i += kWgThreads) out[kW2 + 8 * kTap + i] = all(2 * kTap + i);
+  for (int i = tid; i < 9 * kC; i += kWgThreads) {
+    out[kW1 + i] = all(kWgOwn + i);
+    out[kW3 + i] = all(kWgOwnW3 + i);
+  }
+  if (tid < kC) {
+    out[kB1 + tid] = all(kWgOwnB1 + tid);
+    out[kB2 + tid] = all(kWgOwnB2 + tid);
+  }
+  if (tid == 0) out[kB3] = all(kWgOwnB3);
 }
 
 // grads[k] = sum over blocks (fixed order) of part[block][k], in double: 32 parameters x 8
@@ -1066,10 +1132,12 @@ int gr_cnn_backward(const float* params, const float* x, const float* y, const f
   const int s2 = strip_segments(n_img, h, w, kStBlocks);
   cnn_conv2_kernel<<<dim3((w + kStW - 1) / kStW * s2, n_img), kStThreads, 0, st>>>(params, gz2, h1, gz1,
                                                                                   h, w, 1, s2);
+  cudaError_t e = cudaFuncSetAttribute(cnn_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)sizeof(WgSmem));
+  if (e != cudaSuccess) return fail(GR_ERR_CUDA, "cnn backward: %s", cudaGetErrorString(e));
   cnn_wgrad_kernel<<<dim3((unsigned)(blocks / n_img), n_img), kWgThreads, sizeof(WgSmem), st>>>(
       x, gy, h1, h2, gz1, gz2, part, h, w, segs);
   cnn_reduce_kernel<<<(kCnnParams + 31) / 32, 256, 0, st>>>(part, blocks, grads);
-  cudaError_t e = cudaSuccess;
   if (loss) {
     double lp[lblocks];
     e = cudaMemcpyAsync(lp, lpart, sizeof(lp), cudaMemcpyDeviceToHost, st);

@@ -379,3 +379,50 @@ def test_network_refuses_an_empty_minibatch():
         x = torch.empty(shape, device="cuda")
         with pytest.raises(G.GrError, match="GR_ERR_ARG"):
             net.loss_and_grads(x, x)
+
+
+@pytest.mark.parametrize("shape", [(223, 200, 60), (1, 900, 130), (2, 33, 64), (3, 65, 17)])
+@pytest.mark.parametrize("signs", ["one", "mixed"])
+def test_network_weight_gradients_exact_contraction(shape, signs):
+    """The weight gradients against the float64 contraction of the activations and gradients
+    that the backward pass itself stored (BF16, FP32 for x and the output's gradient), in units
+    of the sum of the terms' magnitudes.  One image's whole height per block, several segments, all
+    terms of one sign (where errors of one sign add up) and of both.  Bound 3e-7: the result's
+    own rounding (2^-24), what an MMA of 16 pixels cuts off (2^-23) and 128 rounded FP32 additions
+    on a growing sum (0.6 sqrt(128 / 3) 2^-25 = 1.2e-7)."""
+    from projects_b200 import learned as L
+    n, h, w = shape
+    rng = np.random.default_rng(h)
+    p = rng.normal(0, 0.2, 2625).astype(np.float32)
+    x = rng.uniform(0.5, 1.5, shape).astype(np.float32)
+    if signs == "one":
+        p = np.abs(p)
+        target = np.zeros_like(x)
+    else:
+        x -= 1.0
+        target = (x + rng.normal(0, 0.3, shape)).astype(np.float32)
+    net = L.CorrectionNet(p)
+    x = _dev(x)
+    net.loss_and_grads(x, _dev(target))
+    px = n * h * w  # the workspace: h1, h2, gz1, gz2 (BF16 x 16), the output's gradient
+    h1, h2, g1, g2 = (net._ws[k * px * 32:(k + 1) * px * 32].view(torch.bfloat16).view(n, h, w, 16).double()
+                      for k in range(4))
+    gy = net._ws[4 * px * 32:4 * px * 32 + 4 * px].view(torch.float32).view(n, h, w).double()
+
+    def grads(x, h1, h2, g1, g2, gy):
+        out = torch.zeros(2625, dtype=torch.float64, device="cuda")
+        pad = torch.nn.functional.pad
+        X, H, Y = pad(x, (1, 1, 1, 1)), pad(h1, (0, 0, 1, 1, 1, 1)), pad(gy, (1, 1, 1, 1))
+        f1, f2, fh = g1.reshape(-1, 16), g2.reshape(-1, 16), h2.reshape(-1, 16)
+        for tap in range(9):
+            r, c = tap // 3, tap % 3
+            out[tap * 16:tap * 16 + 16] = f1.T @ X[:, r:r + h, c:c + w].reshape(-1)
+            out[160 + tap * 256:416 + tap * 256] = (f2.T @ H[:, r:r + h, c:c + w].reshape(-1, 16)).reshape(-1)
+            out[2480 + tap * 16:2496 + tap * 16] = fh.T @ Y[:, 2 - r:2 - r + h, 2 - c:2 - c + w].reshape(-1)
+        out[144:160], out[2464:2480], out[2624] = f1.sum(0), f2.sum(0), gy.sum()
+        return out
+
+    args = (x.double(), h1, h2, g1, g2, gy)
+    want, size = grads(*args), grads(*(t.abs() for t in args))
+    err = ((net.grads.double() - want).abs() / size.clamp_min(1e-300)).max()
+    assert float(err) < 3e-7
