@@ -11,6 +11,8 @@
 
 namespace gr {
 
+constexpr int kSMs = 148;  // of a B200: what the rules that choose a launch shape count on
+
 // Gridding tile: T x T grid cells per work item.
 constexpr int kTile = 32;
 // Largest number of taps per dimension the gridding kernel handles

@@ -133,7 +133,7 @@ struct Conv2Smem {
 // Segments of a strip, so that `per_sm` blocks per SM fill the GPU about once.
 int strip_segments(int n_img, int h, int w, int per_sm) {
   const long strips = (long)n_img * ((w + kStW - 1) / kStW);
-  return (int)std::max(1L, std::min<long>(h, per_sm * 148L / strips));
+  return (int)std::max(1L, std::min<long>(h, (long)per_sm * kSMs / strips));
 }
 
 __device__ __forceinline__ void cp_async_zfill16(void* dst, const void* src, bool ok) {
@@ -436,7 +436,7 @@ long wg_blocks(int n_img, int h, int w) {
 // room for fewer segments of each.
 size_t wg_blocks_bound(int n_img, int h, int w) {
   const size_t strips = (size_t)n_img * ((w + kWgW - 1) / kWgW);
-  return std::max(strips, std::min(strips * h, (size_t)kWgBlocks * 148));
+  return std::max(strips, std::min(strips * h, (size_t)kWgBlocks * kSMs));
 }
 
 __device__ __forceinline__ void cp_async_zfill4(void* dst, const void* src, bool ok) {

@@ -140,7 +140,7 @@ template <int S>
 cudaError_t launch_backproject(const float* filt, const float2* cs, float* recon, int n, int n_ang,
                                bool finite, int groups, int smem, cudaStream_t st) {
   const long t = (n + kBpTile - 1) / kBpTile;
-  return t * t * groups >= 4 * 148
+  return t * t * groups >= 4 * kSMs
              ? launch_backproject_r<S, 4>(filt, cs, recon, n, n_ang, finite, groups, smem, st)
              : launch_backproject_r<S, 1>(filt, cs, recon, n, n_ang, finite, groups, smem, st);
 }

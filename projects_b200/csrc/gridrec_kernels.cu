@@ -494,8 +494,6 @@ __device__ __forceinline__ float load_sino<U16Linear>(const U16Linear* row, int 
   return __fsub_rn(1.f, __fdiv_rn(__fsub_rn((float)ldg_u16(row, k), d), __fsub_rn(__ldg(&flat[k]), d)));
 }
 
-// Lines of up to 4096 points run 64-register variants (several CTAs per SM);
-// 8192-point lines need 512 threads and use the MAXT = 512 variants.
 // A float row to be shifted and half padded on the way (PaddedInput): the row lands in
 // shared memory at its own length and every padded column takes its two taps from there.  16
 // slices of 2048 x 1500 for a plan 4096 wide: 132 us against 75 for a pass that writes the
@@ -598,6 +596,8 @@ __device__ __forceinline__ float from_staged<U16Linear>(const unsigned short* ro
   return __fsub_rn(1.f, __fdiv_rn(__fsub_rn((float)row[k], d), __fsub_rn(__ldg(&flat[k]), d)));
 }
 
+// Lines of up to 4096 points run 64-register variants (several CTAs per SM);
+// 8192-point lines need 512 threads and use the MAXT = 512 variants.
 template <typename T, int MAXT, int NT>
 __global__ void __launch_bounds__(MAXT, 1024 / MAXT) spectra_kernel(SpectraArgs a) {
   extern __shared__ __align__(16) float2 sm[];
@@ -1368,8 +1368,8 @@ __host__ __device__ constexpr int w32_table_bytes(int ltbl) { return ((ltbl + 2)
 // One sample: x_r = w_r * value (packed (re, im)), then every cell of column pairs
 // C0..C1 adds w_c * x_r; d: the sample's 6 x 16 bytes of doubled weights, rows
 // 0..3 then columns 0..7.  (The packed intrinsics let the compiler keep every accumulator in
-// place across the column-range branches; inline asm with 64-bit operands moved some: 31.1 ->
-// 30.7 us a pair at 2048 x 1500, 8.14 -> 8.06 at 1024 x 720.)
+// place across the column-range branches; inline asm with 64-bit operands moved some.  The time
+// is the same within the noise of the runs: 30.6 us a pair at 2048 x 1500.)
 template <int C0, int C1>
 __device__ __forceinline__ void w32_apply_sample(float2 (&acc)[kWideRows][kWideCols], float2 v,
                                                  const float4* d) {
@@ -2490,7 +2490,7 @@ static int cols_ring_smem(int M, int G) {
 // compiled), in strips of at least two columns whose buffers fit.
 ColForm cols_form(int M, int pairs, int G, int ring) {
   const int Gr = G > 0 ? G : cols_group(M, 1);
-  if (ring < 0) ring = cols_ring_default(M) && (long)(M / Gr) * pairs >= 4 * 148;
+  if (ring < 0) ring = cols_ring_default(M) && (long)(M / Gr) * pairs >= 4 * kSMs;
   int optin = 0, dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);

@@ -890,14 +890,15 @@ GridArgs grid_args_group(const Plan* p, const GroupList* l, int pairs) {
   g.rec = l->d_rec;
   // Items of more than `share` of a warp's part of all records are long, gridded by a warp
   // each: a bundle takes as many steps as its longest item, and one that holds a large
-  // part of a warp's whole work ends after all others.  Per pair at 2048 x 1500, share 0.05 /
-  // 0.15 / 0.4 / 1 / none long: 42.2 / 36.3 / 35.3 / 39.6 / 39.4 us for 8 pairs, 68.2 / 62.0 /
-  // 57.7 / 66.4 / 78.4 for 4, 106 / 89 / 88 / 90 / 90 for 2; at 1024 x 720 12.9 / 12.7 / 12.2 /
-  // 13.9 / 23.1 for 8, 32.3 / 32.9 / 30.4 / 31.8 / 52.8 for 2, 60 / 60 / 64 / 74 / 440 for one (a
-  // bundle of 32 items is the less efficient form of the two).
+  // part of a warp's whole work ends after all others.  Per pair, share 0.05 / 0.15 / 0.3 / 0.4 / 1
+  // / none long, us: 2048 x 1500 8 pairs 42.2 / 37.4 / 35.3 / 36.1 / 39.6 / 39.4, 4 pairs 68.2 / 61.9 /
+  // 57.9 / 57.9 / 66.4 / 78.4; 1024 x 720 8 pairs 12.9 / 12.5 / 12.3 / 12.3 / 13.9 / 23.1, 4 pairs (0.15
+  // to 0.4) 20.0 / 21.0 / 21.5.  Two pairs without 0.3: 106 / 89 / 88 / 90 / 90 and 32.3 / 32.9 / 30.4 / 31.8 /
+  // 52.8; one pair at 1024 x 720 60 / 60 / 64 / 74 / 440 (a bundle of 32 items is the less
+  // efficient form of the two).
   const int G = group_size(pairs);
   const double share = G == 1 ? 0.05 : (G == 2 ? 0.4 : 0.3);
-  const double part = (double)l->records * G * grp_row_split(G) / 32 / (kGrpMinBlocks * 4 * 148);
+  const double part = (double)l->records * G * grp_row_split(G) / 32 / (kGrpMinBlocks * 4 * kSMs);
   g.n_long = l->longer[std::min(grp_class((int)std::min(part * share, 1e9)), kGrpClasses - 1)];
   return g;
 }

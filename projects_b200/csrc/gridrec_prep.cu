@@ -532,9 +532,8 @@ __global__ void ring_update_kernel(float* data, float* rowmean, const float* col
 }
 
 // ---------------------------------------------------------------------------
-// Sub-pixel shift and half padding.  Output slice s reads input slice
-// (s % in_mod) and shift xoff[s / off_div] (x_const when xoff is null).  Column k of the input row maps to
-// kp = k + pad (pad = n_det / 2) and takes
+// Sub-pixel shift and half padding.  Slice s is shifted by x0 = xoff[s].  Column k of the
+// input row maps to kp = k + pad (pad = n_det / 2) and takes
 //   kk = k - x0,  n = floor(kk),  in[clamp(n)] (n + 1 - kk) + in[clamp(n + 1)] (kk - n)
 // with indices clamped to [0, n_det); columns left of pad repeat column pad,
 // the pad columns right of pad + n_det repeat column pad + n_det - 1, and any
@@ -549,13 +548,12 @@ constexpr int kShiftStageMax = 12288;  // 48 KB of dynamic shared memory
 
 template <bool kStaged>
 __global__ void __launch_bounds__(kPrepThreads) shift_pad_kernel(
-    const float* in, long in_slice, int in_mod, const float* xoff, int off_div, float x_const,
-    float* out, int n_det, int n_ang, int out_width) {
+    const float* in, const float* xoff, float* out, int n_det, int n_ang, int out_width) {
   extern __shared__ float srow[];
   const int i = blockIdx.x, s = blockIdx.y;
-  const float* r = in + (size_t)(s % in_mod) * in_slice + (size_t)i * n_det;
+  const float* r = in + ((size_t)s * n_ang + i) * n_det;
   float* o = out + ((size_t)s * n_ang + i) * out_width;
-  const float x0 = xoff ? xoff[s / off_div] : x_const;
+  const float x0 = xoff[s];
   const int pad = n_det / 2;
   if (kStaged) {
     int q0 = 0;
@@ -602,16 +600,14 @@ __global__ void __launch_bounds__(kPrepThreads) shift_pad_kernel(
 // us per slice: 256 threads 11.2, 128 threads 9.9, 64 threads 10.9).
 constexpr int kShiftThreads = 128;
 
-void launch_shift_pad(int n_ang, int n_out, cudaStream_t st, const float* in, long in_slice,
-                      int in_mod, const float* xoff, int off_div, float x_const, float* out,
-                      int n_det, int out_width) {
-  const dim3 grid(n_ang, n_out);
+void launch_shift_pad(int n_ang, int n_slices, cudaStream_t st, const float* in, const float* xoff,
+                      float* out, int n_det, int out_width) {
+  const dim3 grid(n_ang, n_slices);
   if (n_det <= kShiftStageMax)
     shift_pad_kernel<true><<<grid, kShiftThreads, (size_t)n_det * sizeof(float), st>>>(
-        in, in_slice, in_mod, xoff, off_div, x_const, out, n_det, n_ang, out_width);
+        in, xoff, out, n_det, n_ang, out_width);
   else
-    shift_pad_kernel<false><<<grid, kShiftThreads, 0, st>>>(in, in_slice, in_mod, xoff, off_div,
-                                                             x_const, out, n_det, n_ang, out_width);
+    shift_pad_kernel<false><<<grid, kShiftThreads, 0, st>>>(in, xoff, out, n_det, n_ang, out_width);
 }
 
 // ---------------------------------------------------------------------------
@@ -782,7 +778,7 @@ int launch_entropy(const Window& w, int n_groups, float vmin, float vmax, int nb
       cudaMemsetAsync(ghist, 0, (size_t)n_groups * (nbins + 1) * sizeof(unsigned), st);
   if (e != cudaSuccess) return fail(GR_ERR_CUDA, "hist memset: %s", cudaGetErrorString(e));
   const int total_rows = w.rows * w.group;
-  const int bx = std::max(1, std::min(total_rows, (4 * 148 + n_groups - 1) / n_groups));
+  const int bx = std::max(1, std::min(total_rows, (4 * kSMs + n_groups - 1) / n_groups));
   hist_kernel<<<dim3(bx, n_groups), 512, smem, st>>>(w, vmin, inv, nbins, ghist);
   entropy_final_kernel<<<n_groups, kEntropyThreads, 0, st>>>(ghist, nbins,
                                                  (double)w.rows * w.cols * w.group, out);
@@ -992,7 +988,7 @@ constexpr int kRingRB = 2;  // rows at once at 2048 and 4096 columns, twice that
 
 // Rows per block on rows of whole 16-byte pieces: one wave of blocks over the GPU, in equal
 // parts of whole row groups.
-constexpr int ring_wave(int n_det) { return ring_blocks(ring_threads(n_det)) * 148; }
+constexpr int ring_wave(int n_det) { return ring_blocks(ring_threads(n_det)) * kSMs; }
 int ring_rows_vec(int n_slices, int n_det, int n_ang) {
   const long wave = ring_wave(n_det);
   const int rows = (int)(((long)n_ang * n_slices + wave - 1) / wave);
@@ -1116,8 +1112,7 @@ int gr_shift_pad(const float* in, float* out, int n_slices, int n_det, int n_ang
   if (!in || !out || !xoffsets) return fail(GR_ERR_ARG, "shift/pad: null pointer");
   if (n_slices < 1 || n_det < 1 || n_ang < 1 || out_width < n_det)
     return fail(GR_ERR_ARG, "shift/pad: need n_slices, n_det, n_ang >= 1 and out_width >= n_det");
-  launch_shift_pad(n_ang, n_slices, (cudaStream_t)stream, in, (long)n_ang * n_det, n_slices,
-                   xoffsets, 1, 0.f, out, n_det, out_width);
+  launch_shift_pad(n_ang, n_slices, (cudaStream_t)stream, in, xoffsets, out, n_det, out_width);
   return check_launch("shift/pad");
 }
 
@@ -1293,7 +1288,7 @@ int gr_xcorr_scores(const float* templ_roi, const float* match, int width, int h
   const int roi_w = roi_x1 - roi_x0 + 1, roi_h = roi_y1 - roi_y0 + 1;
   const int n_trans = n_tx * n_ty;
   // enough blocks to fill the GPU: split the ROI rows when translations are few
-  const int want_blocks = 4 * 148;
+  const int want_blocks = 4 * kSMs;
   int nblk = std::max(1, std::min(roi_h, (want_blocks + n_trans - 1) / n_trans));
   const int rows_per = (roi_h + nblk - 1) / nblk;
   nblk = (roi_h + rows_per - 1) / rows_per;
