@@ -126,7 +126,10 @@ int gr_plan_destroy(gr_plan* plan);
  * M0 = 2*floor(M/2/sampl - 0.5) + 1 = side of the reconstructed image. */
 int gr_plan_sizes(const gr_plan* plan, int* pdim, int* M, int* M0, float* L, float* scale);
 
-/* Device bytes held by the plan (tables, work list, workspaces). */
+/* Device bytes held by the plan (tables, work list, workspaces).  They include the records
+ * by which chunks of up to 8 pairs grid (32 bytes per sample and 4 x 8 sub-tile it reaches,
+ * 226 MB at 2048 x 1500; two lists in plans of 7 pairs and more), which are left out where the
+ * GPU has no room for them. */
 int gr_plan_device_bytes(const gr_plan* plan, size_t* bytes);
 
 /* One slice pair, device pointers.  sino1/sino2: n_ang x n_det float32, row
